@@ -354,69 +354,159 @@ __global__ void __launch_bounds__(128) k_conv_tc(const bf16 *__restrict__ in, co
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
 }
 
-// dpre = dh * gelu'(pre) over the interior (halo left at zero)
+// dpre = dh * gelu'(pre) over the interior (halo left at zero).  Bound by HBM
+// (6 bytes a value); V values (16 bytes) a thread and step where the channels
+// come in eights and the buffers are 16-byte aligned, V = 1 otherwise.
+// (32 x 144 x 144 x 32 values: see tl_nn_wgrad for the pass's times.)
+template <int V>
 __global__ void k_gelu_back(const bf16 *__restrict__ dh, const bf16 *__restrict__ pre,
                             bf16 *__restrict__ dpre, int C, int B, int H, int W) {
-    const long long n = (long long)B * H * W * C;
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n;
-         k += (long long)gridDim.x * blockDim.x) {
-        const int c = (int)(k % C);
-        const long long px = k / C;
-        const int x = (int)(px % W), y = (int)((px / W) % H), b = (int)(px / ((long long)W * H));
-        const long long o = (((long long)b * (H + 2) + y + 1) * (W + 2) + x + 1) * C + c;
-        dpre[o] = __float2bfloat16(__bfloat162float(dh[o]) * gelu_grad(__bfloat162float(pre[o])));
-    }
-}
-
-// Weight gradient: warp `tap` of each CTA accumulates
-//   dW[tap][co][ci] += sum_p dpre[p][co] * in[p + off(tap)][ci]
-// over the CTA's run of 16-pixel groups with mma (M = co, N = ci, K = pixels);
-// the CTA writes its partial [9][COUTP][CIN].
-template <int CIN, int COUTP>
-__global__ void __launch_bounds__(288) k_wgrad(const bf16 *__restrict__ dpre,
-                                               const bf16 *__restrict__ in,
-                                               float *__restrict__ partial, int B, int H, int W,
-                                               int groups_per_cta) {
-    const int lane = threadIdx.x & 31, tap = threadIdx.x >> 5;
-    const int g = lane >> 2, t = lane & 3;
-    const int dy = tap / 3, dx = tap % 3;
-    constexpr int MT = COUTP / 16, NT = CIN / 8;
-    float acc[MT][NT][4];
+    const int CV = C / V;
+    const long long rows = (long long)B * H;
+    const int per_row = W * CV;
+    for (long long row = blockIdx.x; row < rows; row += gridDim.x) {
+        const int y = (int)(row % H), b = (int)(row / H);
+        const long long o0 = (((long long)b * (H + 2) + y + 1) * (W + 2) + 1) * C;
+        for (int k = threadIdx.x; k < per_row; k += blockDim.x) {
+            const long long o = o0 + (long long)k * V;
+            if constexpr (V == 8) {
+                const uint4 d4 = *reinterpret_cast<const uint4 *>(dh + o);
+                const uint4 p4 = *reinterpret_cast<const uint4 *>(pre + o);
+                const uint32_t dw[4] = {d4.x, d4.y, d4.z, d4.w}, pw[4] = {p4.x, p4.y, p4.z, p4.w};
+                uint32_t ow[4];
 #pragma unroll
-    for (int i = 0; i < MT; ++i)
-#pragma unroll
-        for (int j = 0; j < NT; ++j) acc[i][j][0] = acc[i][j][1] = acc[i][j][2] = acc[i][j][3] = 0.f;
-    const int wx = W / 16;
-    const long long ngroups = (long long)B * H * wx;
-    const long long Wp = W + 2;
-    const long long g0 = (long long)blockIdx.x * groups_per_cta;
-    for (long long q = g0; q < g0 + groups_per_cta && q < ngroups; ++q) {
-        const int b = (int)(q / ((long long)H * wx));
-        const int rem = (int)(q % ((long long)H * wx));
-        const int y = rem / wx, x0 = (rem % wx) * 16;
-        // dpre at interior pixels (y, x0 + k): padded (y + 1, x0 + k + 1)
-        const bf16 *dp = dpre + (((long long)b * (H + 2) + y + 1) * Wp + x0 + 1) * COUTP;
-        // in at padded (y + dy, x0 + k + dx)
-        const bf16 *ip = in + (((long long)b * (H + 2) + y + dy) * Wp + x0 + dx) * CIN;
-#pragma unroll
-        for (int mt = 0; mt < MT; ++mt) {
-            const int co = mt * 16 + g;
-            const uint32_t a0 = pack2(dp[(2 * t) * COUTP + co], dp[(2 * t + 1) * COUTP + co]);
-            const uint32_t a1 = pack2(dp[(2 * t) * COUTP + co + 8], dp[(2 * t + 1) * COUTP + co + 8]);
-            const uint32_t a2 = pack2(dp[(2 * t + 8) * COUTP + co], dp[(2 * t + 9) * COUTP + co]);
-            const uint32_t a3 = pack2(dp[(2 * t + 8) * COUTP + co + 8], dp[(2 * t + 9) * COUTP + co + 8]);
-#pragma unroll
-            for (int nt = 0; nt < NT; ++nt) {
-                const int ci = nt * 8 + g;
-                const uint32_t b0 = pack2(ip[(2 * t) * CIN + ci], ip[(2 * t + 1) * CIN + ci]);
-                const uint32_t b1 = pack2(ip[(2 * t + 8) * CIN + ci], ip[(2 * t + 9) * CIN + ci]);
-                mma16816(acc[mt][nt], a0, a1, a2, a3, b0, b1);
+                for (int e = 0; e < 4; ++e) {
+                    const float d0 = __uint_as_float(dw[e] << 16), d1 = __uint_as_float(dw[e] & 0xFFFF0000u);
+                    const float p0 = __uint_as_float(pw[e] << 16), p1 = __uint_as_float(pw[e] & 0xFFFF0000u);
+                    ow[e] = pack2(__float2bfloat16(d0 * gelu_grad(p0)), __float2bfloat16(d1 * gelu_grad(p1)));
+                }
+                *reinterpret_cast<uint4 *>(dpre + o) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
+            } else {
+                dpre[o] = __float2bfloat16(__bfloat162float(dh[o]) * gelu_grad(__bfloat162float(pre[o])));
             }
         }
     }
+}
+
+// Weight and bias gradients:
+//   dW[tap][co][ci] = sum_p dpre[p][co] * in[p + off(tap)][ci],  db[co] = sum_p dpre[p][co]
+// A contraction over the pixels with M = co and N = ci of 16 or 32 a tap, below
+// the 64 rows of a tensor-memory MMA, so it runs on mma.sync (M = co, N = ci,
+// K = 16 pixels), one warp a tap; warp 4 also multiplies dpre by a column of
+// ones, which is db.  A CTA walks segments of kWgSeg pixels of a row (a
+// grid-stride loop over the segments of all rows): it stages the segment's
+// dpre and the three input rows its taps read in shared memory (16-byte
+// cp.async, two buffers: the next segment loads while this one multiplies),
+// pixels kWgStride bytes apart so that ldmatrix reads eight pixels' 16 bytes
+// without bank conflicts, and takes both operands transposed by
+// ldmatrix.trans.  Each CTA writes one partial [9][COUTP][CIN] (and [COUTP]).
+constexpr int kWgSeg = 64;
+constexpr int kWgThreads = 288;
+__host__ __device__ constexpr int wg_stride(int ch) { return ch * 2 + 16; }
+__host__ __device__ constexpr int wg_buffer(int cin, int coutp) {
+    return 3 * (kWgSeg + 2) * wg_stride(cin) + kWgSeg * wg_stride(coutp);
+}
+
+__device__ __forceinline__ void ldsm4t(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr));
+}
+
+// eight channels to shared memory; buffers that are not 16-byte aligned go
+// through registers
+__device__ __forceinline__ void stage16(uint32_t dst, const bf16 *src, bool aligned) {
+    if (aligned) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src));
+    } else {
+        asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(dst), "r"(pack2(src[0], src[1])),
+                     "r"(pack2(src[2], src[3])), "r"(pack2(src[4], src[5])), "r"(pack2(src[6], src[7]))
+                     : "memory");
+    }
+}
+
+template <int CIN, int COUTP>
+__global__ void __launch_bounds__(kWgThreads) k_wgrad(const bf16 *__restrict__ dpre, const bf16 *__restrict__ in,
+                                                      float *__restrict__ partial, float *__restrict__ dbpart,
+                                                      int B, int H, int W) {
+    constexpr int SI = wg_stride(CIN), SO = wg_stride(COUTP);
+    constexpr int BUF = wg_buffer(CIN, COUTP);
+    constexpr int MT = COUTP / 16, NT = CIN / 8;
+    extern __shared__ __align__(16) unsigned char wsm[];
+    const uint32_t sm0 = smem_addr(wsm);
+    const int tid = threadIdx.x, lane = tid & 31, tap = tid >> 5;
+    const int dy = tap / 3, dx = tap % 3;
+    float acc[MT][NT][4], accb[MT][4];
+#pragma unroll
+    for (int i = 0; i < MT; ++i) {
+        accb[i][0] = accb[i][1] = accb[i][2] = accb[i][3] = 0.f;
+#pragma unroll
+        for (int j = 0; j < NT; ++j) acc[i][j][0] = acc[i][j][1] = acc[i][j][2] = acc[i][j][3] = 0.f;
+    }
+    const int segs = (W + kWgSeg - 1) / kWgSeg;
+    const long long tasks = (long long)B * H * segs;
+    const long long Wp = W + 2;
+    const bool aligned = (((uintptr_t)dpre | (uintptr_t)in) & 15) == 0;
+    auto stage = [&](long long q, int buf) {
+        const int sx = (int)(q % segs);
+        const long long row = q / segs;
+        const int y = (int)(row % H), b = (int)(row / H);
+        const int x0 = sx * kWgSeg, np = min(kWgSeg, W - x0);
+        const uint32_t base = sm0 + buf * BUF;
+        constexpr int CI8 = CIN / 8, CO8 = COUTP / 8;
+        const bf16 *ip = in + (((long long)b * (H + 2) + y) * Wp + x0) * CIN;
+        for (int k = tid; k < 3 * (kWgSeg + 2) * CI8; k += kWgThreads) {
+            const int c = k % CI8, j = (k / CI8) % (kWgSeg + 2), r = k / (CI8 * (kWgSeg + 2));
+            if (j < np + 2) 
+                stage16(base + (r * (kWgSeg + 2) + j) * SI + c * 16, ip + (r * Wp + j) * CIN + 8 * c, aligned);
+        }
+        const bf16 *dp = dpre + (((long long)b * (H + 2) + y + 1) * Wp + x0 + 1) * COUTP;
+        for (int k = tid; k < kWgSeg * CO8; k += kWgThreads) {
+            const int c = k % CO8, j = k / CO8;
+            if (j < np) 
+                stage16(base + 3 * (kWgSeg + 2) * SI + j * SO + c * 16, dp + (long long)j * COUTP + 8 * c, aligned);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    long long q = blockIdx.x;
+    int buf = 0;
+    if (q < tasks) stage(q, 0);
+    for (; q < tasks; q += gridDim.x, buf ^= 1) {
+        if (q + gridDim.x < tasks) {
+            stage(q + gridDim.x, buf ^ 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();
+        const int np = min(kWgSeg, W - (int)(q % segs) * kWgSeg);
+        const uint32_t sin = sm0 + buf * BUF + (dy * (kWgSeg + 2) + dx) * SI;
+        const uint32_t sdp = sm0 + buf * BUF + 3 * (kWgSeg + 2) * SI;
+        for (int p0 = 0; p0 < np; p0 += 16) {
+            // 8 x 8 blocks [pixel][channel], transposed by the load: lane l
+            // addresses pixel l % 8 (+8 by bit 3 or 4) of its block
+            uint32_t a[MT][4], b[NT / 2][4];
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt)  // (co, px): (0,0) (8,0) (0,8) (8,8)
+                ldsm4t(a[mt], sdp + (p0 + (lane & 7) + ((lane >> 4) & 1) * 8) * SO + (mt * 16 + ((lane >> 3) & 1) * 8) * 2);
+#pragma unroll
+            for (int n2 = 0; n2 < NT / 2; ++n2)  // (px, ci): (0,0) (8,0) (0,8) (8,8)
+                ldsm4t(b[n2], sin + (p0 + (lane & 7) + ((lane >> 3) & 1) * 8) * SI + (n2 * 16 + ((lane >> 4) & 1) * 8) * 2);
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt) {
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt)
+                    mma16816(acc[mt][nt], a[mt][0], a[mt][1], a[mt][2], a[mt][3], b[nt / 2][(nt & 1) * 2],
+                             b[nt / 2][(nt & 1) * 2 + 1]);
+                if (tap == 4) mma16816(accb[mt], a[mt][0], a[mt][1], a[mt][2], a[mt][3], 0x3F803F80u, 0x3F803F80u);
+            }
+        }
+        __syncthreads();  // the buffer is loaded again in the next iteration
+    }
+    const int g = lane >> 2, t = lane & 3;
     float *pp = partial + ((long long)blockIdx.x * 9 + tap) * COUTP * CIN;
 #pragma unroll
-    for (int mt = 0; mt < MT; ++mt)
+    for (int mt = 0; mt < MT; ++mt) {
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
             const int co = mt * 16 + g, ci = nt * 8 + 2 * t;
@@ -425,18 +515,40 @@ __global__ void __launch_bounds__(288) k_wgrad(const bf16 *__restrict__ dpre,
             pp[(co + 8) * CIN + ci] = acc[mt][nt][2];
             pp[(co + 8) * CIN + ci + 1] = acc[mt][nt][3];
         }
+        if (tap == 4 && t == 0 && dbpart) {
+            dbpart[(long long)blockIdx.x * COUTP + mt * 16 + g] = accb[mt][0];
+            dbpart[(long long)blockIdx.x * COUTP + mt * 16 + g + 8] = accb[mt][2];
+        }
+    }
 }
 
-// dW = sum over CTAs of the partials, in CTA order
-__global__ void k_wreduce(const float *__restrict__ partial, float *__restrict__ dw, int n, int nparts) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
+// dW (and db) = sum over CTAs of the partials: a CTA takes 32 values, its 8
+// warps every eighth partial each, then the warps' sums in order
+__global__ void __launch_bounds__(256) k_wreduce(const float *__restrict__ partial, float *__restrict__ dw, int n,
+                                                 const float *__restrict__ dbpart, float *__restrict__ db, int nb,
+                                                 int nparts) {
+    const int nblk = (n + 31) / 32;
+    const bool bias = (int)blockIdx.x >= nblk;
+    const int m = bias ? nb : n;
+    const int k = (bias ? (int)blockIdx.x - nblk : (int)blockIdx.x) * 32 + (threadIdx.x & 31);
+    const int w = threadIdx.x >> 5;
+    const float *src = bias ? dbpart : partial;
     float s = 0.f;
-    for (int p = 0; p < nparts; ++p) s += partial[(long long)p * n + k];
-    dw[k] = s;
+    if (k < m)
+        for (int p = w; p < nparts; p += 8) s += src[(long long)p * m + k];
+    __shared__ float sh[8][32];
+    sh[w][threadIdx.x & 31] = s;
+    __syncthreads();
+    if (w == 0 && k < m) {
+        float t = sh[0][threadIdx.x];
+#pragma unroll
+        for (int v = 1; v < 8; ++v) t += sh[v][threadIdx.x];
+        (bias ? db : dw)[k] = t;
+    }
 }
 
-// db[c] = sum over interior pixels of dpre[p][c]; one CTA per channel
+// db[c] = sum over interior pixels of dpre[p][c], one CTA per channel: where
+// the partial buffer has no room for k_wgrad's (one CTA, a few pixels)
 __global__ void k_dbias(const bf16 *__restrict__ dpre, float *__restrict__ db, int C, int B, int H, int W) {
     const int c = blockIdx.x;
     const long long n = (long long)B * H * W;
@@ -594,7 +706,13 @@ int tl_nn_conv_status(void) {
 }
 
 int tl_nn_gelu_backward(const void *dh, const void *pre, void *dpre, int C, int B, int H, int W, void *stream) {
-    k_gelu_back<<<1216, 256, 0, (cudaStream_t)stream>>>((const bf16 *)dh, (const bf16 *)pre, (bf16 *)dpre, C, B, H, W);
+    const bool vec = C % 8 == 0 && (((uintptr_t)dh | (uintptr_t)pre | (uintptr_t)dpre) & 15) == 0;
+    if (vec)
+        k_gelu_back<8><<<1216, 256, 0, (cudaStream_t)stream>>>((const bf16 *)dh, (const bf16 *)pre, (bf16 *)dpre, C, B,
+                                                              H, W);
+    else
+        k_gelu_back<1><<<1216, 256, 0, (cudaStream_t)stream>>>((const bf16 *)dh, (const bf16 *)pre, (bf16 *)dpre, C, B,
+                                                              H, W);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? TL_OK : cuda_fail(e, "gelu backward launch");
 }
@@ -605,6 +723,10 @@ long long tl_nn_wgrad_partial_floats(int cin, int coutp, int B, int H, int W, in
     return ctas * 9LL * cin * coutp;
 }
 
+// The partial buffer holds one [9][coutp][cin] block per groups_per_cta
+// 16-pixel groups (tl_nn_wgrad_partial_floats); the kernel needs far fewer:
+// two CTAs a multiprocessor, and behind their blocks the CTAs' db partials
+// (one block less than the buffer holds leaves them room).
 int tl_nn_wgrad(const void *dpre, const void *in, int cin, int coutp, float *partial, float *dw, float *db,
                 int B, int H, int W, int groups_per_cta, void *stream) {
     cudaStream_t s = (cudaStream_t)stream;
@@ -613,20 +735,34 @@ int tl_nn_wgrad(const void *dpre, const void *in, int cin, int coutp, float *par
         return TL_ERR_ARG;
     }
     const long long groups = (long long)B * H * (W / 16);
-    const unsigned ctas = (unsigned)((groups + groups_per_cta - 1) / groups_per_cta);
-    if (cin == 16 && coutp == 32)
-        k_wgrad<16, 32><<<ctas, 288, 0, s>>>((const bf16 *)dpre, (const bf16 *)in, partial, B, H, W, groups_per_cta);
-    else if (cin == 32 && coutp == 32)
-        k_wgrad<32, 32><<<ctas, 288, 0, s>>>((const bf16 *)dpre, (const bf16 *)in, partial, B, H, W, groups_per_cta);
-    else if (cin == 32 && coutp == 16)
-        k_wgrad<32, 16><<<ctas, 288, 0, s>>>((const bf16 *)dpre, (const bf16 *)in, partial, B, H, W, groups_per_cta);
-    else {
+    const long long blocks = (groups + groups_per_cta - 1) / groups_per_cta;  // room in `partial`
+    const long long tasks = (long long)B * H * ((W + kWgSeg - 1) / kWgSeg);
+    const int n = 9 * cin * coutp;
+    long long ctas = tasks < 304 ? tasks : 304;
+    const bool bias_here = db && blocks >= 2;
+    if (bias_here) {
+        // ctas blocks and ctas * coutp floats: floor(blocks * n / (n + coutp))
+        const long long fit = blocks * n / (n + coutp);
+        if (ctas > fit) ctas = fit;
+    } else if (ctas > blocks) {
+        ctas = blocks;
+    }
+    float *dbpart = bias_here ? partial + ctas * n : nullptr;
+#define TL_WGRAD_CASE(CI, CO)                                                                                  \
+    if (cin == CI && coutp == CO) {                                                                            \
+        constexpr int bytes = 2 * wg_buffer(CI, CO);                                                           \
+        k_wgrad<CI, CO><<<(unsigned)ctas, kWgThreads, bytes, s>>>((const bf16 *)dpre, (const bf16 *)in, partial, \
+                                                                  dbpart, B, H, W);                            \
+    } else
+    TL_WGRAD_CASE(16, 32)
+    TL_WGRAD_CASE(32, 32)
+    TL_WGRAD_CASE(32, 16) {
         set_error("tl_nn_wgrad: unsupported shape cin=%d coutp=%d", cin, coutp);
         return TL_ERR_ARG;
     }
-    const int n = 9 * cin * coutp;
-    k_wreduce<<<(n + 255) / 256, 256, 0, s>>>(partial, dw, n, (int)ctas);
-    if (db) k_dbias<<<coutp, 256, 0, s>>>((const bf16 *)dpre, db, coutp, B, H, W);
+#undef TL_WGRAD_CASE
+    k_wreduce<<<(n + 31) / 32 + (bias_here ? 1 : 0), 256, 0, s>>>(partial, dw, n, dbpart, db, coutp, (int)ctas);
+    if (db && !bias_here) k_dbias<<<coutp, 256, 0, s>>>((const bf16 *)dpre, db, coutp, B, H, W);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? TL_OK : cuda_fail(e, "wgrad launch");
 }
