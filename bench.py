@@ -79,6 +79,10 @@ BYTES_PER_CELL = {
     "cg_w": 32,          # read p, Kx, Ky; write w
     "cg_ur": 64,         # jac_diag: read u, p, r, w, Mi; write u, r, z
     "cg_p": 24,          # read z, p; write p
+    # FP64 solves in fused passes (cg_w, cg_ur and cg_p run with reflective boundaries)
+    "cg_pw": 72,         # read z, p, u, Kx, Ky, diag; write p, u, w
+    "ppcg_pw": 72,       # the same pass in PPCG's outer iteration
+    "cg_up": 40,         # read p, u, z; write p, u (once a solve)
     "residual": 40,      # read u, u0, Kx, Ky; write r
     "cg_init": 48,       # read r, Kx, Ky; write Mi, z, p
     "common_init": 56,   # read density, energy; write Kx, Ky, u, u0
@@ -119,6 +123,8 @@ TRAFFIC_PER_CELL = {
 # (DMUL, DFMA, DMUL, DFMA, DFMA, DADD), or 5 in the mixed-precision outer
 # pass (DMUL + 4 DFMA), plus one DFMA per dot product
 FP64_INSTR_PER_CELL = {
+    "cg_pw": 9.25,    # beta z + p, alpha p + u, the operator, p.w; a neighbour column a strip
+    "ppcg_pw": 9.25,
     "ppcg_w_zr": 7,   # 5-instruction operator, p.w, r.z
     "cg_w": 7,        # 6-instruction operator, p.w
     "residual": 8,    # 6-instruction operator, u0 - Au, r.r
@@ -135,6 +141,19 @@ def bytes_per_cell(kernel, precond):
         # 1/b of the strip solve); write sd', rtemp, utemp (an inner step
         # before the last)
         return {"none": 32, "jac_diag": 36, "jac_block": 40}[precond]
+    if kernel == "cg_rz":
+        # read w, r + the preconditioner (Mi; or Ky, cp, bfp, diag and 1/diag of
+        # three, three and one row in four); write r, z
+        return {"none": 24, "jac_diag": 40, "jac_block": 54}[precond]
+    if kernel == "cheby_step":
+        # read u, Kx, Ky, diag, u0, p + the preconditioner; write p, u
+        return {"none": 64, "jac_diag": 72, "jac_block": 80}[precond]
+    if kernel == "ppcg_step":
+        # read sd, Kx, Ky, diag, rtemp, utemp + the preconditioner; write sd, rtemp, utemp
+        return {"none": 72, "jac_diag": 80, "jac_block": 88}[precond]
+    if kernel == "ppcg_r":
+        # read w, r + the preconditioner; write r_store, r, rtemp, sd, utemp
+        return {"none": 56, "jac_diag": 64, "jac_block": 78}[precond]
     if kernel == "cheby_p":
         # read u, Kx, Ky, diag, u0, p + the preconditioner (Mi; or cp, bfp);
         # write w, r, p

@@ -69,7 +69,7 @@ cudaError_t device_malloc(void **p, size_t bytes) {
     return cudaMalloc(p, bytes);
 }
 
-static int dalloc(Chunk *c, void **p, size_t bytes) {
+int dalloc(Chunk *c, void **p, size_t bytes) {
     cudaError_t e = device_malloc(p, bytes);
     if (e != cudaSuccess) {
         *p = nullptr;
@@ -145,6 +145,16 @@ static int chunk_alloc(const tl_config_t *cfg, Chunk **out) {
     c->sms = sms > 0 ? sms : 152;
     c->grid_red = sms > 0 ? sms * 4 : 512;
     if (c->grid_red > kMaxRedBlocks) c->grid_red = kMaxRedBlocks;
+    c->g.sms = c->sms < kMaxSlots ? c->sms : kMaxSlots;
+    {
+        // the shortest runs that the device's groups take in one go
+        const long long warps = (long long)c->g.sms * kGroupsPerSm * kGroupWarps;
+        const long long bands = warps / c->g.tiles_x > 1 ? warps / c->g.tiles_x : 1;
+        c->g.run = (int)((c->g.nstrips + bands - 1) / bands);
+        c->g.runs = c->g.tiles_x * ((c->g.nstrips + c->g.run - 1) / c->g.run);
+        c->g.sets = (c->g.runs + kGroupWarps - 1) / kGroupWarps;
+        c->g.groups = c->g.sets < c->g.sms * kGroupsPerSm ? c->g.sets : c->g.sms * kGroupsPerSm;
+    }
 
     int rc;
     e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
@@ -165,6 +175,14 @@ static int chunk_alloc(const tl_config_t *cfg, Chunk **out) {
         }
         *f = (double *)p + c->lead;
     }
+    if (cfg->precond == TL_PREC_JAC_BLOCK) {
+        void *p;
+        if ((rc = dalloc(c, &p, ((size_t)c->lead + (size_t)c->pitch * (size_t)c->g.nstrips + 32) * sizeof(double)))) {
+            chunk_release(c);
+            return rc;
+        }
+        c->rdiag = (double *)p + c->lead;
+    }
     double **mesh[] = {&c->vertexx, &c->vertexy, &c->cellx, &c->celly, &c->celldx, &c->celldy};
     size_t mlen = (size_t)(c->nx > c->ny ? c->nx : c->ny) + 2 * c->h + 2;
     for (double **f : mesh) {
@@ -180,6 +198,12 @@ static int chunk_alloc(const tl_config_t *cfg, Chunk **out) {
     c->partials = (double *)p;
     if ((rc = dalloc(c, &p, 256))) { chunk_release(c); return rc; }
     c->counter = (unsigned int *)p;
+    if ((rc = dalloc(c, &p, 256 + 2 * kMaxSlots * 2 * sizeof(double)))) { chunk_release(c); return rc; }
+    c->loop_arrived = (unsigned int *)p;
+    c->loop_partials = (double *)((char *)p + 256);
+    int coop = 0;
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device);
+    c->loop_ok = coop != 0;
     if ((rc = dalloc(c, &p, sizeof(DevScalars)))) { chunk_release(c); return rc; }
     c->sc = (DevScalars *)p;
     size_t nit = (size_t)cfg->max_iters + 4;

@@ -32,4 +32,38 @@ __device__ __forceinline__ void strip_block_solve(const double *__restrict__ dg,
     }
 }
 
+// x / b for b >= 1 whose correctly rounded reciprocal y is known: two residual
+// corrections of x y.  The first leaves an error below an ulp, and from there, y
+// being correctly rounded, the second rounds correctly (Markstein, "Computation
+// of elementary functions on the IBM RISC System/6000 processor", 1990, theorem
+// on division).  5 fused multiply-adds where the division operator takes about
+// twice as many FP64 instructions; the sign of a zero result may differ from it.
+// Values so small that the residuals would underflow are divided.
+static __device__ __noinline__ double div_slow(double x, double b) { return x / b; }
+__device__ __forceinline__ double div_by(double x, double b, double y) {
+    double q = x * y;
+    q = fma(fma(-b, q, x), y, q);
+    q = fma(fma(-b, q, x), y, q);
+    const unsigned int e = ((unsigned int)__double2hiint(x) >> 20) & 0x7FFu;  // biased exponent
+    if (e < 160u && x != 0.0) q = div_slow(x, b);
+    return q;
+}
+
+// strip_block_solve on values that are in registers: the first row's diagonal
+// and its reciprocal, Ky and bfp of rows 1..3, cp of rows 0..2.  A strip cut
+// short by the field's top has zeros in the missing rows (of x too): the
+// same operations then leave z = 0 there and dp in the last row.
+struct StripFactors {
+    double b0, y0, ky[3], bf[3], cp[3];
+};
+__device__ __forceinline__ void strip_solve(const StripFactors &f, const double (&x)[4], double (&z)[4]) {
+    const double d0 = div_by(x[0], f.b0, f.y0);
+    const double d1 = fma(f.ky[0], d0, x[1]) * f.bf[0];
+    const double d2 = fma(f.ky[1], d1, x[2]) * f.bf[1];
+    z[3] = fma(f.ky[2], d2, x[3]) * f.bf[2];
+    z[2] = fma(-f.cp[2], z[3], d2);
+    z[1] = fma(-f.cp[1], z[2], d1);
+    z[0] = fma(-f.cp[0], z[1], d0);
+}
+
 }  // namespace tl

@@ -23,7 +23,11 @@ constexpr int kStrip = 4;          // block-Jacobi strip height (cuda_kernel_hea
 constexpr int kWarpCols = 32;      // columns per warp: one column per lane
 constexpr int kBlockWarps = 8;     // warps per CTA; each warp owns one 4-row strip
 constexpr int kBlockThreads = kWarpCols * kBlockWarps;
-constexpr int kMaxRedBlocks = 152 * 8;  // grid cap for reducing kernels (SMs x 8)
+constexpr int kGroupWarps = 4;     // FP64 kernels: warps (4-row strips) of a tile
+constexpr int kGroupThreads = kWarpCols * kGroupWarps;
+constexpr int kGroupsPerSm = 8;    // 128 threads each: 32 warps a multiprocessor
+constexpr int kMaxSlots = 256;     // multiprocessors a reduction is spread over
+constexpr int kMaxRedBlocks = kMaxSlots * kGroupsPerSm;  // grid cap for reducing kernels
 
 // Scalars of the device-resident solve (the tea_solve.f90 locals).
 struct DevScalars {
@@ -51,10 +55,10 @@ struct DevScalars {
     int presteps;
     int ppcg_inner;
     int ppcg_iters;                // PPCG outer iterations taken in this solve
-    int pad;
+    int p_sel;                     // which of the two buffers holds the iterate (p, u or sd)
 };
 
-enum DoneCode { kRunning = 0, kConverged = 1, kMaxIters = 2, kSwitch = 3, kBreakdown = 4 };
+enum DoneCode { kRunning = 0, kConverged = 1, kMaxIters = 2, kSwitch = 3, kBreakdown = 4, kStalled = 5 };
 
 // What the last CTA of a kernel does with the grid-wide sums.
 enum Epilogue : int {
@@ -73,6 +77,12 @@ enum Epilogue : int {
     kEpiPw,           // pw = p.w
     kEpiFinishNoSwitch,  // exit test once Chebyshev/PPCG has taken over
     kEpiPwZr,         // pw = sum 0, rro = sum 1, alpha = rro/pw (PPCG outer)
+    kEpiCgPw,         // kEpiCgW, and p is in its other buffer
+    kEpiCgUrFinish,   // kEpiCgUr, then the exit test
+    kEpiPpcgPw,       // pw, alpha = rro / pw, and p is in its other buffer
+    kEpiPpcgZrFinish, // rrn = sum 0, beta, rro = sum 1 (r.z of the next iteration), the exit test
+    kEpiJacobiStep,   // kEpiJacobi, and u is in its other buffer
+    kEpiCheby,        // a Chebyshev step: kEpiChebyFinish, and u is in its other buffer
 };
 
 struct Geo {
@@ -82,6 +92,12 @@ struct Geo {
     int tiles_x;        // ceil(nx / 32)
     int tiles_y;        // ceil(nstrips / 8)
     int tiles;
+    // the FP64 kernels' runs of strips (tl_fp64.cuh)
+    int run;            // strips of a run
+    int runs;           // tiles_x * ceil(nstrips / run)
+    int sets;           // ceil(runs / 4): a set is four runs side by side
+    int groups;         // 4-warp groups that share them: min(sets, sms * 8)
+    int sms;            // multiprocessors (at most kMaxSlots): the slots of a sum
 };
 
 struct RedCtx {
@@ -104,6 +120,8 @@ struct Chunk {
     double *density, *energy0, *energy1, *u, *u0, *p, *r, *w, *z, *mi, *kx, *ky, *sd,
         *rtemp, *utemp, *r_store, *cp, *bfp, *volume, *un;
     double *diag;                // diag(A), refreshed with Kx/Ky by common_init
+    double *rdiag;               // block-Jacobi: 1 / diag of each strip's first row (nstrips rows)
+    double *sd_alt;              // FP64 PPCG: second buffer of sd (allocated on first use)
     double *stage;               // (rows x (nx + 2h)) contiguous copy buffer of
                                  // tl_get_field / tl_set_field (allocated on first use)
     std::vector<void *> allocations;
@@ -118,6 +136,10 @@ struct Chunk {
     DevScalars *sc_host;         // pinned mirror
     DevScalars *poll_host;       // two pinned slots polled by the solve loop
     cudaEvent_t poll_ev[2];
+    // the meeting points of the loop kernels (tl_loop.cu)
+    double *loop_partials;
+    unsigned int *loop_arrived;  // [0] arrivals, [1] arrivals before the next launch
+    bool loop_ok;                // the device can hold a loop kernel's CTAs at once
     double *cg_alphas, *cg_betas;          // device, max_iters + 2
     double *ch_alphas, *ch_betas;          // device coefficient arrays
     int n_coefs_cap;
@@ -174,6 +196,7 @@ inline RedCtx red_ctx(Chunk *c, int epi, bool fast) {
 double *field_ptr(Chunk *c, int field);
 // cudaMalloc, except when tl_test_fail_alloc has armed a simulated failure
 cudaError_t device_malloc(void **p, size_t bytes);
+int dalloc(Chunk *c, void **p, size_t bytes);  // zeroed, freed with the chunk
 
 // ------------------------------------------------ kernel launch wrappers
 // (tl_kernels.cu).  `fast` selects the device-resident form: scalars are
@@ -208,6 +231,25 @@ int launch_generate(Chunk *c, int nstates, const tl_state_t *states);
 int launch_fill(Chunk *c, double *f, double v);
 int launch_reflect(Chunk *c, double *f, int depth);
 
+// fused passes and loop kernels (tl_loop.cu), device-resident solves only
+int launch_cg_pass1(Chunk *c, bool ppcg);
+int launch_cg_pass2(Chunk *c);
+int launch_cg_finish(Chunk *c, bool ppcg);  // after the last iteration: u and p up to date
+int launch_cg_loop(Chunk *c);    // many iterations in one launch
+int launch_ppcg_pass2(Chunk *c);             // r_store, r, and the start of the inner steps
+int launch_ppcg_step(Chunk *c, int step);    // one inner step; the last sums (r - r_store).z and r.z
+int launch_ppcg_loop(Chunk *c);
+int ppcg_alloc(Chunk *c);                    // sd_alt
+int launch_ppcg_finish(Chunk *c);            // u, p and sd in their places
+int launch_cheby_step(Chunk *c);
+int launch_cheby_loop(Chunk *c);
+int launch_cheby_finish(Chunk *c);           // u in its place, w and r of the last step
+int launch_jacobi_loop(Chunk *c);
+int launch_jacobi_step(Chunk *c);
+int launch_jacobi_finish(Chunk *c);
+// whether a solve's size is better served by a loop kernel than by a graph of passes
+bool loop_pays(const Chunk *c);
+
 // ------------------------------------------------------ profiling
 // bracket one launch with events when profiling (call before / after)
 int prof_begin(Chunk *c, const char *name, int *slot);
@@ -224,6 +266,9 @@ int solve_timestep(Chunk *c, tl_solve_info_t *info);       // tl_solve.cu
 // run `iters`-iteration graphs of `body` (graph slot `phase`) until the
 // device sets DevScalars::done; *done_out receives it (tl_solve.cu)
 int run_phase(Chunk *c, int (*body)(Chunk *), int iters, int phase, int *done_out);
+// the same with a loop kernel a launch (`loop`), where the device and the
+// chunk's switches allow one; else run_phase
+int run_loop(Chunk *c, int (*loop)(Chunk *), int (*body)(Chunk *), int iters, int phase, int *done_out);
 constexpr int kPhaseMixedInner = 4;
 constexpr int kPhaseMixedPre = 5;
 int solve_timestep_mixed(Chunk *c, tl_solve_info_t *info); // tl_mixed.cu

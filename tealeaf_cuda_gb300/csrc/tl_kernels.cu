@@ -3,258 +3,44 @@
 // Thread mapping: a warp owns 32 adjacent interior columns of one 4-row strip
 // (rows 4s..4s+3, the block-Jacobi strip of tea_block_jacobi.cuknl), one
 // column per lane, so every global access of a warp is a contiguous 256-byte
-// row segment.  A CTA is 8 warps (32 columns x 32 rows); CTAs walk the tiles
-// with a grid-stride loop so a reduction has at most kMaxRedBlocks partials.
+// row segment.  A CTA is a group of 4 warps, each marching down a run of
+// strips; there are as many groups as the device holds at once, so a reduction
+// has at most kMaxRedBlocks partials.
 //
 // Arithmetic follows the reference kernels (kernel_files/*.cuknl) with every
 // a*b+c the reference writes evaluated as one explicit fma(); the file is
 // built with -fmad=false so nvcc adds no other contraction.  The CPU oracle
 // uses the same convention, so a single kernel agrees with it bit for bit.
 //
-// Reductions are deterministic: lanes combine with an xor butterfly, warps in
-// index order, CTAs write one partial each, and the last CTA to finish (an
-// atomic ticket) sums the partials in index order and runs the epilogue that
-// the device-resident solve needs (alpha, beta, exit test).  No CTA ever
-// waits for another.
+// Reductions are deterministic (their order: tl_fp64.cuh): CTAs write one
+// partial each, and the last CTA to finish (an atomic ticket) sums the
+// partials and runs the epilogue that the device-resident solve needs (alpha,
+// beta, exit test).  No CTA of these kernels ever waits for another.
 #include <math.h>
 #include <stdarg.h>
 #include <stdio.h>
 
-#include "tl_internal.cuh"
-#include "tl_device.cuh"
+#include "tl_fp64.cuh"
 
 namespace tl {
 
-// ------------------------------------------------------------ epilogues
-
-__device__ void finish_iteration(DevScalars *s, bool allow_switch) {
-    // tea_solve.f90:400-417: error = sqrt|error|; exit when below eps*||r0||
-    double e = sqrt(fabs(s->error));
-    s->error = e;
-    if (fabs(e) < s->eps * s->initial_residual) {
-        s->done = kConverged;
-        s->n_exit = s->n;
-        return;
-    }
-    if (isnan(e)) {  // breakdown: the reference would carry NaN to max_iters
-        s->done = kBreakdown;
-        s->n_exit = s->n;
-        return;
-    }
-    s->old_error = e;
-    s->n += 1;
-    if (s->n > s->max_iters) {
-        s->done = kMaxIters;
-        s->n_exit = s->n;
-        return;
-    }
-    if (allow_switch && (s->solver == TL_SOLVER_CHEBYSHEV || s->solver == TL_SOLVER_PPCG)) {
-        // tea_solve.f90:157-171, evaluated at the top of the next iteration
-        bool sw = (!s->first && s->solver == TL_SOLVER_PPCG && s->n > 1) ||
-                  (fabs(s->old_error) <= s->epslim && s->n >= s->presteps);
-        if (sw) s->done = kSwitch;
-    }
-}
-
-__device__ void run_epilogue(const RedCtx &red, const double *tot, int nv) {
-    DevScalars *s = red.sc;
-    switch (red.epi) {
-    case kEpiStore:
-        for (int v = 0; v < nv; ++v) s->sum[v] = tot[v];
-        break;
-    case kEpiResid:
-        s->sum[0] = tot[0];
-        s->old_error = tot[0];
-        s->initial_residual = sqrt(fabs(tot[0]));
-        break;
-    case kEpiRro:
-        s->sum[0] = tot[0];
-        s->rro = tot[0];
-        break;
-    case kEpiCgW:
-        s->pw = tot[0];
-        s->alpha = s->rro / s->pw;
-        red.cg_alphas[s->n] = s->alpha;
-        break;
-    case kEpiCgUr:
-        s->rrn = tot[0];
-        s->beta = s->rrn / s->rro;
-        red.cg_betas[s->n] = s->beta;
-        s->error = s->rrn;
-        s->rro = s->rrn;
-        break;
-    case kEpiFinish:
-        finish_iteration(s, true);
-        break;
-    case kEpiFinishNoSwitch:
-        finish_iteration(s, false);
-        break;
-    case kEpiPw:
-        s->pw = tot[0];
-        break;
-    case kEpiPpcgZr:
-        s->rro = tot[0];
-        s->alpha = s->rro / s->pw;
-        break;
-    case kEpiPwZr:
-        s->pw = tot[0];
-        s->rro = tot[1];
-        s->alpha = s->rro / s->pw;
-        break;
-    case kEpiPpcgRrn:
-        s->rrn = tot[0];
-        s->beta = s->rrn / s->rro;
-        s->error = s->rrn;
-        s->rro = s->rrn;
-        s->ppcg_iters += 1;
-        break;
-    case kEpiChebyNorm:
-        s->rr = tot[0];
-        break;
-    case kEpiChebyFinish:
-        // tea_solve.f90:266-283: the residual is read every 10th iteration
-        // after est_itc; cheby_calc_steps += 1 at :284
-        if (s->n >= s->est_itc && s->n % 10 == 0) s->error = s->rr;
-        s->cheby_calc_steps += 1;
-        finish_iteration(s, false);
-        break;
-    case kEpiJacobi:
-        s->error = tot[0];
-        finish_iteration(s, false);
-        break;
-    default:
-        break;
-    }
-}
-
-template <int NV>
-__device__ __forceinline__ void grid_reduce(double (&acc)[NV > 0 ? NV : 1], const RedCtx &red) {
-    __shared__ double sh[kBlockWarps][NV > 0 ? NV : 1];
-    __shared__ int is_last;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-        double x = acc[v];
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) x += __shfl_xor_sync(0xffffffffu, x, off);
-        if (lane == 0) sh[warp][v] = x;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int v = 0; v < NV; ++v) {
-            double t = 0.0;
-            for (int w = 0; w < kBlockWarps; ++w) t += sh[w][v];
-            red.partials[v * kMaxRedBlocks + blockIdx.x] = t;
-        }
-        __threadfence();
-        unsigned int ticket = atomicAdd(red.counter, 1u);
-        is_last = (ticket == gridDim.x - 1);
-    }
-    __syncthreads();
-    if (!is_last) return;
-    __threadfence();
-    double tot[NV > 0 ? NV : 1];
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-        double t = 0.0;
-        for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x)
-            t += __ldcg(&red.partials[v * kMaxRedBlocks + b]);
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) t += __shfl_xor_sync(0xffffffffu, t, off);
-        __syncthreads();
-        if (lane == 0) sh[warp][v] = t;
-        __syncthreads();
-        double s = 0.0;
-        for (int w = 0; w < kBlockWarps; ++w) s += sh[w][v];
-        tot[v] = s;
-    }
-    if (threadIdx.x == 0) {
-        run_epilogue(red, tot, NV);
-        __threadfence();
-        *red.counter = 0u;
-    }
-}
-
 // The grid-stride strip kernel: Body processes one strip column.
 template <int NV, class Body>
-__global__ void __launch_bounds__(kBlockThreads) k_strips(Geo g, Body body, RedCtx red) {
+__global__ void __launch_bounds__(kGroupThreads) k_strips(Geo g, Body body, RedCtx red) {
     if (red.done && *(volatile const int *)red.done) return;
     double acc[NV > 0 ? NV : 1];
 #pragma unroll
     for (int v = 0; v < (NV > 0 ? NV : 1); ++v) acc[v] = 0.0;
     body.setup();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int t = blockIdx.x; t < g.tiles; t += gridDim.x) {
-        const int tx = t % g.tiles_x, ty = t / g.tiles_x;
-        const int i = tx * kWarpCols + lane;
-        const int s = ty * kBlockWarps + warp;
-        if (i < g.nx && s < g.nstrips) {
-            const int j0 = s * kStrip;
-            const int m = min(kStrip, g.ny - j0);
-            const int64_t base = (int64_t)(i + g.h) + (int64_t)(j0 + g.h) * g.pitch;
-            body(base, m, acc);
-        }
-    }
-    if (red.epi != kEpiNone) grid_reduce<NV>(acc, red);
+    for_runs(g, blockIdx.x, warp, [&](int i0, int jb, int je) {
+        const int i = i0 + lane;
+        if (i >= g.nx) return;
+        for (int j0 = jb; j0 < je; j0 += kStrip)
+            body((int64_t)(i + g.h) + (int64_t)(j0 + g.h) * g.pitch, min(kStrip, je - j0), acc);
+    });
+    if (red.epi != kEpiNone) grid_reduce<NV>(acc, red, g.sms);
 }
-
-// ------------------------------------------------------------- helpers
-
-// diag(A) of tea_leaf_common.cuknl:137-139: (1 + (Ky_n + Ky_c)) + (Kx_e + Kx_c)
-__device__ __forceinline__ double diag_at(const double *__restrict__ kx,
-                                          const double *__restrict__ ky, int64_t i, int pitch) {
-    return (1.0 + (ky[i + pitch] + ky[i])) + (kx[i + 1] + kx[i]);
-}
-
-// A x on the m rows of a strip (tea_leaf_common.cuknl:28-34).  xc receives
-// the centre values.  Rows beyond m are neither read nor written.
-// FIVE: the same operator as one product and four fused subtractions
-// (5 FP64 instructions instead of 6; other rounding, so only for callers
-// that do not need the reference's bits)
-template <class X, bool FIVE = false>
-__device__ __forceinline__ void strip_apply(const double *__restrict__ kx,
-                                            const double *__restrict__ ky,
-                                            const double *__restrict__ dg, int pitch,
-                                            int64_t base, int m, X x, double (&xc)[4],
-                                            double (&ax)[4]) {
-    double xr[6];   // rows -1..4
-    double kyr[5];  // faces of rows 0..4
-#pragma unroll
-    for (int k = -1; k <= 4; ++k)
-        if (k <= m) xr[k + 1] = x(base + (int64_t)k * pitch);
-#pragma unroll
-    for (int k = 0; k <= 4; ++k)
-        if (k <= m) kyr[k] = ky[base + (int64_t)k * pitch];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        if (k < m) {
-            const int64_t i = base + (int64_t)k * pitch;
-            const double kxc = kx[i], kxe = kx[i + 1];
-            const double xw = x(i - 1), xe = x(i + 1);
-            const double diag = dg[i];
-            if (FIVE) {
-                double v = diag * xr[k + 1];
-                v = fma(-kyr[k + 1], xr[k + 2], v);
-                v = fma(-kyr[k], xr[k], v);
-                v = fma(-kxe, xe, v);
-                ax[k] = fma(-kxc, xw, v);
-            } else {
-                const double a = fma(kyr[k + 1], xr[k + 2], kyr[k] * xr[k]);
-                const double b = fma(kxe, xe, kxc * xw);
-                ax[k] = fma(diag, xr[k + 1], -a) - b;
-            }
-            xc[k] = xr[k + 1];
-        }
-    }
-}
-
-struct LoadX {
-    const double *__restrict__ f;
-    __device__ __forceinline__ double operator()(int64_t i) const { return f[i]; }
-};
-
-__device__ __forceinline__ double coef(const double *p, double v) { return p ? *p : v; }
 
 // ------------------------------------------------------------- bodies
 
@@ -298,6 +84,8 @@ struct BodyCgInit {  // tea_leaf_kernel_cuda.cu:164-186 fused per strip
     const double *r, *kx, *ky;
     double *p, *z, *mi, *cp, *bfp;
     int pitch;
+    double *rd;  // 1 / diag of the strips' first rows, a row a strip
+    int h;
     __device__ void setup() {}
     __device__ void operator()(int64_t base, int m, double (&acc)[1]) const {
         double rv[4], zv[4];
@@ -305,6 +93,8 @@ struct BodyCgInit {  // tea_leaf_kernel_cuda.cu:164-186 fused per strip
         for (int k = 0; k < 4; ++k)
             if (k < m) rv[k] = r[base + (int64_t)k * pitch];
         if (PC == TL_PREC_JAC_BLOCK) {
+            const int row = (int)(base / pitch);
+            rd[base - (int64_t)row * pitch + (int64_t)((row - h) / kStrip) * pitch] = 1.0 / dg[base];
             // block_init (tea_block_jacobi.cuknl:83-111)
             double cprev = (-ky[base + pitch]) / dg[base];
             cp[base] = cprev;
@@ -927,10 +717,9 @@ __global__ void k_reflect(Geo g, double *__restrict__ f, int depth, int pass) {
 
 template <int NV, class Body>
 static int run(Chunk *c, const char *name, const Body &body, int epi, bool fast) {
-    const int grid = c->g.tiles < c->grid_red ? c->g.tiles : c->grid_red;
     int slot = -1;
     if (c->profiling && !c->capturing) prof_begin(c, name, &slot);
-    k_strips<NV, Body><<<grid, kBlockThreads, 0, c->stream>>>(c->g, body, red_ctx(c, epi, fast));
+    k_strips<NV, Body><<<c->g.groups, kGroupThreads, 0, c->stream>>>(c->g, body, red_ctx(c, epi, fast));
     if (slot >= 0) prof_end(c, slot);
     c->launches++;
     cudaError_t e = cudaGetLastError();
@@ -971,15 +760,18 @@ int launch_norm(Chunk *c, const double *a, const double *bb, int epi) {
 int launch_cg_init(Chunk *c, int epi) {
     switch (c->cfg.precond) {
     case TL_PREC_JAC_BLOCK: {
-        BodyCgInit<TL_PREC_JAC_BLOCK> b{c->diag, c->r, c->kx, c->ky, c->p, c->z, c->mi, c->cp, c->bfp, c->pitch};
+        BodyCgInit<TL_PREC_JAC_BLOCK> b{c->diag, c->r, c->kx, c->ky, c->p, c->z, c->mi, c->cp, c->bfp, c->pitch,
+                                        c->rdiag, c->h};
         return run<1>(c, "cg_init", b, epi, false);
     }
     case TL_PREC_JAC_DIAG: {
-        BodyCgInit<TL_PREC_JAC_DIAG> b{c->diag, c->r, c->kx, c->ky, c->p, c->z, c->mi, c->cp, c->bfp, c->pitch};
+        BodyCgInit<TL_PREC_JAC_DIAG> b{c->diag, c->r, c->kx, c->ky, c->p, c->z, c->mi, c->cp, c->bfp, c->pitch,
+                                        c->rdiag, c->h};
         return run<1>(c, "cg_init", b, epi, false);
     }
     default: {
-        BodyCgInit<TL_PREC_NONE> b{c->diag, c->r, c->kx, c->ky, c->p, c->z, c->mi, c->cp, c->bfp, c->pitch};
+        BodyCgInit<TL_PREC_NONE> b{c->diag, c->r, c->kx, c->ky, c->p, c->z, c->mi, c->cp, c->bfp, c->pitch,
+                                        c->rdiag, c->h};
         return run<1>(c, "cg_init", b, epi, false);
     }
     }

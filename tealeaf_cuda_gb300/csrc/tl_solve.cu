@@ -65,15 +65,33 @@ int ppcg_inner_steps(Chunk *c, bool fast) {
 // one iteration of each phase, launched with fast = true (graph body)
 int body_cg(Chunk *c) {
     int rc;
+    if (!c->cfg.reflective_boundary) {
+        if ((rc = launch_cg_pass1(c, false))) return rc;
+        return launch_cg_pass2(c);
+    }
+    // reflective boundaries mirror p into the halo: p before the operator
     if ((rc = launch_cg_w(c, kEpiCgW, true))) return rc;
     if ((rc = launch_cg_ur(c, 0.0, kEpiCgUr, true))) return rc;
     if ((rc = launch_cg_p(c, 0.0, kEpiFinish, true))) return rc;
     return halo(c, TL_FIELD_P, 1);
 }
 
+// FP64 PPCG in fused passes: not with reflective boundaries (sd and p are
+// mirrored between the pieces) nor without an inner step
+bool ppcg_fused(const Chunk *c) {
+    return c->cfg.precision != TL_PRECISION_MIXED && !c->cfg.reflective_boundary && c->cfg.ppcg_inner_steps >= 1;
+}
+
 int body_ppcg(Chunk *c) {
     int rc;
     const bool mixed = c->cfg.precision == TL_PRECISION_MIXED;
+    if (ppcg_fused(c)) {
+        if ((rc = launch_cg_pass1(c, true))) return rc;
+        if ((rc = launch_ppcg_pass2(c))) return rc;
+        for (int step = 1; step <= c->cfg.ppcg_inner_steps; ++step)
+            if ((rc = launch_ppcg_step(c, step))) return rc;
+        return TL_OK;
+    }
     if ((rc = launch_ppcg_w_store_zr(c, true, mixed))) return rc;
     bool did_rrn = false;
     if (mixed) {
@@ -91,6 +109,7 @@ int body_ppcg(Chunk *c) {
 
 int body_cheby(Chunk *c) {
     int rc;
+    if (!c->cfg.reflective_boundary) return launch_cheby_step(c);
     if ((rc = launch_cheby_calc_p(c, 0, kEpiChebyNorm, true))) return rc;
     if ((rc = launch_cheby_calc_u(c, kEpiChebyFinish, true))) return rc;
     return halo(c, TL_FIELD_U, 1);
@@ -98,6 +117,7 @@ int body_cheby(Chunk *c) {
 
 int body_jacobi(Chunk *c) {
     int rc;
+    if (!c->cfg.reflective_boundary) return launch_jacobi_step(c);
     if ((rc = launch_jacobi(c, kEpiJacobi, true))) return rc;
     return halo(c, TL_FIELD_U, 1);
 }
@@ -169,6 +189,24 @@ int run_phase(Chunk *c, int (*body)(Chunk *), int iters, int phase, int *done_ou
     rc = chunk_sync_scalars(c);
     if (rc) return rc;
     *done_out = c->sc_host->done;
+    return TL_OK;
+}
+
+int run_loop(Chunk *c, int (*loop)(Chunk *), int (*body)(Chunk *), int iters, int phase, int *done_out) {
+    if (!loop_pays(c)) return run_phase(c, body, iters, phase, done_out);
+    for (;;) {
+        int rc = loop(c);
+        if (rc == TL_ERR_STATE && !c->loop_ok) return run_phase(c, body, iters, phase, done_out);
+        if (rc) return rc;
+        if ((rc = chunk_sync_scalars(c))) return rc;
+        if (c->sc_host->done != kRunning) break;
+    }
+    *done_out = c->sc_host->done;
+    if (*done_out == kStalled) {
+        cudaMemsetAsync(c->loop_arrived, 0, 2 * sizeof(unsigned int), c->stream);
+        set_error("the device-resident loop gave up waiting for its thread blocks");
+        return TL_ERR_CUDA;
+    }
     return TL_OK;
 }
 
@@ -285,6 +323,8 @@ int solve_timestep(Chunk *c, tl_solve_info_t *info) {
             h.first = 0;
             h.theta = c->theta;
             h.done = kRunning;
+            h.alpha = h.beta = 0.0;
+            h.p_sel = 0;
             if (use_pp) {
                 // tea_solve.f90:226-250: re-initialise CG with PPCG applied
                 if ((rc = chunk_push_scalars(c))) return rc;
@@ -348,17 +388,26 @@ int solve_timestep(Chunk *c, tl_solve_info_t *info) {
                     done = kSwitch;
                 }
             } else {
-                rc = run_phase(c, body_cg, kItersCg, kPhaseCg, &done);
+                rc = run_loop(c, launch_cg_loop, body_cg, kItersCg, kPhaseCg, &done);
+                if (!rc && !cf.reflective_boundary) rc = launch_cg_finish(c, false);
             }
             break;
         case kPhasePpcg:
-            rc = run_phase(c, body_ppcg, kItersPpcg, kPhasePpcg, &done);
+            if (ppcg_fused(c)) {
+                if ((rc = ppcg_alloc(c))) return rc;
+                rc = run_loop(c, launch_ppcg_loop, body_ppcg, kItersPpcg, kPhasePpcg, &done);
+                if (!rc) rc = launch_ppcg_finish(c);
+            } else {
+                rc = run_phase(c, body_ppcg, kItersPpcg, kPhasePpcg, &done);
+            }
             break;
         case kPhaseCheby:
-            rc = run_phase(c, body_cheby, kItersCheby, kPhaseCheby, &done);
+            rc = run_loop(c, launch_cheby_loop, body_cheby, kItersCheby, kPhaseCheby, &done);
+            if (!rc && !cf.reflective_boundary) rc = launch_cheby_finish(c);
             break;
         case kPhaseJacobi:
-            rc = run_phase(c, body_jacobi, kItersJacobi, kPhaseJacobi, &done);
+            rc = run_loop(c, launch_jacobi_loop, body_jacobi, kItersJacobi, kPhaseJacobi, &done);
+            if (!rc && !cf.reflective_boundary) rc = launch_jacobi_finish(c);
             break;
         }
         if (rc) return rc;
