@@ -90,7 +90,7 @@ BYTES_PER_CELL = {
     "field_summary": 32,
     "finalise": 24,
     "ppcg_p": 24,        # read z, p; write p
-    "ppcg_up": 40,       # read p, u, z; write u, p (mixed PPCG with fused inner passes)
+    "ppcg_wz": 24,       # read w, r, z (mixed PPCG's two dot products)
     "ppcg_update_r": 48,  # read sd, Kx, Ky, diag, rtemp; write rtemp
     "cheby_calc_u": 24,  # read u, p; write u
     "copy": 16,          # read src; write dst
@@ -121,11 +121,10 @@ TRAFFIC_PER_CELL = {
 # FP64 pipe rather than HBM (DFMA, DMUL and DADD each take one issue of the
 # pipe): the operator of tea_leaf_common.cuknl:28-34 as 6 instructions
 # (DMUL, DFMA, DMUL, DFMA, DFMA, DADD), or 5 in the mixed-precision outer
-# pass (DMUL + 4 DFMA), plus one DFMA per dot product
+# pass (DMUL + 4 DFMA), plus one DFMA per dot product and vector update
 FP64_INSTR_PER_CELL = {
     "cg_pw": 9.25,    # beta z + p, alpha p + u, the operator, p.w; a neighbour column a strip
-    "ppcg_pw": 9.25,
-    "ppcg_w_zr": 7,   # 5-instruction operator, p.w, r.z
+    "ppcg_pw": 8.25,  # the same with the 5-instruction operator (mixed precision)
     "cg_w": 7,        # 6-instruction operator, p.w
     "residual": 8,    # 6-instruction operator, u0 - Au, r.r
 }
@@ -171,11 +170,11 @@ def bytes_per_cell(kernel, precond):
     if kernel == "mixed_pp_ur":
         if FUSED_STEPS > 1:
             # read w, r; write r (FP64): the first fused pass starts the inner
-            # steps from r itself and u += alpha p runs in ppcg_up
+            # steps from r itself
             return 24
         # + the FP32 preconditioner (Mi; or Ky, cp, bfp); write rtemp, sd,
         # utemp (FP32)
-        return {"none": 60, "jac_diag": 64, "jac_block": 72}[precond]
+        return {"none": 36, "jac_diag": 40, "jac_block": 48}[precond]
     if kernel == "mixed_pp_fused":
         # the same arrays once per pass of several inner steps; the first
         # pass of a solve reads r (FP64) instead of sd, rtemp and utemp and

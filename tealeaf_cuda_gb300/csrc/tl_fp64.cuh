@@ -150,6 +150,18 @@ static __device__ void run_epilogue(const RedCtx &red, const double *tot, int nv
         s->ppcg_iters += 1;
         finish_iteration(s, false);
         break;
+    case kEpiWzZrFinish:
+        s->rrn = -s->alpha * tot[0];
+        s->beta = s->rrn / s->rro;
+        s->error = s->rrn;
+        s->rro = tot[1];
+        s->ppcg_iters += 1;
+        finish_iteration(s, false);
+        break;
+    case kEpiZrFinish:
+        s->rro = tot[0];
+        finish_iteration(s, false);
+        break;
     case kEpiCheby:
         if (cheby_reads_norm(s)) s->error = s->rr = tot[0];
         s->cheby_calc_steps += 1;
@@ -265,10 +277,7 @@ __device__ __forceinline__ double diag_at(const double *__restrict__ kx,
 
 // A x on the m rows of a strip (tea_leaf_common.cuknl:28-34).  xc receives
 // the centre values.  Rows beyond m are neither read nor written.
-// FIVE: the same operator as one product and four fused subtractions
-// (5 FP64 instructions instead of 6; other rounding, so only for callers
-// that do not need the reference's bits)
-template <class X, bool FIVE = false>
+template <class X>
 __device__ __forceinline__ void strip_apply(const double *__restrict__ kx,
                                             const double *__restrict__ ky,
                                             const double *__restrict__ dg, int pitch,
@@ -289,17 +298,9 @@ __device__ __forceinline__ void strip_apply(const double *__restrict__ kx,
             const double kxc = kx[i], kxe = kx[i + 1];
             const double xw = x(i - 1), xe = x(i + 1);
             const double diag = dg[i];
-            if (FIVE) {
-                double v = diag * xr[k + 1];
-                v = fma(-kyr[k + 1], xr[k + 2], v);
-                v = fma(-kyr[k], xr[k], v);
-                v = fma(-kxe, xe, v);
-                ax[k] = fma(-kxc, xw, v);
-            } else {
-                const double a = fma(kyr[k + 1], xr[k + 2], kyr[k] * xr[k]);
-                const double b = fma(kxe, xe, kxc * xw);
-                ax[k] = fma(diag, xr[k + 1], -a) - b;
-            }
+            const double a = fma(kyr[k + 1], xr[k + 2], kyr[k] * xr[k]);
+            const double b = fma(kxe, xe, kxc * xw);
+            ax[k] = fma(diag, xr[k + 1], -a) - b;
             xc[k] = xr[k + 1];
         }
     }

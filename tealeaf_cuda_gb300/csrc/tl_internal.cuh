@@ -81,6 +81,8 @@ enum Epilogue : int {
     kEpiCgUrFinish,   // kEpiCgUr, then the exit test
     kEpiPpcgPw,       // pw, alpha = rro / pw, and p is in its other buffer
     kEpiPpcgZrFinish, // rrn = sum 0, beta, rro = sum 1 (r.z of the next iteration), the exit test
+    kEpiWzZrFinish,   // rrn = -alpha sum 0, beta, rro = sum 1, the exit test (mixed PPCG)
+    kEpiZrFinish,     // rro = sum 0, the exit test (rrn and beta are there)
     kEpiJacobiStep,   // kEpiJacobi, and u is in its other buffer
     kEpiCheby,        // a Chebyshev step: kEpiChebyFinish, and u is in its other buffer
 };
@@ -220,8 +222,10 @@ int launch_ppcg_calc_sd_new(Chunk *c, int step, bool fast);
 int launch_copy(Chunk *c, double *dst, const double *src, bool fast);
 int launch_ppcg_rrn(Chunk *c, int epi, bool fast);
 int launch_ppcg_zr(Chunk *c, int epi, bool fast);
-int launch_ppcg_w_store_zr(Chunk *c, bool fast, bool five);  // cg_w + ppcg_store_zr, one pass
-int launch_ppcg_up(Chunk *c, int epi, bool fast);  // u += alpha p, p = z + beta p (mixed, fused passes)
+int launch_ppcg_w_store_zr(Chunk *c, bool fast);  // cg_w + ppcg_store_zr, one pass
+// the end of a mixed PPCG iteration: (r - r_store).z (unless the last inner
+// pass summed it), r.z and the exit test
+int launch_mixed_zr(Chunk *c, bool did_rrn);
 int launch_ppcg_p(Chunk *c, double beta, int epi, bool fast);
 int launch_jacobi(Chunk *c, int epi, bool fast);
 int launch_finalise(Chunk *c);
@@ -279,12 +283,9 @@ int mixed_ppcg_prepare(Chunk *c);  // FP32 operator + preconditioner copies
 // FP64; *done_out gets the device's exit code (kSwitch when it switched)
 int mixed_ppcg_presteps(Chunk *c, int *done_out);
 int mixed_ppcg_inner(Chunk *c);    // PPCG inner steps in FP32, z in FP64
-// the outer u/r update fused with the inner start, then the steps; *did_rrn
-// tells whether the last pass also summed (r - r_store).z (kEpiPpcgRrn)
+// r -= alpha w, then the inner steps; *did_rrn tells whether the last pass also
+// summed (r - r_store).z
 int mixed_ppcg_ur_inner(Chunk *c, bool *did_rrn);
-// whether mixed PPCG runs its inner steps as fused passes: its outer pass
-// then updates r alone, and u += alpha p moves into the p pass (launch_ppcg_up)
-bool mixed_fused(const Chunk *c);
 void drop_graphs(Chunk *c);        // after a change that captured graphs depend on
 constexpr int kFusedMax = 5;           // most FP32 PPCG inner steps fused into one pass
 constexpr int kInnerFuseDefault = 5;

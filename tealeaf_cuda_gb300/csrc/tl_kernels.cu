@@ -224,39 +224,6 @@ struct BodyAxpyP {  // p = src + beta p  (tea_leaf_cg.cuknl:141-161, tea_leaf_pp
     }
 };
 
-// mixed PPCG with fused inner passes: u += alpha p (the u half of the outer
-// update, tea_leaf_cg.cuknl:72-137), then p = z + beta p
-// (tea_leaf_ppcg.cuknl:301-313), in one pass over the old p
-struct BodyPpcgUP {
-    double *p, *u;
-    const double *z;
-    const double *alpha_p, *beta_p;
-    int pitch;
-    double alpha, beta;
-    __device__ void setup() {
-        alpha = *alpha_p;
-        beta = *beta_p;
-    }
-    __device__ void operator()(int64_t base, int m, double (&acc)[1]) const {
-        double pv[4], uv[4], zv[4];  // loads first: see BodyCgUr
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-            if (k < m) {
-                const int64_t i = base + (int64_t)k * pitch;
-                pv[k] = p[i];
-                uv[k] = u[i];
-                zv[k] = z[i];
-            }
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-            if (k < m) {
-                const int64_t i = base + (int64_t)k * pitch;
-                u[i] = fma(alpha, pv[k], uv[k]);
-                p[i] = fma(beta, pv[k], zv[k]);
-            }
-    }
-};
-
 template <int PC>
 struct BodyChebyInitP {  // tea_leaf_cheby.cuknl:5-68
     const double *dg;  // diag(A), stored by the diag kernel
@@ -493,10 +460,8 @@ struct BodyCopy {
     }
 };
 
-template <bool FIVE>
 struct BodyCgWStoreZr {  // BodyCgW and BodyStoreZr in one pass: w = A p, r_store = r;
                          // sums p.w and r.z, each in its own kernel's order
-                         // (FIVE: the 5-instruction operator, mixed precision only)
     const double *dg;
     const double *p, *kx, *ky, *r, *z;
     double *w, *r_store;
@@ -504,7 +469,7 @@ struct BodyCgWStoreZr {  // BodyCgW and BodyStoreZr in one pass: w = A p, r_stor
     __device__ void setup() {}
     __device__ void operator()(int64_t base, int m, double (&acc)[2]) const {
         double xc[4], ax[4];
-        strip_apply<LoadX, FIVE>(kx, ky, dg, pitch, base, m, LoadX{p}, xc, ax);
+        strip_apply(kx, ky, dg, pitch, base, m, LoadX{p}, xc, ax);
 #pragma unroll
         for (int k = 0; k < 4; ++k)
             if (k < m) {
@@ -514,6 +479,32 @@ struct BodyCgWStoreZr {  // BodyCgW and BodyStoreZr in one pass: w = A p, r_stor
                 const double rv = r[i];
                 r_store[i] = rv;
                 acc[1] = fma(rv, z[i], acc[1]);
+            }
+    }
+};
+
+// w.z and r.z.  Mixed PPCG's rrn: r - r_store is -alpha w but for r's rounding,
+// so (r - r_store).z = -alpha w.z takes one FP64 instruction a cell instead of
+// two and no stored r; r.z is the next iteration's rro.  HBM-bound.
+struct BodyMixedZr {
+    const double *w, *r, *z;
+    int pitch;
+    __device__ void setup() {}
+    __device__ void operator()(int64_t base, int m, double (&acc)[2]) const {
+        double wv[4], rv[4], zv[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (k < m) {
+                const int64_t i = base + (int64_t)k * pitch;
+                wv[k] = w[i];
+                rv[k] = r[i];
+                zv[k] = z[i];
+            }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (k < m) {
+                acc[0] = fma(wv[k], zv[k], acc[0]);
+                acc[1] = fma(rv[k], zv[k], acc[1]);
             }
     }
 };
@@ -920,18 +911,18 @@ int launch_ppcg_zr(Chunk *c, int epi, bool fast) {
     return run<1>(c, "ppcg_zr", b, epi, fast);
 }
 
-int launch_ppcg_w_store_zr(Chunk *c, bool fast, bool five) {
-    if (five) {
-        BodyCgWStoreZr<true> b{c->diag, c->p, c->kx, c->ky, c->r, c->z, c->w, c->r_store, c->pitch};
-        return run<2>(c, "ppcg_w_zr", b, kEpiPwZr, fast);
-    }
-    BodyCgWStoreZr<false> b{c->diag, c->p, c->kx, c->ky, c->r, c->z, c->w, c->r_store, c->pitch};
+int launch_ppcg_w_store_zr(Chunk *c, bool fast) {
+    BodyCgWStoreZr b{c->diag, c->p, c->kx, c->ky, c->r, c->z, c->w, c->r_store, c->pitch};
     return run<2>(c, "ppcg_w_zr", b, kEpiPwZr, fast);
 }
 
-int launch_ppcg_up(Chunk *c, int epi, bool fast) {
-    BodyPpcgUP b{c->p, c->u, c->z, &c->sc->alpha, &c->sc->beta, c->pitch, 0.0, 0.0};
-    return run<1>(c, "ppcg_up", b, epi, fast);
+int launch_mixed_zr(Chunk *c, bool did_rrn) {
+    if (did_rrn) {
+        BodyNorm b{c->r, c->z, c->pitch};
+        return run<1>(c, "ppcg_zr", b, kEpiZrFinish, true);
+    }
+    BodyMixedZr b{c->w, c->r, c->z, c->pitch};
+    return run<2>(c, "ppcg_wz", b, kEpiWzZrFinish, true);
 }
 
 int launch_ppcg_p(Chunk *c, double beta, int epi, bool fast) {

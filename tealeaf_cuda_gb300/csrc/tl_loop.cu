@@ -219,6 +219,7 @@ struct CgArgs {
     double *p0, *p1;    // p's two buffers (DevScalars::p_sel)
     const double *src;  // z, or r without a preconditioner
     const double *kx, *ky, *dg, *mi, *cp, *bfp, *rd;
+    double *rs;         // r_store, where the last pass sets it
 };
 
 // the block-Jacobi factors of the strip whose first row is at c (row j0)
@@ -249,7 +250,10 @@ struct AlphaBeta {
 // other CTAs write during the launch are read past L1 (__ldcg).  ready():
 // waits for alpha and beta, false if the solve has ended; called once the
 // first loads are on their way.
-template <int D, class Ready>
+// FIVE: the operator as one product and four fused subtractions (5 FP64
+// instructions instead of 6; another rounding, so only for the mixed-precision
+// solve, which has no reference bits to keep)
+template <int D, bool FIVE, class Ready>
 __device__ __forceinline__ void cg_pass1(const Geo &g, const CgArgs &a, const double *__restrict__ pin,
                                          double *__restrict__ pout, int i0, int jb, int je, AlphaBeta &ab, Ready ready,
                                          double &acc) {
@@ -320,16 +324,24 @@ __device__ __forceinline__ void cg_pass1(const Geo &g, const CgArgs &a, const do
                 }
                 // the face east of the last column
                 if (i == g.nx - 1 && lane < 31 && j0 + k < je) kxe = a.kx[c + k * P + 1];
-                t[d] = (d == 0 ? kyv : ky[d > 0 ? d - 1 : 0]) * x[d];
-                b[d] = kx[d] * xw;
-                b[d] = fma(kxe, xe, b[d]);
+                const double kyc = d == 0 ? kyv : ky[d > 0 ? d - 1 : 0];
+                if (FIVE) {
+                    t[d] = fma(-kyc, x[d], dg[d] * x[d + 1]);
+                    t[d] = fma(-kxe, xe, t[d]);
+                    t[d] = fma(-kx[d], xw, t[d]);
+                } else {
+                    t[d] = kyc * x[d];
+                    b[d] = fma(kxe, xe, kx[d] * xw);
+                }
             }
 #pragma unroll
-            for (int d = 0; d < D; ++d) t[d] = fma(ky[d], x[d + 2], t[d]);
+            for (int d = 0; d < D; ++d) t[d] = fma(FIVE ? -ky[d] : ky[d], x[d + 2], t[d]);
+            if (!FIVE) {
 #pragma unroll
-            for (int d = 0; d < D; ++d) t[d] = fma(dg[d], x[d + 1], -t[d]);
+                for (int d = 0; d < D; ++d) t[d] = fma(dg[d], x[d + 1], -t[d]);
 #pragma unroll
-            for (int d = 0; d < D; ++d) t[d] = t[d] - b[d];
+                for (int d = 0; d < D; ++d) t[d] = t[d] - b[d];
+            }
 #pragma unroll
             for (int d = 0; d < D; ++d) {
                 const int64_t at = c + (kb + d) * P;
@@ -402,6 +414,7 @@ __device__ __forceinline__ void cg_pass2(const Geo &g, const CgArgs &a, int i0, 
 }
 
 // the passes as kernels of their own
+template <bool FIVE>
 __global__ void __launch_bounds__(kGroupThreads, 4) k_cg_pass1(Geo g, CgArgs a, RedCtx red) {
     if (*(volatile const int *)red.done) return;
     const bool sel = red.sc->p_sel != 0;
@@ -410,7 +423,7 @@ __global__ void __launch_bounds__(kGroupThreads, 4) k_cg_pass1(Geo g, CgArgs a, 
     AlphaBeta ab{red.sc->alpha, red.sc->beta};
     double acc[1] = {0.0};
     for_runs(g, blockIdx.x, threadIdx.x >> 5, [&](int i0, int jb, int je) {
-        cg_pass1<4>(g, a, pin, pout, i0, jb, je, ab, [] { return true; }, acc[0]);
+        cg_pass1<4, FIVE>(g, a, pin, pout, i0, jb, je, ab, [] { return true; }, acc[0]);
     });
     grid_reduce<1>(acc, red, g.sms);
 }
@@ -458,7 +471,7 @@ __global__ void __launch_bounds__(Shape::kThreads, 1) k_cg_loop(LoopArgs L, CgAr
                 return go;
             };
             loop_pass<1>(L, S, [&](int i0, int jb, int je, double (&acc)[1]) {
-                cg_pass1<Shape::kAhead>(L.g, a, pin, pout, i0, jb, je, ab, ready1, acc[0]);
+                cg_pass1<Shape::kAhead, false>(L.g, a, pin, pout, i0, jb, je, ab, ready1, acc[0]);
             });
             if (!ready1()) break;
             loop_arrive<1>(L, S);
@@ -500,6 +513,7 @@ CgArgs cg_args(Chunk *c, bool ppcg = false) {
     a.cp = c->cp;
     a.bfp = c->bfp;
     a.rd = c->rdiag;
+    a.rs = ppcg && c->cfg.precision == TL_PRECISION_MIXED ? c->r_store : nullptr;
     return a;
 }
 
@@ -542,6 +556,8 @@ __global__ void __launch_bounds__(kGroupThreads) k_cg_finish(Geo g, CgArgs a, co
                     const int64_t c = base + (int64_t)k * g.pitch;
                     a.u[c] = fma(alpha, pv[k], uv[k]);
                     a.p0[c] = fma(beta, pv[k], sv[k]);
+                    // mixed PPCG does without r_store: the r before the last update
+                    if (a.rs) a.rs[c] = fma(alpha, a.w[c], a.r[c]);
                 }
         }
     });
@@ -905,7 +921,7 @@ __global__ void __launch_bounds__(Shape::kThreads, 1) k_ppcg_loop(LoopArgs L, St
                 return go;
             };
             loop_pass<1>(L, S, [&](int i0, int jb, int je, double (&acc)[1]) {
-                cg_pass1<Shape::kAhead>(L.g, cg, pin, pout, i0, jb, je, ab, ready1, acc[0]);
+                cg_pass1<Shape::kAhead, false>(L.g, cg, pin, pout, i0, jb, je, ab, ready1, acc[0]);
             });
             if (!ready1()) break;
             loop_arrive<1>(L, S);
@@ -1149,9 +1165,11 @@ int by_precond(const Chunk *c, F f) {
 }  // namespace
 
 int launch_cg_pass1(Chunk *c, bool ppcg) {
+    const bool five = ppcg && c->cfg.precision == TL_PRECISION_MIXED;
     return launch_named(c, ppcg ? "ppcg_pw" : "cg_pw", [&] {
-        k_cg_pass1<<<c->g.groups, kGroupThreads, 0, c->stream>>>(c->g, cg_args(c, ppcg),
-                                                                  red_ctx(c, ppcg ? kEpiPpcgPw : kEpiCgPw, true));
+        const RedCtx red = red_ctx(c, ppcg ? kEpiPpcgPw : kEpiCgPw, true);
+        if (five) k_cg_pass1<true><<<c->g.groups, kGroupThreads, 0, c->stream>>>(c->g, cg_args(c, ppcg), red);
+        else k_cg_pass1<false><<<c->g.groups, kGroupThreads, 0, c->stream>>>(c->g, cg_args(c, ppcg), red);
     });
 }
 
@@ -1239,7 +1257,7 @@ int launch_ppcg_loop(Chunk *c) {
 
 int launch_ppcg_finish(Chunk *c) {
     const int rc = launch_cg_finish(c, true);
-    if (rc || c->cfg.ppcg_inner_steps % 2 == 0) return rc;
+    if (rc || c->cfg.precision == TL_PRECISION_MIXED || c->cfg.ppcg_inner_steps % 2 == 0) return rc;
     return launch_copy(c, c->sd, c->sd_alt, false);
 }
 

@@ -1266,18 +1266,17 @@ struct BodyUpdateU {  // u += d (FP64)
     }
 };
 
-// PPCG outer update fused with the start of the FP32 inner steps:
-// u += alpha p, r -= alpha w (FP64, as BodyCgUr of tl_kernels.cu), then
-// rtemp = r, z = M^-1 r and sd = utemp = z / theta in FP32 (as k_pp_init):
-// z only seeds the FP32 polynomial preconditioner, so M^-1 uses the FP32
-// operator copies (the block solve of k_pp_step, 1/diag in bfp's first row).
-// START false: the r update alone (the first fused inner pass then starts
-// the inner steps from r itself, and u += alpha p runs in the p pass,
-// BodyPpcgUP)
+// PPCG's r -= alpha w (FP64; u += alpha p runs with the next p, cg_pass1) fused
+// with the start of the FP32 inner steps: rtemp = r, z = M^-1 r and sd = utemp =
+// z / theta in FP32 (as k_pp_init): z only seeds the FP32 polynomial
+// preconditioner, so M^-1 uses the FP32 operator copies (the block solve of
+// k_pp_step, 1/diag in bfp's first row).  START false: the r update alone
+// (the first fused inner pass then starts the inner steps from r itself).
+// rs: r_store, where the last inner pass sums (r - r_store).z.
 template <int PC, bool START>
 struct BodyPpUr {
-    const double *p, *w;
-    double *u, *r;
+    const double *w;
+    double *r, *rs;
     const float *mi, *ky, *cp, *bfp;
     float *sd, *rtemp, *utemp;
     int pitch32, pitch64;
@@ -1290,17 +1289,13 @@ struct BodyPpUr {
     __device__ void operator()(int64_t b32, int64_t b64, int m, CSum &) const {
         // every load of the strip before the first store (the arrays may
         // alias as far as the compiler knows, so it would not hoist them)
-        double uv[4], pv[4], wv[4], rv[4];
+        double wv[4], rv[4];
         float kyv[4], cpv[4], bfv[4], miv[4], rf[4], zf[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k)
             if (k < m) {
                 const int64_t i = b64 + (int64_t)k * pitch64;
                 const int64_t j = b32 + (int64_t)k * pitch32;
-                if (START) {
-                    uv[k] = u[i];
-                    pv[k] = p[i];
-                }
                 wv[k] = w[i];
                 rv[k] = r[i];
                 if (!START) {
@@ -1316,7 +1311,7 @@ struct BodyPpUr {
         for (int k = 0; k < 4; ++k)
             if (k < m) {
                 const int64_t i = b64 + (int64_t)k * pitch64;
-                if (START) u[i] = fma(alpha, pv[k], uv[k]);
+                if (rs) rs[i] = rv[k];
                 rv[k] = fma(-alpha, wv[k], rv[k]);
                 r[i] = rv[k];
                 rf[k] = (float)rv[k];
@@ -1653,18 +1648,17 @@ int mixed_ppcg_inner(Chunk *c) {
     return inner_steps(c, false, &did_rrn, false);
 }
 
-bool mixed_fused(const Chunk *c) { return fused_steps(c) > 1; }
-
 int mixed_ppcg_ur_inner(Chunk *c, bool *did_rrn) {
     if (!inner_ready(c)) return TL_ERR_STATE;
     Mixed *mx = mixed_of(c);
     int rc;
     // with fused passes the first pass starts the inner steps from r, and
-    // this pass only updates r (u += alpha p runs in the p pass)
+    // this pass only updates r
     const bool start = fused_steps(c) == 1;
+    const bool fold = !start && c->inner_fold_rrn;
 #define TL_PP_UR(PC, S)                                                                                       \
-    BodyPpUr<PC, S>{c->p, c->w, c->u, c->r, mx->mi, mx->ky, mx->cp, mx->bfp, mx->sd[0], mx->rtemp, mx->utemp, \
-                    c->pitch, c->pitch, 0.0, 0.f}
+    BodyPpUr<PC, S>{c->w, c->r, fold ? c->r_store : nullptr, mx->mi, mx->ky, mx->cp, mx->bfp, mx->sd[0],     \
+                    mx->rtemp, mx->utemp, c->pitch, c->pitch, 0.0, 0.f}
     if (!start) rc = run32(c, "mixed_pp_ur", TL_PP_UR(TL_PREC_NONE, false), kInNone, true);
     else if (c->cfg.precond == TL_PREC_JAC_BLOCK)
         rc = run32(c, "mixed_pp_ur", TL_PP_UR(TL_PREC_JAC_BLOCK, true), kInNone, true);

@@ -92,18 +92,17 @@ int body_ppcg(Chunk *c) {
             if ((rc = launch_ppcg_step(c, step))) return rc;
         return TL_OK;
     }
-    if ((rc = launch_ppcg_w_store_zr(c, true, mixed))) return rc;
-    bool did_rrn = false;
     if (mixed) {
+        bool did_rrn = false;
+        if ((rc = launch_cg_pass1(c, true))) return rc;
         if ((rc = mixed_ppcg_ur_inner(c, &did_rrn))) return rc;
-    } else {
-        if ((rc = launch_cg_ur(c, 0.0, kEpiNone, true))) return rc;
-        if ((rc = ppcg_inner_steps(c, true))) return rc;
+        return launch_mixed_zr(c, did_rrn);
     }
-    if (!did_rrn && (rc = launch_ppcg_rrn(c, kEpiPpcgRrn, true))) return rc;
-    if (mixed && mixed_fused(c)) rc = launch_ppcg_up(c, kEpiFinishNoSwitch, true);
-    else rc = launch_ppcg_p(c, 0.0, kEpiFinishNoSwitch, true);
-    if (rc) return rc;
+    if ((rc = launch_ppcg_w_store_zr(c, true))) return rc;
+    if ((rc = launch_cg_ur(c, 0.0, kEpiNone, true))) return rc;
+    if ((rc = ppcg_inner_steps(c, true))) return rc;
+    if ((rc = launch_ppcg_rrn(c, kEpiPpcgRrn, true))) return rc;
+    if ((rc = launch_ppcg_p(c, 0.0, kEpiFinishNoSwitch, true))) return rc;
     return halo(c, TL_FIELD_P, 1);
 }
 
@@ -399,6 +398,7 @@ int solve_timestep(Chunk *c, tl_solve_info_t *info) {
                 if (!rc) rc = launch_ppcg_finish(c);
             } else {
                 rc = run_phase(c, body_ppcg, kItersPpcg, kPhasePpcg, &done);
+                if (!rc && cf.precision == TL_PRECISION_MIXED) rc = launch_ppcg_finish(c);
             }
             break;
         case kPhaseCheby:

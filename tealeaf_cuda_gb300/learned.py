@@ -127,9 +127,9 @@ def parse_decks(text):
 
 # algorithmic HBM bytes per cell of one outer iteration of the headline
 # method's PPCG phase (mixed precision, two fused passes of 5 inner steps):
-# w = Ap with p.w, r.z and r_store (64), rrn (24), u and p (40), r (24),
-# and the two fused passes (36 each)
-PPCG_OUTER_BYTES_PER_CELL = 64 + 24 + 40 + 24 + 2 * 36
+# u, p and w = Ap with p.w (72), r (24), w.z and r.z (24), and the two fused
+# passes (36 each)
+PPCG_OUTER_BYTES_PER_CELL = 72 + 24 + 24 + 2 * 36
 
 
 # ---------------------------------------------------------------- model
