@@ -90,6 +90,7 @@ BYTES_PER_CELL = {
     "field_summary": 32,
     "finalise": 24,
     "ppcg_p": 24,        # read z, p; write p
+    "ppcg_up": 40,       # the last pass of a PPCG solve: read p, u, z; write u, p
     "ppcg_wz": 24,       # read w, r, z (mixed PPCG's two dot products)
     "ppcg_update_r": 48,  # read sd, Kx, Ky, diag, rtemp; write rtemp
     "cheby_calc_u": 24,  # read u, p; write u

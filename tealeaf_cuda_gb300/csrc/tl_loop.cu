@@ -1183,7 +1183,7 @@ int launch_cg_pass2(Chunk *c) {
 }
 
 int launch_cg_finish(Chunk *c, bool ppcg) {
-    return launch_named(c, "cg_up", [&] {
+    return launch_named(c, ppcg ? "ppcg_up" : "cg_up", [&] {
         k_cg_finish<<<c->g.groups, kGroupThreads, 0, c->stream>>>(c->g, cg_args(c, ppcg), c->sc);
     });
 }
