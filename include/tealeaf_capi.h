@@ -272,7 +272,8 @@ int tl_warm_start_features(tl_chunk_t *ch, float *dst);
 
 /* Network kernels on caller-owned device buffers (NHWC BF16 activations with
  * a one-pixel zero halo, [B][H+2][W+2][C]; W a multiple of 16), used by the
- * trainer.  mode 0: out = GELU(conv(in) + b), pre-activation to pre;
+ * trainer.  mode 0: out = GELU(conv(in) + b), pre-activation to
+ * pre (NULL: not stored);
  * 1: out = res + GELU(conv(in) + b); 2: outf[B][H][W] = conv(in)[0] + b[0];
  * 3: out = res + conv(in) (data gradient, weights from tl_nn_pack's wb). */
 int tl_nn_conv(int mode, int cin, int coutp, const void *in, const void *w, const float *bias,

@@ -109,8 +109,9 @@ __global__ void __launch_bounds__(128) k_conv(const bf16 *__restrict__ in, const
             if (MODE == kModeGelu || MODE == kModeGeluRes) {
                 v0 += bias[co];
                 v1 += bias[co + 1];
-                *reinterpret_cast<uint32_t *>(pre + o * COUTP + co) =
-                    pack2(__float2bfloat16(v0), __float2bfloat16(v1));
+                if (pre)
+                    *reinterpret_cast<uint32_t *>(pre + o * COUTP + co) =
+                        pack2(__float2bfloat16(v0), __float2bfloat16(v1));
                 v0 = gelu(v0);
                 v1 = gelu(v1);
             }
@@ -126,12 +127,17 @@ __global__ void __launch_bounds__(128) k_conv(const bf16 *__restrict__ in, const
 }
 
 // ---------------------------------------------------------------------------
-// The same convolution on the 5th-generation tensor cores (tcgen05): a CTA
-// of 4 warps computes a tile of 128 pixels of one row (M = 128) for all
-// COUTP output channels (N), accumulating in tensor memory.
+// The same convolution on the 5th-generation tensor cores (tcgen05).  Pixels are
+// counted over the padded rows, q = y (W + 2) + x: the input of tap (dy, dx) is
+// then q + dy (W + 2) + dx and the output q + (W + 2) + 1, whatever the row, so
+// a tile is any 128 consecutive q (M = 128) for all COUTP output channels (N),
+// and the two columns a row that are no output are all that is computed in
+// vain (1.4 % at W = 144, where tiles of one row's pixels wasted 44 %).
 //
-// Shared memory holds, per kernel row dy, the 130 input pixels the tile's
-// three taps dx = 0, 1, 2 read, in the K-major no-swizzle layout of the MMA
+// A CTA of 4 warps walks tiles: the weights stay in shared memory, and the next
+// tile's input is on its way (cp.async, two buffers) while this one multiplies
+// and is written.  Shared memory holds, per kernel row dy, the 130 input pixels
+// the three taps dx = 0, 1, 2 read, in the K-major no-swizzle layout of the MMA
 // operands: 16-byte core-matrix rows (one pixel, 8 channels), the pixels of
 // an 8-channel chunk contiguous (16 bytes apart) and the chunks kChunkA bytes
 // apart.  The A operand of tap (dy, dx) and 16-channel step kk is that block
@@ -141,9 +147,12 @@ __global__ void __launch_bounds__(128) k_conv(const bf16 *__restrict__ in, const
 // thread issues the 9 * CIN / 16 MMAs (M 128, N COUTP, K 16, BF16 in, FP32
 // accumulate) and commits them to an mbarrier; each warp then reads its 32
 // TMEM lanes (one pixel a lane, one channel a column) and runs the epilogue
-// of k_conv.
+// of k_conv.  Lanes trade half of their chunks with their neighbours before a
+// store, so that every store writes whole 32-byte sectors.
+// What bounds it: HBM for a layer's activations (64 bytes a pixel in and 64 or
+// 128 out).
 constexpr int kTcPix = 128;               // pixels of a tile (MMA M)
-constexpr int kTcRow = kTcPix + 2;        // input pixels a kernel row reads
+constexpr int kTcRow = kTcPix + 2;        // input pixels a kernel row of a tile reads
 constexpr int kChunkA = kTcRow * 16;      // bytes between 8-channel chunks of A
 constexpr int kTmemCols = 32;             // accumulator columns allocated (>= COUTP)
 constexpr long long kTcWaitCycles = 2000000000LL;  // ~1 s: the MMA wait gives up after this
@@ -221,6 +230,32 @@ __device__ __forceinline__ void tmem_load<16>(uint32_t taddr, float (&v)[16]) {
     for (int k = 0; k < 16; ++k) v[k] = __uint_as_float(r[k]);
 }
 
+template <int CIN, int COUTP>
+constexpr int conv_tc_smem() {
+    return 2 * 3 * (CIN / 8) * kChunkA + 9 * (CIN / 8) * COUTP * 16;
+}
+
+// store 8 channels a lane of COUTP, `at` the lane's pixel: two chunks of the
+// lane's own pixel become one chunk of each of the pair's pixels
+template <int COUTP>
+__device__ __forceinline__ void store_chunks(bf16 *dst, long long at, int chunk, const uint32_t (&c0)[4],
+                                             const uint32_t (&c1)[4], bool mine, bool partner, int lane) {
+    const bool odd = lane & 1;
+    uint32_t even_px[4], odd_px[4];  // this lane's chunk of the pair's even and odd pixel
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? c0[e] : c1[e], 1);
+        even_px[e] = odd ? got : c0[e];
+        odd_px[e] = odd ? c1[e] : got;
+    }
+    const int c = chunk + (odd ? 1 : 0);
+    const long long e0 = odd ? at - 1 : at;
+    if (odd ? partner : mine)
+        *reinterpret_cast<uint4 *>(dst + e0 * COUTP + 8 * c) = make_uint4(even_px[0], even_px[1], even_px[2], even_px[3]);
+    if (odd ? mine : partner)
+        *reinterpret_cast<uint4 *>(dst + (e0 + 1) * COUTP + 8 * c) = make_uint4(odd_px[0], odd_px[1], odd_px[2], odd_px[3]);
+}
+
 template <int CIN, int COUTP, int MODE>
 __global__ void __launch_bounds__(128) k_conv_tc(const bf16 *__restrict__ in, const bf16 *__restrict__ wt,
                                                  const float *__restrict__ bias,
@@ -231,18 +266,14 @@ __global__ void __launch_bounds__(128) k_conv_tc(const bf16 *__restrict__ in, co
     constexpr int CA = CIN / 8;                    // 8-channel chunks of a pixel
     constexpr int CHUNK_B = COUTP * 16;            // bytes between chunks of the weights
     constexpr int A_BYTES = 3 * CA * kChunkA;      // three kernel rows
-    constexpr int B_BYTES = 9 * CA * CHUNK_B;      // nine taps
-    __shared__ __align__(1024) unsigned char sa[A_BYTES];
-    __shared__ __align__(1024) unsigned char sb[B_BYTES];
+    extern __shared__ __align__(128) unsigned char conv_smem[];
+    unsigned char *const sb = conv_smem + 2 * A_BYTES;
     __shared__ __align__(8) uint64_t mbar;
     __shared__ uint32_t tmem_slot;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int tiles_x = (W + kTcPix - 1) / kTcPix;
-    const long long task = blockIdx.x;  // (b, y, tile)
-    const int b = (int)(task / ((long long)H * tiles_x));
-    const int rem = (int)(task % ((long long)H * tiles_x));
-    const int y = rem / tiles_x, x0 = (rem % tiles_x) * kTcPix;
-    const long long Wp = W + 2;
+    const int Wp = W + 2;
+    const long long npix = (long long)H * Wp, in_pix = (long long)(H + 2) * Wp;  // q range, padded image
+    const long long per_image = (npix + kTcPix - 1) / kTcPix, tiles = per_image * B;
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -255,103 +286,134 @@ __global__ void __launch_bounds__(128) k_conv_tc(const bf16 *__restrict__ in, co
         // the tensor cores arrive on it: make the initialisation visible to them
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    // A: padded input rows y + dy, pixels x0 .. x0 + 129, 16 bytes a load;
-    // pixels past the padded row read as zero (partial last tile)
-    const bf16 *img = in + (long long)b * (H + 2) * Wp * CIN;
-    for (int k = tid; k < 3 * kTcRow * CA; k += 128) {
-        const int c = k % CA, j = (k / CA) % kTcRow, dy = k / (CA * kTcRow);
-        uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (x0 + j < Wp) v = *reinterpret_cast<const uint4 *>(img + ((long long)(y + dy) * Wp + x0 + j) * CIN + 8 * c);
-        *reinterpret_cast<uint4 *>(sa + (dy * CA + c) * kChunkA + j * 16) = v;
-    }
+    // A: padded pixels q0 + dy Wp + 0..129, 16 bytes a copy; pixels past the
+    // image read as zero (last tile)
+    auto stage = [&](long long t, int buf) {
+        const int b = (int)(t / per_image);
+        const long long q0 = (t - b * per_image) * kTcPix;
+        const bf16 *img = in + (long long)b * in_pix * CIN;
+        const uint32_t dst = smem_addr(conv_smem) + buf * A_BYTES;
+        for (int k = tid; k < 3 * kTcRow * CA; k += 128) {
+            const int c = k % CA, j = (k / CA) % kTcRow, dy = k / (CA * kTcRow);
+            const long long s = q0 + (long long)dy * Wp + j;
+            const bool ok = s < in_pix;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + (dy * CA + c) * kChunkA + j * 16),
+                         "l"(img + (ok ? s : 0) * CIN + 8 * c), "r"(ok ? 16 : 0));
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    long long t = blockIdx.x;
+    if (t < tiles) stage(t, 0);
     // B: weights [tap][cout][cin]
     for (int k = tid; k < 9 * COUTP * CA; k += 128) {
         const int c = k % CA, co = (k / CA) % COUTP, tap = k / (CA * COUTP);
         const uint4 v = *reinterpret_cast<const uint4 *>(wt + ((long long)tap * COUTP + co) * CIN + 8 * c);
         *reinterpret_cast<uint4 *>(sb + (tap * CA + c) * CHUNK_B + co * 16) = v;
     }
-    // the MMAs read shared memory through the async proxy
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = tmem_slot;
     const uint32_t bar = smem_addr(&mbar);
-    if (tid == 0) {
-        constexpr uint32_t idesc = mma_idesc(kTcPix, COUTP);
-        const uint32_t a0 = smem_addr(sa), b0 = smem_addr(sb);
-#pragma unroll
-        for (int tap = 0; tap < 9; ++tap) {
-            const int dy = tap / 3, dx = tap % 3;
-#pragma unroll
-            for (int kk = 0; kk < CIN / 16; ++kk) {
-                const uint64_t ad = mma_desc(a0 + (dy * CA + 2 * kk) * kChunkA + dx * 16, kChunkA, 128);
-                const uint64_t bd = mma_desc(b0 + (tap * CA + 2 * kk) * CHUNK_B, CHUNK_B, 128);
-                const uint32_t acc = (tap | kk) != 0 ? 1u : 0u;
-                asm volatile(
-                    "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
-                    "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
-            }
+    uint32_t tmem = 0, phase = 0;
+    bool ok = true;
+    for (int buf = 0; t < tiles; t += gridDim.x, buf ^= 1, phase ^= 1) {
+        if (t + gridDim.x < tiles) {
+            stage(t + gridDim.x, buf ^ 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
         }
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-                     : "memory");
-    }
-    // warp-uniform outcome: tcgen05.ld below is executed by whole warps
-    const bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(bar, 0));
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (!ok) {
-        // the accumulator never became ready: flag it, wait once more
-        // (bounded) for the MMAs in flight, release the columns and leave
-        if (lane == 0) atomicExch(&g_conv_tc_error, 1);
-        mbar_wait_bounded(bar, 0);
-    } else {
+        // the MMAs read shared memory through the async proxy
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncthreads();
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        tmem = tmem_slot;
+        if (tid == 0) {
+            constexpr uint32_t idesc = mma_idesc(kTcPix, COUTP);
+            const uint32_t a0 = smem_addr(conv_smem) + buf * A_BYTES, b0 = smem_addr(sb);
+#pragma unroll
+            for (int tap = 0; tap < 9; ++tap) {
+                const int dy = tap / 3, dx = tap % 3;
+#pragma unroll
+                for (int kk = 0; kk < CIN / 16; ++kk) {
+                    const uint64_t ad = mma_desc(a0 + (dy * CA + 2 * kk) * kChunkA + dx * 16, kChunkA, 128);
+                    const uint64_t bd = mma_desc(b0 + (tap * CA + 2 * kk) * CHUNK_B, CHUNK_B, 128);
+                    const uint32_t acc = (tap | kk) != 0 ? 1u : 0u;
+                    asm volatile(
+                        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+                        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
+                        "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
+                }
+            }
+            asm volatile(
+                "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
+                : "memory");
+        }
+        // this lane's pixel, while the tensor cores work
+        const int b = (int)(t / per_image);
+        const long long q = (t - b * per_image) * kTcPix + 32 * warp + lane;
+        const int x = (int)(q % Wp), y = (int)(q / Wp);
+        const bool valid = q < npix && x < W;
+        const bool pvalid = __shfl_xor_sync(0xffffffffu, (int)valid, 1) != 0;
+        const long long o = (long long)b * in_pix + q + Wp + 1;
+        // warp-uniform outcome: tcgen05.ld below is executed by whole warps
+        ok = __all_sync(0xffffffffu, mbar_wait_bounded(bar, phase));
+        if (!__syncthreads_and(ok)) {
+            // the accumulator never became ready: flag it, wait once more
+            // (bounded) for the MMAs in flight, release the columns and leave
+            if (lane == 0) atomicExch(&g_conv_tc_error, 1);
+            mbar_wait_bounded(bar, phase);
+            break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         // warp w holds TMEM lanes 32w..32w+31: pixel m = 32 w + lane
         float acc[COUTP];
         tmem_load<COUTP>(tmem + ((uint32_t)(32 * warp) << 16), acc);
-        const int px = x0 + 32 * warp + lane;
-        if (px < W) {
-            const long long o = ((long long)b * (H + 2) + y + 1) * Wp + px + 1;
-            if (MODE == kModeHead) {
-                outf[((long long)b * H + y) * W + px] = acc[0] + bias[0];
-            } else {
+        if (MODE == kModeHead) {
+            if (valid) outf[((long long)b * H + y) * W + x] = acc[0] + bias[0];
+        } else {
 #pragma unroll
-                for (int q = 0; q < COUTP / 8; ++q) {
-                    float v[8];
+            for (int q2 = 0; q2 < COUTP / 8; q2 += 2) {
+                uint32_t pk[2][4];
+                if (MODE == kModeGelu || MODE == kModeGeluRes) {
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) v[e] = acc[8 * q + e];
-                    if (MODE == kModeGelu || MODE == kModeGeluRes) {
-                        uint32_t pk[4];
+                    for (int h = 0; h < 2; ++h)
 #pragma unroll
-                        for (int e = 0; e < 8; ++e) v[e] += bias[8 * q + e];
+                        for (int e = 0; e < 4; ++e) {
+                            float &v0 = acc[8 * (q2 + h) + 2 * e], &v1 = acc[8 * (q2 + h) + 2 * e + 1];
+                            v0 += bias[8 * (q2 + h) + 2 * e];
+                            v1 += bias[8 * (q2 + h) + 2 * e + 1];
+                            pk[h][e] = pack2(__float2bfloat16(v0), __float2bfloat16(v1));
+                            v0 = gelu(v0);
+                            v1 = gelu(v1);
+                        }
+                    if (pre) store_chunks<COUTP>(pre, o, q2, pk[0], pk[1], valid, pvalid, lane);
+                }
+                if ((MODE == kModeGeluRes || MODE == kModeLinear) && res && valid) {
 #pragma unroll
-                        for (int e = 0; e < 4; ++e)
-                            pk[e] = pack2(__float2bfloat16(v[2 * e]), __float2bfloat16(v[2 * e + 1]));
-                        *reinterpret_cast<uint4 *>(pre + o * COUTP + 8 * q) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) v[e] = gelu(v[e]);
-                    }
-                    if ((MODE == kModeGeluRes || MODE == kModeLinear) && res) {
-                        const uint4 rv = *reinterpret_cast<const uint4 *>(res + o * COUTP + 8 * q);
+                    for (int h = 0; h < 2; ++h) {
+                        const uint4 rv = *reinterpret_cast<const uint4 *>(res + o * COUTP + 8 * (q2 + h));
                         const uint32_t rw[4] = {rv.x, rv.y, rv.z, rv.w};
 #pragma unroll
                         for (int e = 0; e < 4; ++e) {
-                            v[2 * e] += __bfloat162float(__ushort_as_bfloat16((unsigned short)(rw[e] & 0xFFFFu)));
-                            v[2 * e + 1] += __bfloat162float(__ushort_as_bfloat16((unsigned short)(rw[e] >> 16)));
+                            acc[8 * (q2 + h) + 2 * e] += __uint_as_float(rw[e] << 16);
+                            acc[8 * (q2 + h) + 2 * e + 1] += __uint_as_float(rw[e] & 0xFFFF0000u);
                         }
                     }
-                    uint32_t pk[4];
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) pk[e] = pack2(__float2bfloat16(v[2 * e]), __float2bfloat16(v[2 * e + 1]));
-                    *reinterpret_cast<uint4 *>(out + o * COUTP + 8 * q) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
                 }
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        pk[h][e] = pack2(__float2bfloat16(acc[8 * (q2 + h) + 2 * e]),
+                                         __float2bfloat16(acc[8 * (q2 + h) + 2 * e + 1]));
+                store_chunks<COUTP>(out, o, q2, pk[0], pk[1], valid, pvalid, lane);
             }
         }
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_slot), "r"(kTmemCols));
 }
 
 // dpre = dh * gelu'(pre) over the interior (halo left at zero).  Bound by HBM
@@ -643,10 +705,14 @@ template <int CIN, int COUTP, int MODE>
 int launch_conv(const void *in, const void *w, const float *bias, const void *res, void *out, void *pre,
                 float *outf, int B, int H, int W, cudaStream_t s) {
     if (g_conv_tcgen05) {
-        const long long tiles = (long long)B * H * ((W + kTcPix - 1) / kTcPix);
-        k_conv_tc<CIN, COUTP, MODE><<<(unsigned)tiles, 128, 0, s>>>((const bf16 *)in, (const bf16 *)w, bias,
-                                                                    (const bf16 *)res, (bf16 *)out, (bf16 *)pre,
-                                                                    outf, B, H, W);
+        constexpr int bytes = conv_tc_smem<CIN, COUTP>();
+        const cudaError_t e = cudaFuncSetAttribute(k_conv_tc<CIN, COUTP, MODE>,
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        if (e != cudaSuccess) return cuda_fail(e, "conv shared memory");
+        const long long tiles = (((long long)H * (W + 2) + kTcPix - 1) / kTcPix) * B;
+        const long long ctas = 152 * 3;  // 3 CTAs of 68 KB a multiprocessor
+        k_conv_tc<CIN, COUTP, MODE><<<(unsigned)(tiles < ctas ? tiles : ctas), 128, bytes, s>>>(
+            (const bf16 *)in, (const bf16 *)w, bias, (const bf16 *)res, (bf16 *)out, (bf16 *)pre, outf, B, H, W);
     } else {
         const long long tasks = (long long)B * H * (W / 16);
         const unsigned grid = (unsigned)((tasks + 3) / 4);

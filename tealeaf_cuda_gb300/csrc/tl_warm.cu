@@ -97,7 +97,7 @@ struct Warm {
     float *params;              // FP32 master copy on the device
     bf16 *wf[kLayers];          // BF16 [9][coutp][cin]
     float *bias[kLayers];
-    bf16 *x, *h0, *h1, *pre;    // activations [1][ny+2][nxp+2][C]
+    bf16 *x, *h0, *h1;          // activations [1][ny+2][nxp+2][C]
     float *y;                   // [ny][nxp] predicted du / max|r0|
     int nxp;
     std::vector<void *> model_allocs;
@@ -378,11 +378,11 @@ int net_direction(Chunk *c, Warm *w) {
                                     c->ky, w->scale, c->dt, w->x, w->nxp, nullptr);
     if ((rc = launched(c, "features launch"))) return rc;
     bf16 *h = w->h0, *hn = w->h1;
-    if ((rc = tl_nn_conv(0, 16, 32, w->x, w->wf[0], w->bias[0], nullptr, h, w->pre, nullptr, 1, c->ny,
+    if ((rc = tl_nn_conv(0, 16, 32, w->x, w->wf[0], w->bias[0], nullptr, h, nullptr, nullptr, 1, c->ny,
                          w->nxp, s)))
         return rc;
     for (int l = 1; l < 5; ++l) {
-        if ((rc = tl_nn_conv(1, 32, 32, h, w->wf[l], w->bias[l], h, hn, w->pre, nullptr, 1, c->ny, w->nxp, s)))
+        if ((rc = tl_nn_conv(1, 32, 32, h, w->wf[l], w->bias[l], h, hn, nullptr, nullptr, 1, c->ny, w->nxp, s)))
             return rc;
         bf16 *t = h;
         h = hn;
@@ -543,7 +543,7 @@ int warm_set_model(Chunk *c, const float *params, long long n) {
     const size_t px = (size_t)(c->ny + 2) * (w->nxp + 2);
     if ((rc = dmalloc(L, &p, sizeof(bf16) * px * 16, s))) return rc;
     w->x = (bf16 *)p;
-    bf16 **acts[3] = {&w->h0, &w->h1, &w->pre};
+    bf16 **acts[2] = {&w->h0, &w->h1};
     for (bf16 **a : acts) {
         if ((rc = dmalloc(L, &p, sizeof(bf16) * px * 32, s))) return rc;
         *a = (bf16 *)p;

@@ -1,5 +1,5 @@
-"""The network's weight and bias gradients and the GELU gradient at the sizes
-where their kernels' tiles end: one 16-pixel group, segments of 64 pixels and
+"""The network's convolution, its weight and bias gradients and the GELU gradient
+at the sizes where their kernels' tiles end: one 16-pixel group, segments of 64 pixels and
 their remainders, partial buffers with room for one block only, buffers that
 are not 16-byte aligned.
 
@@ -78,3 +78,39 @@ def test_gelu_gradient_wide_and_narrow_loads_agree(ch, shape, offset):
     torch.cuda.synchronize()
     assert torch.equal(got[:, 1:-1, 1:-1], want[:, 1:-1, 1:-1])
     assert float(got[:, 0].abs().sum() + got[:, :, 0].abs().sum()) == 0.0
+
+
+@pytest.mark.parametrize("cin,cout,mode", [(16, 32, 0), (32, 32, 1), (32, 16, 2), (16, 32, 3), (32, 32, 3)])
+@pytest.mark.parametrize("shape", [(1, 1, 16), (1, 7, 16), (2, 3, 112), (1, 2, 128), (3, 160, 144)])
+@pytest.mark.parametrize("with_pre", [True, False])
+def test_tensor_memory_conv_tiles(cin, cout, mode, shape, with_pre):
+    """tiles of 128 pixels across the rows' ends and the image's, one and several a thread block, against the
+    warp-level kernel: BF16 outputs within one rounding (2^-7), the FP32 head within its sum's rounding; the
+    halo and what lies behind the buffers stay as they are"""
+    torch = pytest.importorskip("torch")
+    lib = tl.load()
+    lib.tl_nn_set_conv_kernel.argtypes = [C.c_int]
+    B, H, W = shape
+    gen = torch.Generator(device="cuda").manual_seed(3 * cin + cout + mode + W)
+    x, res = _field(torch, shape, cin, 0, gen), _field(torch, shape, cout, 0, gen)
+    w = (0.2 * torch.randn((9, cout, cin), generator=gen, device="cuda")).bfloat16()
+    bias = 0.1 * torch.randn(cout, generator=gen, device="cuda")
+    got = {}
+    for tc in (1, 0):
+        n = B * (H + 2) * (W + 2) * cout
+        out, pre = (torch.full((n + 256,), 3.0, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+        head = torch.full((B * H * W + 64,), 5.0, device="cuda")
+        out[:n], pre[:n] = 0, 0
+        assert lib.tl_nn_set_conv_kernel(tc) == 0
+        rc = lib.tl_nn_conv(mode, cin, cout, _p(x), _p(w), _p(bias), _p(res) if mode in (1, 3) else None, _p(out),
+                            _p(pre) if with_pre else None, _p(head), B, H, W, None)
+        lib.tl_nn_set_conv_kernel(1)
+        assert rc == 0, tl.last_error()
+        torch.cuda.synchronize()
+        assert lib.tl_nn_conv_status() == 0, tl.last_error()
+        assert bool((out[n:] == 3.0).all() and (pre[n:] == 3.0).all() and (head[B * H * W:] == 5.0).all())
+        got[tc] = [t[:n].float().view(B, H + 2, W + 2, cout) for t in (out, pre)] + [head[:B * H * W]]
+        for t in got[tc][:2]:
+            assert float(t[:, 0].abs().sum() + t[:, -1].abs().sum() + t[:, :, 0].abs().sum() + t[:, :, -1].abs().sum()) == 0
+    for a, b in zip(got[1], got[0]):
+        assert bool(((a - b).abs() <= 2.0 ** -7 * b.abs() + 1e-5).all())
