@@ -423,13 +423,15 @@ __global__ void __launch_bounds__(128) k_conv_tc(const bf16 *__restrict__ in, co
 template <int V>
 __global__ void k_gelu_back(const bf16 *__restrict__ dh, const bf16 *__restrict__ pre,
                             bf16 *__restrict__ dpre, int C, int B, int H, int W) {
-    const int CV = C / V;
-    const long long rows = (long long)B * H;
-    const int per_row = W * CV;
-    for (long long row = blockIdx.x; row < rows; row += gridDim.x) {
-        const int y = (int)(row % H), b = (int)(row / H);
-        const long long o0 = (((long long)b * (H + 2) + y + 1) * (W + 2) + 1) * C;
-        for (int k = threadIdx.x; k < per_row; k += blockDim.x) {
+    const int per_row = W * (C / V);
+    const long long n = (long long)B * H * per_row;
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
+        // (32-bit division where the count allows)
+        const long long row = n >> 32 ? t / per_row : (long long)((unsigned int)t / (unsigned int)per_row);
+        const int k = (int)(t - row * per_row);
+        const int b = (int)(row / H), y = (int)(row - (long long)b * H);
+        {
+            const long long o0 = (((long long)b * (H + 2) + y + 1) * (W + 2) + 1) * C;
             const long long o = o0 + (long long)k * V;
             if constexpr (V == 8) {
                 const uint4 d4 = *reinterpret_cast<const uint4 *>(dh + o);
@@ -455,9 +457,10 @@ __global__ void k_gelu_back(const bf16 *__restrict__ dh, const bf16 *__restrict_
 // A contraction over the pixels with M = co and N = ci of 16 or 32 a tap, below
 // the 64 rows of a tensor-memory MMA, so it runs on mma.sync (M = co, N = ci,
 // K = 16 pixels), one warp a tap; warp 4 also multiplies dpre by a column of
-// ones, which is db.  A CTA walks segments of kWgSeg pixels of a row (a
-// grid-stride loop over the segments of all rows): it stages the segment's
-// dpre and the three input rows its taps read in shared memory (16-byte
+// ones, which is db.  A CTA walks segments of kWgSeg pixels counted over the
+// padded rows as k_conv_tc counts them (a grid-stride loop over the segments
+// of all images; dpre enters as 0 for the two columns a row that are no pixels):
+// it stages the segment's dpre and the input that its taps read in shared memory (16-byte
 // cp.async, two buffers: the next segment loads while this one multiplies),
 // pixels kWgStride bytes apart so that ldmatrix reads eight pixels' 16 bytes
 // without bank conflicts, and takes both operands transposed by
@@ -475,14 +478,18 @@ __device__ __forceinline__ void ldsm4t(uint32_t (&r)[4], uint32_t addr) {
                  : "r"(addr));
 }
 
-// eight channels to shared memory; buffers that are not 16-byte aligned go
-// through registers
-__device__ __forceinline__ void stage16(uint32_t dst, const bf16 *src, bool aligned) {
+// eight channels to shared memory, or zeros; buffers that are not 16-byte
+// aligned go through registers
+__device__ __forceinline__ void stage16(uint32_t dst, const bf16 *src, bool ok, const bf16 *any, bool aligned) {
     if (aligned) {
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src));
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(ok ? src : any), "r"(ok ? 16 : 0));
     } else {
-        asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(dst), "r"(pack2(src[0], src[1])),
-                     "r"(pack2(src[2], src[3])), "r"(pack2(src[4], src[5])), "r"(pack2(src[6], src[7]))
+        uint32_t v[4] = {0u, 0u, 0u, 0u};
+        if (ok) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[e] = pack2(src[2 * e], src[2 * e + 1]);
+        }
+        asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(dst), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3])
                      : "memory");
     }
 }
@@ -505,28 +512,30 @@ __global__ void __launch_bounds__(kWgThreads) k_wgrad(const bf16 *__restrict__ d
 #pragma unroll
         for (int j = 0; j < NT; ++j) acc[i][j][0] = acc[i][j][1] = acc[i][j][2] = acc[i][j][3] = 0.f;
     }
-    const int segs = (W + kWgSeg - 1) / kWgSeg;
-    const long long tasks = (long long)B * H * segs;
-    const long long Wp = W + 2;
+    const int Wp = W + 2;
+    const long long npix = (long long)H * Wp, in_pix = (long long)(H + 2) * Wp;
+    const long long segs = (npix + kWgSeg - 1) / kWgSeg, tasks = segs * B;
     const bool aligned = (((uintptr_t)dpre | (uintptr_t)in) & 15) == 0;
-    auto stage = [&](long long q, int buf) {
-        const int sx = (int)(q % segs);
-        const long long row = q / segs;
-        const int y = (int)(row % H), b = (int)(row / H);
-        const int x0 = sx * kWgSeg, np = min(kWgSeg, W - x0);
+    auto stage = [&](long long t, int buf) {
+        const int b = (int)(t / segs);
+        const long long q0 = (t - b * segs) * kWgSeg;
         const uint32_t base = sm0 + buf * BUF;
         constexpr int CI8 = CIN / 8, CO8 = COUTP / 8;
-        const bf16 *ip = in + (((long long)b * (H + 2) + y) * Wp + x0) * CIN;
+        const bf16 *ip = in + (long long)b * in_pix * CIN;
         for (int k = tid; k < 3 * (kWgSeg + 2) * CI8; k += kWgThreads) {
             const int c = k % CI8, j = (k / CI8) % (kWgSeg + 2), r = k / (CI8 * (kWgSeg + 2));
-            if (j < np + 2) 
-                stage16(base + (r * (kWgSeg + 2) + j) * SI + c * 16, ip + (r * Wp + j) * CIN + 8 * c, aligned);
+            const long long s = q0 + (long long)r * Wp + j;
+            stage16(base + (r * (kWgSeg + 2) + j) * SI + c * 16, ip + s * CIN + 8 * c, s < in_pix, ip, aligned);
         }
-        const bf16 *dp = dpre + (((long long)b * (H + 2) + y + 1) * Wp + x0 + 1) * COUTP;
+        const bf16 *dp = dpre + (long long)b * in_pix * COUTP;
+        const int x0 = (int)(q0 % Wp);
         for (int k = tid; k < kWgSeg * CO8; k += kWgThreads) {
             const int c = k % CO8, j = k / CO8;
-            if (j < np) 
-                stage16(base + 3 * (kWgSeg + 2) * SI + j * SO + c * 16, dp + (long long)j * COUTP + 8 * c, aligned);
+            const long long q = q0 + j;
+            int x = x0 + j;
+            while (x >= Wp) x -= Wp;
+            stage16(base + 3 * (kWgSeg + 2) * SI + j * SO + c * 16, dp + (q + Wp + 1) * COUTP + 8 * c,
+                    q < npix && x < W, dp, aligned);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
@@ -541,10 +550,10 @@ __global__ void __launch_bounds__(kWgThreads) k_wgrad(const bf16 *__restrict__ d
             asm volatile("cp.async.wait_group 0;" ::: "memory");
         }
         __syncthreads();
-        const int np = min(kWgSeg, W - (int)(q % segs) * kWgSeg);
         const uint32_t sin = sm0 + buf * BUF + (dy * (kWgSeg + 2) + dx) * SI;
         const uint32_t sdp = sm0 + buf * BUF + 3 * (kWgSeg + 2) * SI;
-        for (int p0 = 0; p0 < np; p0 += 16) {
+#pragma unroll 2
+        for (int p0 = 0; p0 < kWgSeg; p0 += 16) {
             // 8 x 8 blocks [pixel][channel], transposed by the load: lane l
             // addresses pixel l % 8 (+8 by bit 3 or 4) of its block
             uint32_t a[MT][4], b[NT / 2][4];
@@ -791,7 +800,7 @@ long long tl_nn_wgrad_partial_floats(int cin, int coutp, int B, int H, int W, in
 
 // The partial buffer holds one [9][coutp][cin] block per groups_per_cta
 // 16-pixel groups (tl_nn_wgrad_partial_floats); the kernel needs far fewer:
-// two CTAs a multiprocessor, and behind their blocks the CTAs' db partials
+// three CTAs a multiprocessor, and behind their blocks the CTAs' db partials
 // (one block less than the buffer holds leaves them room).
 int tl_nn_wgrad(const void *dpre, const void *in, int cin, int coutp, float *partial, float *dw, float *db,
                 int B, int H, int W, int groups_per_cta, void *stream) {
@@ -802,9 +811,9 @@ int tl_nn_wgrad(const void *dpre, const void *in, int cin, int coutp, float *par
     }
     const long long groups = (long long)B * H * (W / 16);
     const long long blocks = (groups + groups_per_cta - 1) / groups_per_cta;  // room in `partial`
-    const long long tasks = (long long)B * H * ((W + kWgSeg - 1) / kWgSeg);
+    const long long tasks = (((long long)H * (W + 2) + kWgSeg - 1) / kWgSeg) * B;
     const int n = 9 * cin * coutp;
-    long long ctas = tasks < 304 ? tasks : 304;
+    long long ctas = tasks < 152 * 3 ? tasks : 152 * 3;
     const bool bias_here = db && blocks >= 2;
     if (bias_here) {
         // ctas blocks and ctas * coutp floats: floor(blocks * n / (n + coutp))
