@@ -293,12 +293,22 @@ __global__ void __launch_bounds__(128) k_conv_tc(const bf16 *__restrict__ in, co
         const long long q0 = (t - b * per_image) * kTcPix;
         const bf16 *img = in + (long long)b * in_pix * CIN;
         const uint32_t dst = smem_addr(conv_smem) + buf * A_BYTES;
-        for (int k = tid; k < 3 * kTcRow * CA; k += 128) {
-            const int c = k % CA, j = (k / CA) % kTcRow, dy = k / (CA * kTcRow);
-            const long long s = q0 + (long long)dy * Wp + j;
-            const bool ok = s < in_pix;
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + (dy * CA + c) * kChunkA + j * 16),
-                         "l"(img + (ok ? s : 0) * CIN + 8 * c), "r"(ok ? 16 : 0));
+        // a thread copies chunk tid % CA of every 128 / CA-th pixel
+        constexpr int PX = 128 / CA;
+        const int c = tid % CA, j0 = tid / CA;
+        const bf16 *src = img + (q0 + j0) * CIN + 8 * c;
+        const bool inside = q0 + 2LL * Wp + kTcRow <= in_pix;  // all but an image's last tiles
+#pragma unroll
+        for (int dy = 0; dy < 3; ++dy) {
+            const uint32_t d0 = dst + (dy * CA + c) * kChunkA + j0 * 16;
+            const bf16 *s0 = src + (long long)dy * Wp * CIN;
+#pragma unroll
+            for (int i = 0; i < (kTcRow + PX - 1) / PX; ++i) {
+                if ((i + 1) * PX > kTcRow && j0 + i * PX >= kTcRow) break;
+                const bool ok = inside || q0 + (long long)dy * Wp + j0 + i * PX < in_pix;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d0 + i * PX * 16),
+                             "l"(ok ? s0 + i * PX * CIN : img), "r"(ok ? 16 : 0));
+            }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
@@ -354,6 +364,11 @@ __global__ void __launch_bounds__(128) k_conv_tc(const bf16 *__restrict__ in, co
         const bool valid = q < npix && x < W;
         const bool pvalid = __shfl_xor_sync(0xffffffffu, (int)valid, 1) != 0;
         const long long o = (long long)b * in_pix + q + Wp + 1;
+        uint4 rv[COUTP / 8];
+        const bool add = (MODE == kModeGeluRes || MODE == kModeLinear) && res;
+#pragma unroll
+        for (int h = 0; h < COUTP / 8; ++h)
+            if (add && valid) rv[h] = *reinterpret_cast<const uint4 *>(res + o * COUTP + 8 * h);
         // warp-uniform outcome: tcgen05.ld below is executed by whole warps
         ok = __all_sync(0xffffffffu, mbar_wait_bounded(bar, phase));
         if (!__syncthreads_and(ok)) {
@@ -387,11 +402,10 @@ __global__ void __launch_bounds__(128) k_conv_tc(const bf16 *__restrict__ in, co
                         }
                     if (pre) store_chunks<COUTP>(pre, o, q2, pk[0], pk[1], valid, pvalid, lane);
                 }
-                if ((MODE == kModeGeluRes || MODE == kModeLinear) && res && valid) {
+                if (add && valid) {
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
-                        const uint4 rv = *reinterpret_cast<const uint4 *>(res + o * COUTP + 8 * (q2 + h));
-                        const uint32_t rw[4] = {rv.x, rv.y, rv.z, rv.w};
+                        const uint32_t rw[4] = {rv[q2 + h].x, rv[q2 + h].y, rv[q2 + h].z, rv[q2 + h].w};
 #pragma unroll
                         for (int e = 0; e < 4; ++e) {
                             acc[8 * (q2 + h) + 2 * e] += __uint_as_float(rw[e] << 16);
@@ -522,20 +536,26 @@ __global__ void __launch_bounds__(kWgThreads) k_wgrad(const bf16 *__restrict__ d
         const uint32_t base = sm0 + buf * BUF;
         constexpr int CI8 = CIN / 8, CO8 = COUTP / 8;
         const bf16 *ip = in + (long long)b * in_pix * CIN;
-        for (int k = tid; k < 3 * (kWgSeg + 2) * CI8; k += kWgThreads) {
-            const int c = k % CI8, j = (k / CI8) % (kWgSeg + 2), r = k / (CI8 * (kWgSeg + 2));
-            const long long s = q0 + (long long)r * Wp + j;
-            stage16(base + (r * (kWgSeg + 2) + j) * SI + c * 16, ip + s * CIN + 8 * c, s < in_pix, ip, aligned);
+        static_assert(kWgThreads / CI8 >= kWgSeg + 2 && kWgThreads / CO8 >= kWgSeg, "one copy a thread and row");
+        {
+            const int c = tid % CI8, j = tid / CI8;
+            if (j < kWgSeg + 2) {
+                const long long s = q0 + j;
+                const bf16 *src = ip + s * CIN + 8 * c;
+#pragma unroll
+                for (int r = 0; r < 3; ++r)
+                    stage16(base + (r * (kWgSeg + 2) + j) * SI + c * 16, src + (long long)r * Wp * CIN,
+                            s + (long long)r * Wp < in_pix, ip, aligned);
+            }
         }
         const bf16 *dp = dpre + (long long)b * in_pix * COUTP;
-        const int x0 = (int)(q0 % Wp);
-        for (int k = tid; k < kWgSeg * CO8; k += kWgThreads) {
-            const int c = k % CO8, j = k / CO8;
-            const long long q = q0 + j;
-            int x = x0 + j;
-            while (x >= Wp) x -= Wp;
-            stage16(base + 3 * (kWgSeg + 2) * SI + j * SO + c * 16, dp + (q + Wp + 1) * COUTP + 8 * c,
-                    q < npix && x < W, dp, aligned);
+        {
+            const int c = tid % CO8, j = tid / CO8;
+            if (j < kWgSeg) {
+                const long long q = q0 + j;
+                stage16(base + 3 * (kWgSeg + 2) * SI + j * SO + c * 16, dp + (q + Wp + 1) * COUTP + 8 * c,
+                        q < npix && (int)(q % Wp) < W, dp, aligned);
+            }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
