@@ -286,6 +286,7 @@ int mixed_ppcg_inner(Chunk *c);    // PPCG inner steps in FP32, z in FP64
 // r -= alpha w, then the inner steps; *did_rrn tells whether the last pass also
 // summed (r - r_store).z
 int mixed_ppcg_ur_inner(Chunk *c, bool *did_rrn);
+int launch_mixed_ppcg_loop(Chunk *c);  // many outer iterations in one launch (tl_mixed_loop.cu)
 void drop_graphs(Chunk *c);        // after a change that captured graphs depend on
 constexpr int kFusedMax = 5;           // most FP32 PPCG inner steps fused into one pass
 constexpr int kInnerFuseDefault = 5;

@@ -25,23 +25,12 @@
 #include <chrono>
 #include <type_traits>
 
-#include "tl_internal.cuh"
+#include "tl_mixed.cuh"
 #include "tl_device.cuh"
 
 namespace tl {
 
 namespace {
-
-struct Mixed {
-    float *kx, *ky, *mi, *d, *r, *p, *w, *z;
-    float *sd[2], *rtemp, *utemp, *cp, *bfp;   // PPCG inner steps
-    float *rtemp2;                             // second rtemp of the fused inner passes
-    double *fpartials;                         // one per CTA of a fused inner pass
-    double *partials;            // one per CTA of the vectorised kernels
-    unsigned int *counter;
-    int vtiles_x, vtiles;        // tiles of the vectorised kernels
-    std::vector<void *> allocs;
-};
 
 // Vectorised FP32 kernels of the inner iteration: a lane owns four adjacent
 // columns (one float4, 16-byte aligned: the interior starts on a 128-byte
@@ -217,14 +206,6 @@ __device__ __forceinline__ void st4(float *__restrict__ f, int64_t i, float4 v, 
         if (nv > 1) f[i + 1] = v.y;
         if (nv > 2) f[i + 2] = v.z;
     }
-}
-
-__device__ __forceinline__ float cell_apply(float c, float n, float s, float w, float e, float kyn,
-                                            float kyc, float kxe, float kxc) {
-    float v = fmaf(kyn, c - n, c);
-    v = fmaf(kyc, c - s, v);
-    v = fmaf(kxe, c - e, v);
-    return fmaf(kxc, c - w, v);
 }
 
 // block + grid reduction of a compensated sum; the last CTA runs the inner
@@ -1340,8 +1321,6 @@ struct BodyPpUr {
             }
     }
 };
-
-Mixed *mixed_of(Chunk *c) { return (Mixed *)c->mixed; }
 
 // the FP32 state; on failure nothing of it is kept (mixed_alloc frees it)
 int mixed_alloc_fields(Chunk *c) {

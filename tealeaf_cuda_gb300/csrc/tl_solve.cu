@@ -82,6 +82,17 @@ bool ppcg_fused(const Chunk *c) {
     return c->cfg.precision != TL_PRECISION_MIXED && !c->cfg.reflective_boundary && c->cfg.ppcg_inner_steps >= 1;
 }
 
+// Mixed PPCG in loops: while the fused passes cannot fill the device, and only
+// with the inner steps' default settings (and fields of 32-bit offsets).
+// Microseconds an outer iteration with block-Jacobi, loop and graph of fused
+// passes: 32 and 126 at 128^2, 42 and 151 at 512^2, 91 and 181 at 1024^2 (run 2),
+// 185 and 208 at 1400^2 (4), 447 and 303 at 2048^2 (7).
+bool mixed_loop_pays(const Chunk *c) {
+    return c->inner_fuse == kInnerFuseDefault && c->inner_seg == kInnerSegDefault && !c->inner_fold_rrn &&
+           c->cfg.ppcg_inner_steps >= 1 && c->g.sets == c->g.groups && c->alloc_elems < ((size_t)1 << 31) &&
+           c->g.run <= 4;
+}
+
 int body_ppcg(Chunk *c) {
     int rc;
     const bool mixed = c->cfg.precision == TL_PRECISION_MIXED;
@@ -397,7 +408,10 @@ int solve_timestep(Chunk *c, tl_solve_info_t *info) {
                 rc = run_loop(c, launch_ppcg_loop, body_ppcg, kItersPpcg, kPhasePpcg, &done);
                 if (!rc) rc = launch_ppcg_finish(c);
             } else {
-                rc = run_phase(c, body_ppcg, kItersPpcg, kPhasePpcg, &done);
+                if (cf.precision == TL_PRECISION_MIXED && mixed_loop_pays(c))
+                    rc = run_loop(c, launch_mixed_ppcg_loop, body_ppcg, kItersPpcg, kPhasePpcg, &done);
+                else
+                    rc = run_phase(c, body_ppcg, kItersPpcg, kPhasePpcg, &done);
                 if (!rc && cf.precision == TL_PRECISION_MIXED) rc = launch_ppcg_finish(c);
             }
             break;
