@@ -98,11 +98,9 @@ BYTES_PER_CELL = {
     "ppcg_w_zr": 64,     # read p, Kx, Ky, diag, r, z; write w, r_store
     "ppcg_rrn": 24,      # read r, r_store, z
     # mixed precision: FP32 inner iteration (4-byte elements)
-    "mixed_w": 16,       # read p, Kx, Ky; write w
-    "mixed_ur": 32,      # jac_diag: read d, p, r, w, Mi; write d, r, z
-    "mixed_p": 12,       # read z, p; write p
+    "mixed_pw": 32,      # read z, p, d, Kx, Ky; write p, d, w
     "mixed_init": 28,    # read r (FP64), Mi; write r, z, p, d
-    "mixed_update_u": 20,  # read u (FP64), d; write u (FP64)
+    "mixed_update_u": 24,  # read u (FP64), d, p; write u (FP64)
     "mixed_convert": 40,   # read Kx, Ky (FP64); write Kx, Ky, Mi (FP32)
     "mixed_pp_init": 28,   # read r, z (FP64); write sd, rtemp, utemp
 }
@@ -162,9 +160,9 @@ def bytes_per_cell(kernel, precond):
         # read rtemp, sd, utemp + the preconditioner (Mi; or diag, Ky, cp,
         # bfp); write sd, utemp
         return {"none": 40, "jac_diag": 48, "jac_block": 72}[precond]
-    if kernel == "mixed_ur":
-        # read d, p, r, w + the preconditioner (Mi; or Ky, cp, bfp); write d, r, z
-        return {"none": 28, "jac_diag": 32, "jac_block": 40}[precond]
+    if kernel == "mixed_rz":
+        # read r, w + the preconditioner (Mi; or Ky, cp, bfp); write r, z
+        return {"none": 12, "jac_diag": 20, "jac_block": 28}[precond]
     if kernel == "mixed_init":
         # read r (FP64) + the preconditioner; write r, z, p, d
         return {"none": 24, "jac_diag": 28, "jac_block": 36}[precond]

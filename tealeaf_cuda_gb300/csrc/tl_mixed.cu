@@ -40,6 +40,7 @@ namespace {
 constexpr int kVRows = 8;
 constexpr int kVCols = 128;
 constexpr int kVTileRows = kVRows * kBlockWarps;
+constexpr int kVUnroll = 4;
 
 constexpr int kItersInner = 16;
 constexpr int kMaxOuter = 40;
@@ -85,6 +86,7 @@ __device__ void inner_epilogue(DevScalars *s, int epi, double tot) {
         break;
     case kInW:
         s->in_pw = tot;
+        s->p_sel ^= 1;
         s->in_alpha = s->in_rro / s->in_pw;
         if (s->prestep) s->lanczos_a[s->n] = s->in_alpha;  // cg_alphas (tea_leaf_cg.f90)
         break;
@@ -191,6 +193,7 @@ __global__ void __launch_bounds__(kBlockThreads) k_mixed(Geo g, int pitch32, Bod
 struct GeoV {
     int nx, ny, h, pitch;
     int tiles_x, tiles;
+    int rows;  // of a warp's run in the CG kernels
 };
 
 __device__ __forceinline__ float4 ld4(const float *__restrict__ f, int64_t i) {
@@ -250,62 +253,77 @@ __device__ __forceinline__ void reduce_v(CSum acc, double *partials, unsigned in
     }
 }
 
-// w = A p on a 128 x 64 tile; sum p.w
-__global__ void __launch_bounds__(kBlockThreads) k_v_w(GeoV g, const float *__restrict__ p,
-                                                       const float *__restrict__ kx,
-                                                       const float *__restrict__ ky,
-                                                       float *__restrict__ w, double *partials,
-                                                       unsigned int *counter, DevScalars *sc) {
+// The FP32 CG iteration in two passes (as the FP64 one, tl_loop.cuh): alpha and
+// beta here are those of the iteration before, 0 in the first.
+//   k_v_pw  d += alpha p, p' = z + beta p, w = A p'; sum p'.w
+//   k_v_rz  r -= alpha w, z = M^-1 r; sum r.z and the exit test
+// 32 + 20 bytes a cell (jac_diag) where separate d/r, p and w passes took 60.
+// HBM-bound.  A warp marches down a run of rows of 128 columns, runs side by
+// side at the same rows; there are as many runs as the device's warps take at
+// once, so no wave of blocks is left half empty and little is read twice.
+// p' goes to the other of two buffers (DevScalars::p_sel): the
+// neighbours' p' are computed again from z and p.
+__global__ void __launch_bounds__(kBlockThreads) k_v_pw(GeoV g, float *__restrict__ d, float *__restrict__ p0,
+                                                        float *__restrict__ p1, const float *__restrict__ z,
+                                                        const float *__restrict__ kx, const float *__restrict__ ky,
+                                                        float *__restrict__ w, double *partials, unsigned int *counter,
+                                                        DevScalars *sc) {
     if (*(volatile const int *)&sc->done) return;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int c = (blockIdx.x % g.tiles_x) * kVCols + lane * 4;
-    const int j0 = (blockIdx.x / g.tiles_x) * kVTileRows + warp * kVRows;
+    const bool sel = sc->p_sel != 0;
+    const float *__restrict__ p = sel ? p1 : p0;
+    float *__restrict__ po = sel ? p0 : p1;
+    const float alpha = (float)sc->in_alpha, beta = (float)sc->in_beta;
+    const int lane = threadIdx.x & 31, run = blockIdx.x * kBlockWarps + (threadIdx.x >> 5);
+    const int band = run / g.tiles_x, c = (run - band * g.tiles_x) * kVCols + lane * 4;
+    const int jb = band * g.rows, je = min(jb + g.rows, g.ny);
     const int nv = min(4, g.nx - c);           // valid columns of this lane
     const bool live = c < g.nx + 4;            // lanes that load (the first one past nx reads the halo)
     CSum acc = {0.f, 0.f};
-    if (j0 < g.ny) {
+    if (jb < je) {
         const int64_t P = g.pitch;
-        int64_t i = (int64_t)(c + g.h) + (int64_t)(j0 + g.h) * P;
+        int64_t i = (int64_t)(c + g.h) + (int64_t)(jb + g.h) * P;
+        int j0 = jb;
         const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-        // software pipeline, two rows deep: while row rr is computed, the p
-        // and Ky rows rr+2 and the Kx row rr+1 (with the lanes' edge values)
-        // are in flight.  A row is loaded only when it exists: padded rows
-        // run to ny + h, so row ny (the halo) is the last one read.
-        auto ldrow = [&](const float *f, int64_t at, int row) { return (live && row <= g.ny) ? ld4(f, at) : z4; };
-        float4 xm = ldrow(p, i - P, j0 - 1);
-        float4 x0 = ldrow(p, i, j0);
-        float4 xp = ldrow(p, i + P, j0 + 1);
-        float4 ky0 = ldrow(ky, i, j0);
-        float4 ky1 = ldrow(ky, i + P, j0 + 1);
-        float4 kxv = ldrow(kx, i, j0);
-        float kxe_edge = 0.f, xe_edge = 0.f, xw_edge = 0.f;  // the last / first lane's neighbours
-        if (lane == 31 && live) {
-            kxe_edge = kx[i + 4];
-            xe_edge = p[i + 4];
-        }
-        if (lane == 0 && live) xw_edge = p[i - 1];
+        auto next_p = [&](const float4 &zv, const float4 &pv) {
+            return make_float4(fmaf(beta, pv.x, zv.x), fmaf(beta, pv.y, zv.y), fmaf(beta, pv.z, zv.z),
+                               fmaf(beta, pv.w, zv.w));
+        };
+        // software pipeline: while row rr is computed, z, p and Ky of row rr + 2
+        // and d and Kx of row rr + 1 (with the edge lanes' neighbours) are in
+        // flight.  A row is loaded only when it exists: padded rows run to ny + h,
+        // so row ny (the halo) is the last one read; nothing past the run's next row.
+        auto ldrow = [&](const float *f, int64_t at, int row) { return (live && row <= je) ? ld4(f, at) : z4; };
+        float4 xm = next_p(ldrow(z, i - P, j0 - 1), ldrow(p, i - P, j0 - 1));
+        float4 pc = ldrow(p, i, j0), pn = ldrow(p, i + P, j0 + 1);  // old p of rows rr, rr + 1
+        float4 x0 = next_p(ldrow(z, i, j0), pc), xp = next_p(ldrow(z, i + P, j0 + 1), pn);
+        float4 ky0 = ldrow(ky, i, j0), ky1 = ldrow(ky, i + P, j0 + 1);
+        float4 kxv = ldrow(kx, i, j0), dv = ldrow(d, i, j0);
+        // the last lane's east face; the first and last lane's neighbours
+        const bool edge = live && (lane == 0 || lane == 31);
+        const int eo = lane == 0 ? -1 : 4;
+        float kxe_edge = lane == 31 && live ? kx[i + 4] : 0.f;
+        float ze = edge ? z[i + eo] : 0.f, pe = edge ? p[i + eo] : 0.f;
+        for (; j0 < je; j0 += kVUnroll)
 #pragma unroll
-        for (int rr = 0; rr < kVRows; ++rr) {
-            if (j0 + rr >= g.ny) break;
+        for (int rr = 0; rr < kVUnroll; ++rr) {
+            if (j0 + rr >= je) break;
             const int64_t in = i + P, inn = i + 2 * P;
             const int rn = j0 + rr + 1, rnn = j0 + rr + 2;
-            const float4 xpp = ldrow(p, inn, rnn);
+            const float4 zpp = ldrow(z, inn, rnn), ppp = ldrow(p, inn, rnn);
             const float4 ky2 = ldrow(ky, inn, rnn);
-            const float4 kxn = ldrow(kx, in, rn);
-            float kxe_n = 0.f, xe_n = 0.f, xw_n = 0.f;
-            if (lane == 31 && live && rn <= g.ny) {
-                kxe_n = kx[in + 4];
-                xe_n = p[in + 4];
-            }
-            if (lane == 0 && live && rn <= g.ny) xw_n = p[in - 1];
+            const float4 kxn = ldrow(kx, in, rn), dn = ldrow(d, in, rn);
+            const bool more = rn < je;
+            const float kxe_n = lane == 31 && live && more ? kx[in + 4] : 0.f;
+            const float ze_n = edge && more ? z[in + eo] : 0.f, pe_n = edge && more ? p[in + eo] : 0.f;
             float kxe = __shfl_down_sync(0xffffffffu, kxv.x, 1);
             float xe = __shfl_down_sync(0xffffffffu, x0.x, 1);
             float xw = __shfl_up_sync(0xffffffffu, x0.w, 1);
+            const float xb = fmaf(beta, pe, ze);
             if (lane == 31 && live) {
                 kxe = kxe_edge;
-                xe = xe_edge;
+                xe = xb;
             }
-            if (lane == 0 && live) xw = xw_edge;
+            if (lane == 0 && live) xw = xb;
             float4 o;
             o.x = cell_apply(x0.x, xp.x, xm.x, xw, x0.y, ky1.x, ky0.x, kxv.y, kxv.x);
             o.y = cell_apply(x0.y, xp.y, xm.y, x0.x, x0.z, ky1.y, ky0.y, kxv.z, kxv.y);
@@ -313,6 +331,9 @@ __global__ void __launch_bounds__(kBlockThreads) k_v_w(GeoV g, const float *__re
             o.w = cell_apply(x0.w, xp.w, xm.w, x0.z, xe, ky1.w, ky0.w, kxe, kxv.w);
             if (nv > 0) {
                 st4(w, i, o, nv);
+                st4(po, i, x0, nv);
+                st4(d, i, make_float4(fmaf(alpha, pc.x, dv.x), fmaf(alpha, pc.y, dv.y), fmaf(alpha, pc.z, dv.z),
+                                      fmaf(alpha, pc.w, dv.w)), nv);
                 csum_add(acc, x0.x * o.x);
                 if (nv > 1) csum_add(acc, x0.y * o.y);
                 if (nv > 2) csum_add(acc, x0.z * o.z);
@@ -320,158 +341,101 @@ __global__ void __launch_bounds__(kBlockThreads) k_v_w(GeoV g, const float *__re
             }
             xm = x0;
             x0 = xp;
-            xp = xpp;
+            pc = pn;
+            xp = next_p(zpp, ppp);
+            pn = ppp;
             ky0 = ky1;
             ky1 = ky2;
             kxv = kxn;
+            dv = dn;
             kxe_edge = kxe_n;
-            xe_edge = xe_n;
-            xw_edge = xw_n;
+            ze = ze_n;
+            pe = pe_n;
             i += P;
         }
     }
     reduce_v(acc, partials, counter, sc, kInW);
 }
 
-// d += alpha p; r -= alpha w; z = M^-1 r; sum r.z.  PC: TL_PREC_NONE (z = r,
-// not stored), TL_PREC_JAC_DIAG (z = Mi r) or TL_PREC_JAC_BLOCK (the 4-row
-// strip solve of k_pp_step on the warp's two strips; ky, cp and bfp with
-// 1/diag in each strip's first row)
+// r -= alpha w; z = M^-1 r; sum r.z.  PC: TL_PREC_NONE (z = r, not stored),
+// TL_PREC_JAC_DIAG (z = Mi r) or TL_PREC_JAC_BLOCK (the 4-row strip solve of
+// k_pp_step on the warp's two strips; ky, cp and bfp with 1/diag in each
+// strip's first row)
 template <int PC>
-__global__ void __launch_bounds__(kBlockThreads) k_v_ur(GeoV g, float *__restrict__ d,
-                                                        float *__restrict__ r,
-                                                        float *__restrict__ z,
-                                                        const float *__restrict__ p,
-                                                        const float *__restrict__ w,
-                                                        const float *__restrict__ mi,
-                                                        const float *__restrict__ ky,
-                                                        const float *__restrict__ cp,
-                                                        const float *__restrict__ bfp,
-                                                        double *partials, unsigned int *counter,
-                                                        DevScalars *sc) {
-    constexpr bool DIAG = PC == TL_PREC_JAC_DIAG;
+__global__ void __launch_bounds__(kBlockThreads, 3) k_v_rz(GeoV g, float *__restrict__ r, float *__restrict__ z,
+                                                        const float *__restrict__ w, const float *__restrict__ mi,
+                                                        const float *__restrict__ ky, const float *__restrict__ cp,
+                                                        const float *__restrict__ bfp, double *partials,
+                                                        unsigned int *counter, DevScalars *sc) {
     if (*(volatile const int *)&sc->done) return;
     const float alpha = (float)sc->in_alpha;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int c = (blockIdx.x % g.tiles_x) * kVCols + lane * 4;
-    const int j0 = (blockIdx.x / g.tiles_x) * kVTileRows + warp * kVRows;
+    const int lane = threadIdx.x & 31, run = blockIdx.x * kBlockWarps + (threadIdx.x >> 5);
+    const int band = run / g.tiles_x, c = (run - band * g.tiles_x) * kVCols + lane * 4;
+    const int jb = band * g.rows, je = min(jb + g.rows, g.ny);
     const int nv = min(4, g.nx - c);
     CSum acc = {0.f, 0.f};
-    if (PC == TL_PREC_JAC_BLOCK && j0 < g.ny && nv > 0) {
+    if (nv > 0) {
         const int64_t P = g.pitch;
-#pragma unroll
-        for (int s0 = 0; s0 < kVRows; s0 += 4) {
-            if (j0 + s0 >= g.ny) break;
-            const int m = min(4, g.ny - (j0 + s0));
-            const int64_t i0 = (int64_t)(c + g.h) + (int64_t)(j0 + s0 + g.h) * P;
-            float4 rv[4], zv[4];
+#pragma unroll 1
+        for (int j0 = jb; j0 < je; j0 += 4) {
+            const int m = min(4, je - j0);
+            const int64_t i0 = (int64_t)(c + g.h) + (int64_t)(j0 + g.h) * P;
+            float4 rv[4], zv[4], wv[4], f[4];
+            // the strip's loads before its first store
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 if (k >= m) break;
                 const int64_t i = i0 + (int64_t)k * P;
-                const float4 pv = ld4(p, i), wv = ld4(w, i), rv0 = ld4(r, i), dv0 = ld4(d, i);
-                float4 dv;
-                dv.x = fmaf(alpha, pv.x, dv0.x);
-                dv.y = fmaf(alpha, pv.y, dv0.y);
-                dv.z = fmaf(alpha, pv.z, dv0.z);
-                dv.w = fmaf(alpha, pv.w, dv0.w);
-                rv[k].x = fmaf(-alpha, wv.x, rv0.x);
-                rv[k].y = fmaf(-alpha, wv.y, rv0.y);
-                rv[k].z = fmaf(-alpha, wv.z, rv0.z);
-                rv[k].w = fmaf(-alpha, wv.w, rv0.w);
-                st4(d, i, dv, nv);
-                st4(r, i, rv[k], nv);
-                // Thomas forward sweep: dp0 = x0 / b0, dp_k = (x_k + Ky_k dp_{k-1}) bfp_k
-                const float4 bf = ld4(bfp, i);
-                if (k == 0) {
-                    zv[0] = make_float4(rv[0].x * bf.x, rv[0].y * bf.y, rv[0].z * bf.z, rv[0].w * bf.w);
-                } else {
-                    const float4 kyk = ld4(ky, i);
-                    zv[k].x = fmaf(kyk.x, zv[k - 1].x, rv[k].x) * bf.x;
-                    zv[k].y = fmaf(kyk.y, zv[k - 1].y, rv[k].y) * bf.y;
-                    zv[k].z = fmaf(kyk.z, zv[k - 1].z, rv[k].z) * bf.z;
-                    zv[k].w = fmaf(kyk.w, zv[k - 1].w, rv[k].w) * bf.w;
-                }
-            }
-#pragma unroll
-            for (int k = 2; k >= 0; --k) {
-                if (k >= m - 1) continue;
-                const float4 cv = ld4(cp, i0 + (int64_t)k * P);
-                zv[k].x = fmaf(-cv.x, zv[k + 1].x, zv[k].x);
-                zv[k].y = fmaf(-cv.y, zv[k + 1].y, zv[k].y);
-                zv[k].z = fmaf(-cv.z, zv[k + 1].z, zv[k].z);
-                zv[k].w = fmaf(-cv.w, zv[k + 1].w, zv[k].w);
+                wv[k] = ld4(w, i);
+                rv[k] = ld4(r, i);
+                if (PC == TL_PREC_JAC_DIAG) f[k] = ld4(mi, i);
+                if (PC == TL_PREC_JAC_BLOCK) f[k] = ld4(bfp, i);
             }
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 if (k >= m) break;
-                st4(z, i0 + (int64_t)k * P, zv[k], nv);
+                const int64_t i = i0 + (int64_t)k * P;
+                rv[k].x = fmaf(-alpha, wv[k].x, rv[k].x);
+                rv[k].y = fmaf(-alpha, wv[k].y, rv[k].y);
+                rv[k].z = fmaf(-alpha, wv[k].z, rv[k].z);
+                rv[k].w = fmaf(-alpha, wv[k].w, rv[k].w);
+                st4(r, i, rv[k], nv);
+                if (PC == TL_PREC_NONE) {
+                    zv[k] = rv[k];
+                } else if (PC == TL_PREC_JAC_DIAG || k == 0) {
+                    // (Thomas forward sweep: dp0 = x0 / b0, dp_k = (x_k + Ky_k dp_{k-1}) bfp_k)
+                    zv[k] = make_float4(rv[k].x * f[k].x, rv[k].y * f[k].y, rv[k].z * f[k].z, rv[k].w * f[k].w);
+                } else {
+                    const float4 kyk = ld4(ky, i);
+                    zv[k].x = fmaf(kyk.x, zv[k - 1].x, rv[k].x) * f[k].x;
+                    zv[k].y = fmaf(kyk.y, zv[k - 1].y, rv[k].y) * f[k].y;
+                    zv[k].z = fmaf(kyk.z, zv[k - 1].z, rv[k].z) * f[k].z;
+                    zv[k].w = fmaf(kyk.w, zv[k - 1].w, rv[k].w) * f[k].w;
+                }
+            }
+            if (PC == TL_PREC_JAC_BLOCK) {
+#pragma unroll
+                for (int k = 2; k >= 0; --k) {
+                    if (k >= m - 1) continue;
+                    const float4 cv = ld4(cp, i0 + (int64_t)k * P);
+                    zv[k].x = fmaf(-cv.x, zv[k + 1].x, zv[k].x);
+                    zv[k].y = fmaf(-cv.y, zv[k + 1].y, zv[k].y);
+                    zv[k].z = fmaf(-cv.z, zv[k + 1].z, zv[k].z);
+                    zv[k].w = fmaf(-cv.w, zv[k + 1].w, zv[k].w);
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                if (k >= m) break;
+                if (PC != TL_PREC_NONE) st4(z, i0 + (int64_t)k * P, zv[k], nv);
                 csum_add(acc, rv[k].x * zv[k].x);
                 if (nv > 1) csum_add(acc, rv[k].y * zv[k].y);
                 if (nv > 2) csum_add(acc, rv[k].z * zv[k].z);
                 if (nv > 3) csum_add(acc, rv[k].w * zv[k].w);
             }
         }
-    } else if (j0 < g.ny && nv > 0) {
-        const int64_t P = g.pitch;
-        int64_t i = (int64_t)(c + g.h) + (int64_t)(j0 + g.h) * P;
-#pragma unroll
-        for (int rr = 0; rr < kVRows; ++rr) {
-            if (j0 + rr >= g.ny) break;
-            const float4 pv = ld4(p, i), wv = ld4(w, i), rv0 = ld4(r, i), dv0 = ld4(d, i);
-            float4 dv, rv, zv;
-            dv.x = fmaf(alpha, pv.x, dv0.x);
-            dv.y = fmaf(alpha, pv.y, dv0.y);
-            dv.z = fmaf(alpha, pv.z, dv0.z);
-            dv.w = fmaf(alpha, pv.w, dv0.w);
-            rv.x = fmaf(-alpha, wv.x, rv0.x);
-            rv.y = fmaf(-alpha, wv.y, rv0.y);
-            rv.z = fmaf(-alpha, wv.z, rv0.z);
-            rv.w = fmaf(-alpha, wv.w, rv0.w);
-            if (DIAG) {
-                const float4 m = ld4(mi, i);
-                zv = make_float4(rv.x * m.x, rv.y * m.y, rv.z * m.z, rv.w * m.w);
-                st4(z, i, zv, nv);
-            } else {
-                zv = rv;
-            }
-            st4(d, i, dv, nv);
-            st4(r, i, rv, nv);
-            csum_add(acc, rv.x * zv.x);
-            if (nv > 1) csum_add(acc, rv.y * zv.y);
-            if (nv > 2) csum_add(acc, rv.z * zv.z);
-            if (nv > 3) csum_add(acc, rv.w * zv.w);
-            i += P;
-        }
     }
     reduce_v(acc, partials, counter, sc, kInUr);
-}
-
-// p = z + beta p
-__global__ void __launch_bounds__(kBlockThreads) k_v_p(GeoV g, float *__restrict__ p,
-                                                       const float *__restrict__ z,
-                                                       DevScalars *sc) {
-    if (*(volatile const int *)&sc->done) return;
-    const float beta = (float)sc->in_beta;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int c = (blockIdx.x % g.tiles_x) * kVCols + lane * 4;
-    const int j0 = (blockIdx.x / g.tiles_x) * kVTileRows + warp * kVRows;
-    const int nv = min(4, g.nx - c);
-    if (j0 >= g.ny || nv <= 0) return;
-    const int64_t P = g.pitch;
-    int64_t i = (int64_t)(c + g.h) + (int64_t)(j0 + g.h) * P;
-#pragma unroll
-    for (int rr = 0; rr < kVRows; ++rr) {
-        if (j0 + rr >= g.ny) break;
-        const float4 pv = ld4(p, i), zv = ld4(z, i);
-        float4 o;
-        o.x = fmaf(beta, pv.x, zv.x);
-        o.y = fmaf(beta, pv.y, zv.y);
-        o.z = fmaf(beta, pv.z, zv.z);
-        o.w = fmaf(beta, pv.w, zv.w);
-        st4(p, i, o, nv);
-        i += P;
-    }
 }
 
 // ------------------------------------ PPCG inner steps in FP32 (mixed form)
@@ -1232,18 +1196,30 @@ struct BodyInnerInit {  // r = (float) r64; z = M^-1 r; p = z; d = 0; sum r.z
     }
 };
 
-struct BodyUpdateU {  // u += d (FP64)
+struct BodyUpdateU {  // u += d (FP64), with the last iteration's d += alpha p (FP32)
     double *u;
-    const float *d;
+    const float *d, *p0, *p1;
     int pitch32, pitch64;
-    __device__ void setup(DevScalars *) {}
+    const float *p;
+    float alpha;
+    __device__ void setup(DevScalars *sc) {
+        p = sc->p_sel ? p1 : p0;
+        alpha = (float)sc->in_alpha;
+    }
     __device__ void operator()(int64_t b32, int64_t b64, int m, CSum &) const {
+        float dv[4], pv[4];
+        double uv[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k)
             if (k < m) {
-                const int64_t i = b64 + (int64_t)k * pitch64;
-                u[i] = u[i] + (double)d[b32 + (int64_t)k * pitch32];
+                const int64_t j = b32 + (int64_t)k * pitch32;
+                dv[k] = d[j];
+                pv[k] = p[j];
+                uv[k] = u[b64 + (int64_t)k * pitch64];
             }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (k < m) u[b64 + (int64_t)k * pitch64] = uv[k] + (double)fmaf(alpha, pv[k], dv[k]);
     }
 };
 
@@ -1390,26 +1366,35 @@ int launch_v(Chunk *c, const char *name, F &&launch) {
     return TL_OK;
 }
 
+// runs for `ctas` blocks a multiprocessor: at least 8 rows, whole strips.
+// (Never more blocks than the tiles that the partial sums have room for.)
+GeoV run_geo(const Chunk *c, int ctas, unsigned *grid) {
+    const Mixed *mx = (const Mixed *)c->mixed;
+    GeoV g{c->nx, c->ny, c->h, c->pitch, mx->vtiles_x, mx->vtiles, 0};
+    const int warps = c->sms * ctas * kBlockWarps, bands = warps / g.tiles_x > 1 ? warps / g.tiles_x : 1;
+    const int strips = (c->ny + 3) / 4, per = (strips + bands - 1) / bands;
+    g.rows = 4 * (per > 2 ? per : 2);
+    const long long runs = (long long)g.tiles_x * ((c->ny + g.rows - 1) / g.rows);
+    *grid = (unsigned)((runs + kBlockWarps - 1) / kBlockWarps);
+    return g;
+}
+
 template <int PC>
 int inner_body_pc(Chunk *c) {
     Mixed *mx = mixed_of(c);
     const bool diag = PC != TL_PREC_NONE;
-    const GeoV g{c->nx, c->ny, c->h, c->pitch, mx->vtiles_x, mx->vtiles};
-    const unsigned grid = (unsigned)mx->vtiles;
+    unsigned grid, grid_rz;
+    const GeoV g = run_geo(c, 2, &grid), g_rz = run_geo(c, 3, &grid_rz);
     cudaStream_t s = c->stream;
     int rc;
-    if ((rc = launch_v(c, "mixed_w", [&] {
-             k_v_w<<<grid, kBlockThreads, 0, s>>>(g, mx->p, mx->kx, mx->ky, mx->w, mx->partials,
-                                                   mx->counter, c->sc);
+    if ((rc = launch_v(c, "mixed_pw", [&] {
+             k_v_pw<<<grid, kBlockThreads, 0, s>>>(g, mx->d, mx->p, mx->sd[0], diag ? mx->z : mx->r, mx->kx, mx->ky,
+                                                    mx->w, mx->partials, mx->counter, c->sc);
          })))
         return rc;
-    if ((rc = launch_v(c, "mixed_ur", [&] {
-             k_v_ur<PC><<<grid, kBlockThreads, 0, s>>>(g, mx->d, mx->r, mx->z, mx->p, mx->w, mx->mi, mx->ky,
-                                                       mx->cp, mx->bfp, mx->partials, mx->counter, c->sc);
-         })))
-        return rc;
-    return launch_v(c, "mixed_p", [&] {
-        k_v_p<<<grid, kBlockThreads, 0, s>>>(g, mx->p, diag ? mx->z : mx->r, c->sc);
+    return launch_v(c, "mixed_rz", [&] {
+        k_v_rz<PC><<<grid_rz, kBlockThreads, 0, s>>>(g_rz, mx->r, mx->z, mx->w, mx->mi, mx->ky, mx->cp, mx->bfp,
+                                                  mx->partials, mx->counter, c->sc);
     });
 }
 
@@ -1662,6 +1647,8 @@ int mixed_ppcg_presteps(Chunk *c, int *done_out) {
     h.lanczos_a = c->cg_alphas;
     h.lanczos_b = c->cg_betas;
     h.in_target = 0.0;
+    h.in_alpha = h.in_beta = 0.0;
+    h.p_sel = 0;
     if ((rc = chunk_push_scalars(c))) return rc;
     // r = (float) r, z = M^-1 r, p = z, d = 0, in_rro = r.z
 #define TL_PRE_INIT(PC)                                                                                        \
@@ -1677,7 +1664,7 @@ int mixed_ppcg_presteps(Chunk *c, int *done_out) {
     if ((rc = run_phase(c, prestep_body, kItersInner, kPhaseMixedPre, &done))) return rc;
     // u += d, r = u0 - A u (FP64): the phase after the switch starts from the
     // true residual
-    BodyUpdateU bu{c->u, mx->d, c->pitch, c->pitch};
+    BodyUpdateU bu{c->u, mx->d, mx->p, mx->sd[0], c->pitch, c->pitch, nullptr, 0.f};
     if ((rc = run32(c, "mixed_update_u", bu, kInNone, false))) return rc;
     if ((rc = launch_residual(c, kEpiNone))) return rc;
     if ((rc = chunk_sync_scalars(c))) return rc;
@@ -1757,6 +1744,8 @@ int solve_timestep_mixed(Chunk *c, tl_solve_info_t *info) {
         h.done = kRunning;
         h.in_target = cf.inner_eps;
         h.in_max = cf.max_iters;
+        h.in_alpha = h.in_beta = 0.0;
+        h.p_sel = 0;
         if ((rc = chunk_push_scalars(c))) return rc;
         if (diag) {
             BodyInnerInit<TL_PREC_JAC_DIAG> bi{c->r, mx->mi, mx->ky, mx->cp, mx->bfp, mx->r, mx->z, mx->p, mx->d,
@@ -1777,7 +1766,7 @@ int solve_timestep_mixed(Chunk *c, tl_solve_info_t *info) {
         inner_total += h.in_n;
         if (h.in_n >= cf.max_iters) capped = true;
         // u += d (FP64), r = u0 - A u (FP64)
-        BodyUpdateU bu{c->u, mx->d, c->pitch, c->pitch};
+        BodyUpdateU bu{c->u, mx->d, mx->p, mx->sd[0], c->pitch, c->pitch, nullptr, 0.f};
         if ((rc = run32(c, "mixed_update_u", bu, kInNone, false))) return rc;
         if ((rc = launch_residual(c, kEpiStore))) return rc;
         if ((rc = chunk_sync_scalars(c))) return rc;
