@@ -44,26 +44,6 @@ __global__ void __launch_bounds__(kGroupThreads) k_strips(Geo g, Body body, RedC
 
 // ------------------------------------------------------------- bodies
 
-struct BodyResidual {  // r = u0 - A u  (+ r.r)
-    const double *dg;  // diag(A), stored by the diag kernel
-    const double *u, *u0, *kx, *ky;
-    double *r;
-    int pitch;
-    __device__ void setup() {}
-    __device__ void operator()(int64_t base, int m, double (&acc)[1]) const {
-        double xc[4], ax[4];
-        strip_apply(kx, ky, dg, pitch, base, m, LoadX{u}, xc, ax);
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-            if (k < m) {
-                const int64_t i = base + (int64_t)k * pitch;
-                const double rv = u0[i] - ax[k];
-                r[i] = rv;
-                acc[0] = fma(rv, rv, acc[0]);
-            }
-    }
-};
-
 struct BodyNorm {  // sum a.b
     const double *a, *b;
     int pitch;
@@ -736,11 +716,6 @@ int launch_common_init(Chunk *c, int coefficient, double rx, double ry, const in
     if (e != cudaSuccess) return cuda_fail(e, "common_init launch");
     BodyDiag bd{c->kx, c->ky, c->diag, c->pitch};
     return run<1>(c, "diag", bd, kEpiNone, false);
-}
-
-int launch_residual(Chunk *c, int epi) {
-    BodyResidual b{c->diag, c->u, c->u0, c->kx, c->ky, c->r, c->pitch};
-    return run<1>(c, "residual", b, epi, false);
 }
 
 int launch_norm(Chunk *c, const double *a, const double *bb, int epi) {

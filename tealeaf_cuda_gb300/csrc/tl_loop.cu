@@ -194,10 +194,11 @@ __global__ void __launch_bounds__(kGroupThreads) k_cg_finish(Geo g, CgArgs a, co
 //   Chebyshev  r = u0 - A u, p = al p + be M^-1 r, u' = u + p       (x = u)
 //   PPCG       rtemp -= A sd, sd' = al sd + be M^-1 rtemp, utemp += sd'  (x = sd)
 // x' goes to the other of two buffers, so that the neighbours still read x.
+// The residual r = u0 - A u (+ r.r) is the same walk without an update.
 // FP64-bound: 10 (none), 11 (diag) or 14 (block) instructions a cell; a pass
 // of its own for u += p or the sd update read and wrote 24 to 48 bytes a cell
 // more and waited once more for the grid.
-enum StepMode { kStepCheby, kStepPpcg, kStepPpcgLast };
+enum StepMode { kStepCheby, kStepPpcg, kStepPpcgLast, kStepResidual };
 
 struct StepArgs {
     double *x0, *x1;   // u or sd: the two buffers
@@ -221,23 +222,26 @@ __device__ __forceinline__ void step_pass(const Geo &g, const StepArgs &a, const
                                           double (&acc)[MODE == kStepPpcgLast ? 2 : 1]) {
     constexpr bool BLOCK = PC == TL_PREC_JAC_BLOCK, DIAG = PC == TL_PREC_JAC_DIAG;
     constexpr bool CHEBY = MODE == kStepCheby, LAST = MODE == kStepPpcgLast;
+    // cells around the field that x is read from: the residual's u has its halo, which
+    // reflective boundaries couple in
+    constexpr int H = MODE == kStepResidual ? 1 : 0;
     const int lane = threadIdx.x & 31, i = i0 + lane;
-    const bool own = i < g.nx;
+    const bool own = i < g.nx, ownx = i < g.nx + H;
     const int64_t P = g.pitch;
     int64_t c = (int64_t)(i + g.h) + (int64_t)(jb + g.h) * P;
     const int ek = (lane >> 1) & 3, ecol = (lane & 1) ? i0 + kWarpCols : i0 - 1;
-    const bool eon = lane < 8 && ecol >= 0 && ecol < g.nx, fon = lane < 8 && (lane & 1) && ecol <= g.nx;
+    const bool eon = lane < 8 && ecol >= -H && ecol < g.nx + H, fon = lane < 8 && (lane & 1) && ecol <= g.nx;
     int64_t e = (int64_t)(ecol + g.h) + (int64_t)(jb + ek + g.h) * P;
     // a row's Kx, diag, f and q (and Mi), the next row's x and Ky; x and Kx beside
     double xl[D], ky[D], kx[D], dg[D], f[D], q[D], mi[D], ex, ef;
     auto load_row = [&](int k, int row, int64_t at) {
         const bool in = own && row < je;
-        xl[k] = in && row + 1 < g.ny ? __ldcg(xin + at + P) : 0.0;
+        xl[k] = ownx && row < je && row + 1 < g.ny + H ? __ldcg(xin + at + P) : 0.0;
         ky[k] = in ? a.ky[at + P] : 0.0;
         kx[k] = in ? a.kx[at] : 0.0;
         dg[k] = in ? a.dg[at] : 0.0;
         f[k] = in ? __ldcg(a.f + at) : 0.0;
-        if (!BLOCK) q[k] = in ? __ldcg(a.q + at) : 0.0;
+        if (!BLOCK && MODE != kStepResidual) q[k] = in ? __ldcg(a.q + at) : 0.0;
         if (DIAG) mi[k] = in ? a.mi[at] : 0.0;
     };
     auto load_edge = [&](int j0) {
@@ -245,7 +249,7 @@ __device__ __forceinline__ void step_pass(const Geo &g, const StepArgs &a, const
         ex = v && eon ? __ldcg(xin + e) : 0.0;
         ef = v && fon ? a.kx[e] : 0.0;
     };
-    double xm = own && jb > 0 ? __ldcg(xin + c - P) : 0.0, x0 = own ? __ldcg(xin + c) : 0.0;
+    double xm = ownx && jb > -H ? __ldcg(xin + c - P) : 0.0, x0 = ownx ? __ldcg(xin + c) : 0.0;
     double kyv = own ? a.ky[c] : 0.0;
 #pragma unroll
     for (int k = 0; k < D; ++k) load_row(k, jb + k, c + k * P);
@@ -259,6 +263,11 @@ __device__ __forceinline__ void step_pass(const Geo &g, const StepArgs &a, const
         // the row's new values from its r and z
         auto finish = [&](int k, double r, double z, double m) {
             const int64_t at = c + k * P;
+            if (MODE == kStepResidual) {
+                a.r[at] = r;
+                acc[0] = fma(r, r, acc[0]);
+                return;
+            }
             double be_z;
             if (PC == TL_PREC_NONE || BLOCK) be_z = co.be * z;
             else if (CHEBY) be_z = (co.be * m) * r;
@@ -314,7 +323,7 @@ __device__ __forceinline__ void step_pass(const Geo &g, const StepArgs &a, const
                 const int k = kb + d;
                 rv[k] = f[d] - (t[d] - b[d]);
                 xc[k] = x[d + 1];
-                if (!BLOCK) qv[k] = q[d];
+                if (!BLOCK && MODE != kStepResidual) qv[k] = q[d];
             }
             if (!BLOCK) {
 #pragma unroll
@@ -428,6 +437,15 @@ __global__ void __launch_bounds__(kGroupThreads, 4) k_step(Geo g, StepArgs a, in
         step_pass<PC, MODE, 4>(g, a, odd ? a.x1 : a.x0, odd ? a.x0 : a.x1, i0, jb, je, co, [] { return true; }, acc);
     });
     if (NV > 0) grid_reduce<NV>(acc, red, g.sms);
+}
+
+__global__ void __launch_bounds__(kGroupThreads, 4) k_residual(Geo g, StepArgs a, RedCtx red) {
+    StepCoef co{};
+    double acc[1] = {0.0};
+    for_runs(g, blockIdx.x, threadIdx.x >> 5, [&](int i0, int jb, int je) {
+        step_pass<TL_PREC_NONE, kStepResidual, 4>(g, a, a.x0, nullptr, i0, jb, je, co, [] { return true; }, acc);
+    });
+    if (red.epi != kEpiNone) grid_reduce<1>(acc, red, g.sms);
 }
 
 template <int PC, class Shape>
@@ -706,6 +724,15 @@ StepArgs step_args(Chunk *c) {
 }
 
 }  // namespace
+
+int launch_residual(Chunk *c, int epi) {
+    StepArgs a = step_args(c);
+    a.x0 = c->u;
+    a.f = c->u0;
+    return launch_named(c, "residual", [&] {
+        k_residual<<<c->g.groups, kGroupThreads, 0, c->stream>>>(c->g, a, red_ctx(c, epi, false));
+    });
+}
 
 int launch_cg_pass1(Chunk *c, bool ppcg) {
     const bool five = ppcg && c->cfg.precision == TL_PRECISION_MIXED;

@@ -106,8 +106,13 @@ struct Warm {
 long long layer_floats(int l) { return 9LL * kCin[l] * kCout[l] + kCout[l]; }
 
 __device__ __forceinline__ int64_t cell_of(const Geo &g, long long k, int *i, int *j) {
-    *i = (int)(k % g.nx);
-    *j = (int)(k / g.nx);
+    if (k >> 32) {
+        *j = (int)(k / g.nx);
+        *i = (int)(k - (long long)*j * g.nx);
+    } else {  // a division of 32 bits takes a third of the instructions
+        *j = (int)((unsigned)k / (unsigned)g.nx);
+        *i = (int)((unsigned)k - (unsigned)*j * (unsigned)g.nx);
+    }
     return (int64_t)(*i + g.h) + (int64_t)(*j + g.h) * g.pitch;
 }
 
@@ -172,9 +177,18 @@ __global__ void k_prev(Geo g, const double *__restrict__ u0, double *__restrict_
 
 __device__ __forceinline__ float clampf(float v) { return fminf(fmaxf(v, -kClamp), kClamp); }
 
+// (float)(x / b), y the correctly rounded 1 / b: the quotient within 0.5000001
+// ulps of FP64 (x / b below FP64's smallest residuals is zero in FP32)
+__device__ __forceinline__ float quotient(double x, double b, double y) {
+    const double q = x * y;
+    return (float)fma(fma(-b, q, x), y, q);
+}
+
 // network inputs of cell (i, j), as BF16 into the padded NHWC input
 // (x != nullptr) and/or as FP32 [ny][nx][kFeatures] with the target
-// (u - ubase) / max|rr| (f != nullptr); rr is the residual of ubase
+// (u - ubase) / max|rr| (f != nullptr); rr is the residual of ubase.  Both
+// divisors are the same in all cells: their reciprocals replace 3 FP64
+// divisions a cell, which bound the kernel
 __global__ void k_features(Geo g, const double *__restrict__ u0, const double *__restrict__ u,
                            const double *__restrict__ ubase, const double *__restrict__ rr,
                            const double *__restrict__ dprev,
@@ -183,21 +197,31 @@ __global__ void k_features(Geo g, const double *__restrict__ u0, const double *_
                            bf16 *__restrict__ x, int nxp, float *__restrict__ f) {
     const long long n = (long long)g.nx * g.ny;
     const double su = fmax((double)scale[0], 1e-300), sr = fmax((double)scale[1], 1e-300);
+    // out of this range a quotient may overflow where the residual correction does not work
+    const bool tame = su > 1e-30 && su < 1e30 && sr > 1e-30 && sr < 1e30;
+    const double yu = 1.0 / su, yr = 1.0 / sr;
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n;
          k += (long long)gridDim.x * blockDim.x) {
         int i, j;
         const int64_t c = cell_of(g, k, &i, &j);
         float v[kInputs];
-        v[0] = (float)(u0[c] / su);
+        v[0] = tame ? quotient(u0[c], su, yu) : (float)(u0[c] / su);
         v[1] = logf((float)density[c]);
         v[2] = log1pf((float)kx[c]);
         v[3] = log1pf((float)ky[c]);
         v[4] = (float)(100.0 * dt);
-        v[5] = clampf((float)(rr[c] / sr));
-        v[6] = clampf((float)(dprev[c] / sr));
+        v[5] = clampf(tame ? quotient(rr[c], sr, yr) : (float)(rr[c] / sr));
+        v[6] = clampf(tame ? quotient(dprev[c], sr, yr) : (float)(dprev[c] / sr));
         if (x) {
-            bf16 *d = x + (((int64_t)(j + 1)) * (nxp + 2) + i + 1) * 16;
-            for (int q = 0; q < kInputs; ++q) d[q] = __float2bfloat16(v[q]);
+            // the first 8 of the 16 channels in one 16-byte store (the eighth is unused: zero)
+            static_assert(kInputs == 7, "one store of 8 channels");
+            union {
+                bf16 h[8];
+                uint4 all;
+            } o;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) o.h[q] = __float2bfloat16(q < kInputs ? v[q] : 0.f);
+            *reinterpret_cast<uint4 *>(x + (((int64_t)(j + 1)) * (nxp + 2) + i + 1) * 16) = o.all;
         }
         if (f) {
             float *d = f + k * kFeatures;
@@ -232,50 +256,61 @@ __host__ __device__ constexpr int pair_index(int i, int j) { return i * kMaxDirs
 // Gram entries of the projection, per CTA in a fixed order.  Energy
 // (Galerkin): d_i.Ad_j for i <= j, then d_i.r0, then r0.r0.  MR (minimal
 // residual): Ad_i.Ad_j, then Ad_i.r0, then r0.r0.
-template <bool MR>
+// N directions: the sums that N of them have, N (N + 1) / 2 + N + 1, and 5 N
+// FP64 instructions a cell for the A d_i, which bound it.  (8192^2 cells: one
+// direction 1.17 ms, two 2.19; with all nine always, 6.7 and 7.5.)
+template <bool MR, int N>
 __global__ void __launch_bounds__(256) k_gram(Geo g, Dirs D, const double *__restrict__ r0,
                                               const double *__restrict__ dg, const double *__restrict__ kx,
                                               const double *__restrict__ ky, double *__restrict__ partials) {
-    double s[kGramSums];
+    constexpr int NP = N * (N + 1) / 2, NS = NP + N + 1;  // pairs i <= j row by row, d_i.r0, r0.r0
+    double s[NS];
 #pragma unroll
-    for (int q = 0; q < kGramSums; ++q) s[q] = 0.0;
+    for (int q = 0; q < NS; ++q) s[q] = 0.0;
     const long long n = (long long)g.nx * g.ny;
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n;
          k += (long long)gridDim.x * blockDim.x) {
         int i, j;
         const int64_t c = cell_of(g, k, &i, &j);
         const double r = r0[c];
-        double dv[kMaxDirs], av[kMaxDirs];
+        double dv[N], av[N];
 #pragma unroll
-        for (int a = 0; a < kMaxDirs; ++a) {
-            dv[a] = av[a] = 0.0;
-            if (a < D.n) {
-                dv[a] = D.d[a][c];
-                av[a] = apply_a(D.d[a], dg, kx, ky, c, g.pitch);
-            }
+        for (int a = 0; a < N; ++a) {
+            dv[a] = D.d[a][c];
+            av[a] = apply_a(D.d[a], dg, kx, ky, c, g.pitch);
         }
+        int q = 0;
 #pragma unroll
-        for (int a = 0; a < kMaxDirs; ++a) {
-#pragma unroll
+        for (int a = 0; a < N; ++a) {
             const double la = MR ? av[a] : dv[a];
-            for (int b = a; b < kMaxDirs; ++b) s[pair_index(a, b)] = fma(la, av[b], s[pair_index(a, b)]);
-            s[kGramPairs + a] = fma(la, r, s[kGramPairs + a]);
+#pragma unroll
+            for (int b = a; b < N; ++b, ++q) s[q] = fma(la, av[b], s[q]);
+            s[NP + a] = fma(la, r, s[NP + a]);
         }
-        s[kGramSums - 1] = fma(r, r, s[kGramSums - 1]);
+        s[NS - 1] = fma(r, r, s[NS - 1]);
     }
-    __shared__ double red[8][kGramSums];
+    __shared__ double red[8][NS];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-    for (int q = 0; q < kGramSums; ++q) {
+    for (int q = 0; q < NS; ++q) {
         double v = s[q];
         for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
         if (lane == 0) red[warp][q] = v;
     }
     __syncthreads();
-    if (threadIdx.x < kGramSums) {
+    // to the places that the sums have among all directions'
+    for (int q = threadIdx.x; q < NS; q += blockDim.x) {
         double t = 0.0;
-        for (int w = 0; w < 8; ++w) t += red[w][threadIdx.x];
-        partials[(int64_t)blockIdx.x * kGramSums + threadIdx.x] = t;
+        for (int w = 0; w < 8; ++w) t += red[w][q];
+        int to = kGramSums - 1;
+        if (q < NP) {
+            int a = 0, left = q;
+            while (left >= N - a) left -= N - a++;
+            to = pair_index(a, a + left);
+        } else if (q < NP + N) {
+            to = kGramPairs + q - NP;
+        }
+        partials[(int64_t)blockIdx.x * kGramSums + to] = t;
     }
 }
 
@@ -284,6 +319,9 @@ struct Coefs {
 };
 
 // u = u0 + sum_i c_i d_i on the interior
+// (N: directions; one loop over all the places, whose unused ones' FP64
+// instructions are issued all the same, took 1.11 ms at 8192^2 with one, now 0.25)
+template <int N>
 __global__ void k_combine(Geo g, const double *__restrict__ u0, Dirs D, Coefs C, double *__restrict__ u) {
     const long long n = (long long)g.nx * g.ny;
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n;
@@ -292,8 +330,7 @@ __global__ void k_combine(Geo g, const double *__restrict__ u0, Dirs D, Coefs C,
         const int64_t c = cell_of(g, k, &i, &j);
         double v = u0[c];
 #pragma unroll
-        for (int a = 0; a < kMaxDirs; ++a)
-            if (a < D.n) v = fma(C.c[a], D.d[a][c], v);
+        for (int a = 0; a < N; ++a) v = fma(C.c[a], D.d[a][c], v);
         u[c] = v;
     }
 }
@@ -444,6 +481,23 @@ double project(const double *S, int n, double *coef) {
     return gain;
 }
 
+// k_gram of D.n directions
+template <int N = 1>
+void launch_gram(Chunk *c, Warm *w, const Dirs &D) {
+    if constexpr (N < kMaxDirs)
+        if (D.n > N) return launch_gram<N + 1>(c, w, D);
+    auto kernel = c->warm_projection == TL_WARM_PROJ_RESIDUAL ? k_gram<true, N> : k_gram<false, N>;
+    kernel<<<kGramBlocks, 256, 0, c->stream>>>(c->g, D, w->r0, c->diag, c->kx, c->ky, w->partials);
+}
+
+// k_combine of D.n directions
+template <int N = 0>
+void launch_combine(Chunk *c, const Dirs &D, const Coefs &C, double *u) {
+    if constexpr (N < kMaxDirs)
+        if (D.n > N) return launch_combine<N + 1>(c, D, C, u);
+    k_combine<N><<<1216, 256, 0, c->stream>>>(c->g, c->u0, D, C, u);
+}
+
 // Gram sums of the directions D (k_gram, partials summed on the host in CTA
 // order) and their projection: coefficients into *C, twice the energy
 // decrease into *gain (0 when D is empty or nothing helps)
@@ -453,16 +507,14 @@ int gram_project(Chunk *c, Warm *w, const Dirs &D, Coefs *C, double *gain) {
     if (D.n == 0) return TL_OK;
     cudaStream_t s = c->stream;
     int rc;
-    if (c->warm_projection == TL_WARM_PROJ_RESIDUAL)
-        k_gram<true><<<kGramBlocks, 256, 0, s>>>(c->g, D, w->r0, c->diag, c->kx, c->ky, w->partials);
-    else
-        k_gram<false><<<kGramBlocks, 256, 0, s>>>(c->g, D, w->r0, c->diag, c->kx, c->ky, w->partials);
+    launch_gram(c, w, D);
     if ((rc = launched(c, "gram launch"))) return rc;
     std::vector<double> part((size_t)kGramBlocks * kGramSums);
     TL_CUDA(cudaMemcpyAsync(part.data(), w->partials, sizeof(double) * part.size(), cudaMemcpyDeviceToHost, s));
     TL_CUDA(cudaStreamSynchronize(s));
     double S[kGramSums];
     for (int q = 0; q < kGramSums; ++q) S[q] = 0.0;
+    // (those of directions beyond D.n are not written, nor read by project)
     for (int b = 0; b < kGramBlocks; ++b)
         for (int q = 0; q < kGramSums; ++q) S[q] += part[(size_t)b * kGramSums + q];
     *gain = project(S, D.n, C->c);
@@ -591,8 +643,7 @@ int warm_start_or_fallback(Chunk *c, tl_solve_info_t *info, double *r0, double *
     Coefs CH;
     double gh = 0.0;
     if ((rc = gram_project(c, w, H, &CH, &gh))) return rc;
-    if (gh > 0.0) k_combine<<<1216, 256, 0, s>>>(c->g, c->u0, H, CH, w->ustart);
-    else k_combine<<<1216, 256, 0, s>>>(c->g, c->u0, Dirs{{nullptr}, 0}, CH, w->ustart);
+    launch_combine(c, gh > 0.0 ? H : Dirs{{nullptr}, 0}, CH, w->ustart);
     if ((rc = launched(c, "history start"))) return rc;
     Dirs D = H;
     Coefs C = CH;
@@ -625,7 +676,7 @@ int warm_start_or_fallback(Chunk *c, tl_solve_info_t *info, double *r0, double *
     *r0 = sqrt(fabs(rr0));
     *rr = rr0;
     if (!(gain > 0.0)) return TL_OK;  // the plain start: u = u^n, r = r0
-    k_combine<<<1216, 256, 0, s>>>(c->g, c->u0, D, C, c->u);
+    launch_combine(c, D, C, c->u);
     if ((rc = launched(c, "warm start combine"))) return rc;
     if ((rc = launch_residual(c, kEpiStore))) return rc;
     if ((rc = chunk_sync_scalars(c))) return rc;
