@@ -42,17 +42,37 @@ __device__ __forceinline__ uint32_t pack2(bf16 lo, bf16 hi) {
     return (uint32_t)__bfloat16_as_ushort(lo) | ((uint32_t)__bfloat16_as_ushort(hi) << 16);
 }
 
-// GELU, tanh form: 0.5 x (1 + tanh(sqrt(2/pi) (x + 0.044715 x^3)))
-constexpr float kG0 = 0.7978845608028654f, kG1 = 0.044715f;
-__device__ __forceinline__ float gelu(float x) {
-    const float u = kG0 * (x + kG1 * x * x * x);
-    return 0.5f * x * (1.f + tanhf(u));
+// GELU, tanh form: 0.5 x (1 + tanh(u)) = x / (1 + exp(-2 u)), u = sqrt(2/pi) (x + 0.044715 x^3).
+// With e = exp(-2 |u|) in (0, 1]: x - x e / (1 + e) for x > 0, |x| e / (1 + e) below
+// zero.  11 instructions with the hardware's exponential and reciprocal where
+// tanhf takes some 50, which bound the convolutions; its largest error
+// against FP64 over -20..20 is 2.4e-7 (with tanhf, whose 1 + tanh cancels
+// for x < 0: 4.3e-7), the root mean square lower too.
+__device__ __forceinline__ float exp2_hw(float x) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
 }
+__device__ __forceinline__ float rcp_hw(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+constexpr float kG0 = 0.7978845608028654f, kG1 = 0.044715f;
+constexpr float kE0 = (float)(2.0 * 0.7978845608028654 * 1.4426950408889634);  // 2 sqrt(2/pi) log2(e)
+constexpr float kE1 = (float)(2.0 * 0.7978845608028654 * 1.4426950408889634 * 0.044715);
+__device__ __forceinline__ float gelu(float x) {
+    float a;  // |x|, finite for x = inf (whose e is 0); NaN stays
+    asm("min.NaN.f32 %0, %1, 0f7F7FFFFF;" : "=f"(a) : "f"(x));
+    a = fabsf(a);
+    const float e = exp2_hw(-a * fmaf(kE1, x * x, kE0));
+    return fmaf(-a, e * rcp_hw(1.f + e), fmaxf(x, 0.f));
+}
+// s + 2 x s (1 - s) u' with s = 1 / (1 + exp(-2 u)), s (1 - s) = e / (1 + e)^2
 __device__ __forceinline__ float gelu_grad(float x) {
-    const float u = kG0 * (x + kG1 * x * x * x);
-    const float th = tanhf(u);
-    const float du = kG0 * (1.f + 3.f * kG1 * x * x);
-    return 0.5f * (1.f + th) + 0.5f * x * (1.f - th * th) * du;
+    const float x2 = x * x, e = exp2_hw(-fabsf(x) * fmaf(kE1, x2, kE0));
+    const float r = rcp_hw(1.f + e), er = e * r;
+    return fmaf((x * er) * r, fmaf(6.f * kG0 * kG1, x2, 2.f * kG0), x < 0.f ? er : r);
 }
 
 enum ConvMode { kModeGelu = 0, kModeGeluRes = 1, kModeHead = 2, kModeLinear = 3 };
@@ -127,34 +147,46 @@ __global__ void __launch_bounds__(128) k_conv(const bf16 *__restrict__ in, const
 }
 
 // ---------------------------------------------------------------------------
-// The same convolution on the 5th-generation tensor cores (tcgen05).  Pixels are
-// counted over the padded rows, q = y (W + 2) + x: the input of tap (dy, dx) is
-// then q + dy (W + 2) + dx and the output q + (W + 2) + 1, whatever the row, so
-// a tile is any 128 consecutive q (M = 128) for all COUTP output channels (N),
-// and the two columns a row that are no output are all that is computed in
-// vain (1.4 % at W = 144, where tiles of one row's pixels wasted 44 %).
+// The same convolution on the 5th-generation tensor cores (tcgen05).  A tile is
+// 128 columns (M = 128) of kTcRows output rows.  Columns are counted over the
+// padded rows of a group of kTcRows rows and on into the next group, q = group
+// (W + 2) + x, and a tile is any 128 consecutive q, so the two columns a row
+// that are no output are all that is computed in vain (1.4 % at W = 144, where
+// tiles of one row's pixels wasted 44 %).  W + 2 is even: an even q and the
+// next are neighbours in memory.
 //
 // A CTA of 4 warps walks tiles: the weights stay in shared memory, and the next
-// tile's input is on its way (cp.async, two buffers) while this one multiplies
-// and is written.  Shared memory holds, per kernel row dy, the 130 input pixels
+// tile's input is on its way (cp.async) while this one's result is written.
+// Shared memory holds, per input row k of kTcRows + 2, the 130 input pixels that
 // the three taps dx = 0, 1, 2 read, in the K-major no-swizzle layout of the MMA
 // operands: 16-byte core-matrix rows (one pixel, 8 channels), the pixels of
 // an 8-channel chunk contiguous (16 bytes apart) and the chunks kChunkA bytes
-// apart.  The A operand of tap (dy, dx) and 16-channel step kk is that block
+// apart.  The A operand of input row k, dx and 16-channel step kk is that block
 // shifted by dx pixels: start + dx * 16, core matrices 128 bytes apart along
-// M (SBO) and kChunkA along K (LBO).  The weights [tap][cout][cin] sit in the
-// same layout (cout rows 16 bytes apart, chunks 16 * COUTP apart).  One
-// thread issues the 9 * CIN / 16 MMAs (M 128, N COUTP, K 16, BF16 in, FP32
-// accumulate) and commits them to an mbarrier; each warp then reads its 32
-// TMEM lanes (one pixel a lane, one channel a column) and runs the epilogue
-// of k_conv.  Lanes trade half of their chunks with their neighbours before a
-// store, so that every store writes whole 32-byte sectors.
-// What bounds it: HBM for a layer's activations (64 bytes a pixel in and 64 or
-// 128 out).
+// M (SBO) and kChunkA along K (LBO).  The weights sit in the same layout, per
+// dx, with the couts of dy = 2, 1, 0 one after the other along N (16 bytes
+// apart): input row k is the dy = 2, 1, 0 neighbour of the output rows k - 2,
+// k - 1 and k, whose accumulators lie side by side in the same order, so that one
+// MMA adds it to all three (N = 3 COUTP; fewer at the tile's first and last rows).
+// One thread issues the MMAs (M 128, K 16, BF16 in, FP32 accumulate) and commits
+// them to an mbarrier; each warp then reads its 32 TMEM lanes (one pixel a
+// lane, one channel a column) row by row and runs the epilogue of k_conv.
+// Lanes trade half of their chunks with their neighbours before a store, so
+// that every store writes whole 32-byte sectors.
+// What bounds it: latency, with three CTAs (12 warps) a multiprocessor that wait
+// for their loads between the MMAs and the epilogue; then L2, from which an
+// input row is read (kTcRows + 2) / kTcRows times (tensor cores 11-15 % busy,
+// HBM 29 %).  4096 x 4096 pixels, 32 to 32 channels with GELU and the input
+// added: 947 us, HBM's 2.1 GB take 317.  One row a tile (three reads): two
+// buffers and 3 CTAs 1250, one buffer and 5 CTAs 1090; two rows and 4 CTAs 930,
+// but 605 for the head where four rows take 527; three rows 986.  32 x 144 x 144
+// pixels with the pre-activation written: one row 64 and 58, two 53, four 53 us.
+constexpr int kTcRows = 4;                // output rows of a tile (above: 1 to 4 measured)
 constexpr int kTcPix = 128;               // pixels of a tile (MMA M)
 constexpr int kTcRow = kTcPix + 2;        // input pixels a kernel row of a tile reads
 constexpr int kChunkA = kTcRow * 16;      // bytes between 8-channel chunks of A
-constexpr int kTmemCols = 32;             // accumulator columns allocated (>= COUTP)
+constexpr int kTmemCols = 32 * kTcRows;   // accumulator columns allocated (>= kTcRows COUTP)
+constexpr int kTcCtas = 3;                // CTAs a multiprocessor (68 KB of shared memory each)
 constexpr long long kTcWaitCycles = 2000000000LL;  // ~1 s: the MMA wait gives up after this
 
 // set by a tcgen05 conv whose MMA completion wait ran out (read and cleared
@@ -232,7 +264,7 @@ __device__ __forceinline__ void tmem_load<16>(uint32_t taddr, float (&v)[16]) {
 
 template <int CIN, int COUTP>
 constexpr int conv_tc_smem() {
-    return 2 * 3 * (CIN / 8) * kChunkA + 9 * (CIN / 8) * COUTP * 16;
+    return (kTcRows + 2) * (CIN / 8) * kChunkA + 9 * (CIN / 8) * COUTP * 16;
 }
 
 // store 8 channels a lane of COUTP, `at` the lane's pixel: two chunks of the
@@ -257,23 +289,26 @@ __device__ __forceinline__ void store_chunks(bf16 *dst, long long at, int chunk,
 }
 
 template <int CIN, int COUTP, int MODE>
-__global__ void __launch_bounds__(128) k_conv_tc(const bf16 *__restrict__ in, const bf16 *__restrict__ wt,
+__global__ void __launch_bounds__(128, kTcCtas) k_conv_tc(const bf16 *__restrict__ in, const bf16 *__restrict__ wt,
                                                  const float *__restrict__ bias,
                                                  const bf16 *__restrict__ res, bf16 *__restrict__ out,
                                                  bf16 *__restrict__ pre, float *__restrict__ outf, int B,
                                                  int H, int W) {
-    static_assert(CIN % 16 == 0 && COUTP % 16 == 0 && COUTP <= kTmemCols, "conv shape");
+    static_assert(CIN % 16 == 0 && COUTP % 16 == 0 && kTcRows * COUTP <= kTmemCols, "conv shape");
     constexpr int CA = CIN / 8;                    // 8-channel chunks of a pixel
-    constexpr int CHUNK_B = COUTP * 16;            // bytes between chunks of the weights
-    constexpr int A_BYTES = 3 * CA * kChunkA;      // three kernel rows
+    constexpr int CHUNK_B = 3 * COUTP * 16;        // bytes between chunks of the weights
+    constexpr int R = kTcRows;
+    constexpr int A_BYTES = (R + 2) * CA * kChunkA;
     extern __shared__ __align__(128) unsigned char conv_smem[];
-    unsigned char *const sb = conv_smem + 2 * A_BYTES;
+    unsigned char *const sb = conv_smem + A_BYTES;
     __shared__ __align__(8) uint64_t mbar;
     __shared__ uint32_t tmem_slot;
+    __shared__ __align__(16) float sbias[COUTP];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int Wp = W + 2;
-    const long long npix = (long long)H * Wp, in_pix = (long long)(H + 2) * Wp;  // q range, padded image
-    const long long per_image = (npix + kTcPix - 1) / kTcPix, tiles = per_image * B;
+    const long long npix = (long long)((H + R - 1) / R) * Wp, in_pix = (long long)(H + 2) * Wp;  // q range, padded image
+    // (tiles count in 32 bits: 2^32 of them would be 2^39 pixels)
+    const unsigned int per_image = (unsigned int)((npix + kTcPix - 1) / kTcPix), tiles = per_image * (unsigned int)B;
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -286,50 +321,53 @@ __global__ void __launch_bounds__(128) k_conv_tc(const bf16 *__restrict__ in, co
         // the tensor cores arrive on it: make the initialisation visible to them
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    // A: padded pixels q0 + dy Wp + 0..129, 16 bytes a copy; pixels past the
-    // image read as zero (last tile)
-    auto stage = [&](long long t, int buf) {
-        const int b = (int)(t / per_image);
-        const long long q0 = (t - b * per_image) * kTcPix;
+    // row group and column of q
+    auto place = [&](long long q, int &y, int &x) {
+        const int gr = npix >> 31 ? (int)(q / Wp) : (int)((unsigned int)q / (unsigned int)Wp);
+        x = (int)(q - (long long)gr * Wp);
+        y = gr * R;
+    };
+    // A: pixels q0 + 0..129 of R + 2 input rows, 16 bytes a copy; those past
+    // the image read as zero (last tiles)
+    auto stage = [&](unsigned int t) {
+        const unsigned int b = t / per_image;
+        const long long q0 = (long long)(t - b * per_image) * kTcPix;
         const bf16 *img = in + (long long)b * in_pix * CIN;
-        const uint32_t dst = smem_addr(conv_smem) + buf * A_BYTES;
+        const uint32_t dst = smem_addr(conv_smem);
         // a thread copies chunk tid % CA of every 128 / CA-th pixel
         constexpr int PX = 128 / CA;
         const int c = tid % CA, j0 = tid / CA;
-        const bf16 *src = img + (q0 + j0) * CIN + 8 * c;
-        const bool inside = q0 + 2LL * Wp + kTcRow <= in_pix;  // all but an image's last tiles
+        int y, x;
+        place(q0 + j0, y, x);
 #pragma unroll
-        for (int dy = 0; dy < 3; ++dy) {
-            const uint32_t d0 = dst + (dy * CA + c) * kChunkA + j0 * 16;
-            const bf16 *s0 = src + (long long)dy * Wp * CIN;
+        for (int i = 0; i < (kTcRow + PX - 1) / PX; ++i) {
+            if ((i + 1) * PX > kTcRow && j0 + i * PX >= kTcRow) break;
+            const bf16 *src = img + ((long long)y * Wp + x) * CIN + 8 * c;
+            const uint32_t d = dst + c * kChunkA + (j0 + i * PX) * 16;
 #pragma unroll
-            for (int i = 0; i < (kTcRow + PX - 1) / PX; ++i) {
-                if ((i + 1) * PX > kTcRow && j0 + i * PX >= kTcRow) break;
-                const bool ok = inside || q0 + (long long)dy * Wp + j0 + i * PX < in_pix;
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d0 + i * PX * 16),
-                             "l"(ok ? s0 + i * PX * CIN : img), "r"(ok ? 16 : 0));
+            for (int k = 0; k < R + 2; ++k) {
+                const bool ok = y + k < H + 2;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d + k * CA * kChunkA),
+                             "l"(ok ? src + (long long)k * Wp * CIN : img), "r"(ok ? 16 : 0));
             }
+            for (x += PX; x >= Wp; x -= Wp) y += R;
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    long long t = blockIdx.x;
-    if (t < tiles) stage(t, 0);
+    unsigned int t = blockIdx.x;
+    if (t < tiles) stage(t);
+    if (MODE != kModeLinear && tid < (MODE == kModeHead ? 1 : COUTP)) sbias[tid] = bias[tid];
     // B: weights [tap][cout][cin]
     for (int k = tid; k < 9 * COUTP * CA; k += 128) {
         const int c = k % CA, co = (k / CA) % COUTP, tap = k / (CA * COUTP);
         const uint4 v = *reinterpret_cast<const uint4 *>(wt + ((long long)tap * COUTP + co) * CIN + 8 * c);
-        *reinterpret_cast<uint4 *>(sb + (tap * CA + c) * CHUNK_B + co * 16) = v;
+        *reinterpret_cast<uint4 *>(sb + ((tap % 3) * CA + c) * CHUNK_B + ((2 - tap / 3) * COUTP + co) * 16) = v;
     }
     const uint32_t bar = smem_addr(&mbar);
     uint32_t tmem = 0, phase = 0;
     bool ok = true;
-    for (int buf = 0; t < tiles; t += gridDim.x, buf ^= 1, phase ^= 1) {
-        if (t + gridDim.x < tiles) {
-            stage(t + gridDim.x, buf ^ 1);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-        }
+    for (; t < tiles; t += gridDim.x, phase ^= 1) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
         // the MMAs read shared memory through the async proxy
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -337,40 +375,64 @@ __global__ void __launch_bounds__(128) k_conv_tc(const bf16 *__restrict__ in, co
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         tmem = tmem_slot;
         if (tid == 0) {
-            constexpr uint32_t idesc = mma_idesc(kTcPix, COUTP);
-            const uint32_t a0 = smem_addr(conv_smem) + buf * A_BYTES, b0 = smem_addr(sb);
+            const uint32_t a0 = smem_addr(conv_smem), b0 = smem_addr(sb);
+            // one MMA for the output rows lo..hi of an input row, dx and 16 channels
+            auto mma = [&](int k, int dx, int kk, int lo, int hi, uint32_t acc) {
+                const uint64_t ad = mma_desc(a0 + (k * CA + 2 * kk) * kChunkA + dx * 16, kChunkA, 128);
+                const uint64_t bd = mma_desc(b0 + (dx * CA + 2 * kk) * CHUNK_B + (2 - k + lo) * COUTP * 16, CHUNK_B, 128);
+                asm volatile(
+                    "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem + lo * COUTP),
+                    "l"(ad), "l"(bd), "r"(mma_idesc(kTcPix, (hi - lo + 1) * COUTP)), "r"(acc));
+            };
 #pragma unroll
-            for (int tap = 0; tap < 9; ++tap) {
-                const int dy = tap / 3, dx = tap % 3;
+            for (int k = 0; k < R + 2; ++k) {
+                const int lo = k < 2 ? 0 : k - 2, hi = k < R ? k : R - 1;
 #pragma unroll
-                for (int kk = 0; kk < CIN / 16; ++kk) {
-                    const uint64_t ad = mma_desc(a0 + (dy * CA + 2 * kk) * kChunkA + dx * 16, kChunkA, 128);
-                    const uint64_t bd = mma_desc(b0 + (tap * CA + 2 * kk) * CHUNK_B, CHUNK_B, 128);
-                    const uint32_t acc = (tap | kk) != 0 ? 1u : 0u;
-                    asm volatile(
-                        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-                        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
-                        "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
+                for (int q = 0; q < 3 * (CIN / 16); ++q) {
+                    const int dx = q % 3, kk = q / 3;
+                    if (q == 0 && k < R) {  // row k's first product; its accumulator is overwritten
+                        mma(k, dx, kk, k, k, 0u);
+                        if (lo < k) mma(k, dx, kk, lo, k - 1, 1u);
+                    } else {
+                        mma(k, dx, kk, lo, hi, 1u);
+                    }
                 }
             }
             asm volatile(
                 "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
                 : "memory");
         }
-        // this lane's pixel, while the tensor cores work
-        const int b = (int)(t / per_image);
-        const long long q = (t - b * per_image) * kTcPix + 32 * warp + lane;
-        const int x = (int)(q % Wp), y = (int)(q / Wp);
-        const bool valid = q < npix && x < W;
-        const bool pvalid = __shfl_xor_sync(0xffffffffu, (int)valid, 1) != 0;
-        const long long o = (long long)b * in_pix + q + Wp + 1;
-        uint4 rv[COUTP / 8];
+        // this lane's pixels, while the tensor cores work
+        const unsigned int b = t / per_image;
+        int x, y;
+        const long long q = (long long)(t - b * per_image) * kTcPix + 32 * warp + lane;
+        place(q, y, x);
+        const bool column = q < npix && x < W;
+        const long long o0 = (long long)b * in_pix + (long long)(y + 1) * Wp + x + 1;
+        uint4 rv[R][COUTP / 8];
         const bool add = (MODE == kModeGeluRes || MODE == kModeLinear) && res;
+        // what is added: where it is the input itself, the staged centre tap's
+        // pixels (below), else from memory
+        const bool own = add && CIN == COUTP && res == in;
+        if (add && !own) {
 #pragma unroll
-        for (int h = 0; h < COUTP / 8; ++h)
-            if (add && valid) rv[h] = *reinterpret_cast<const uint4 *>(res + o * COUTP + 8 * h);
+            for (int row = 0; row < R; ++row)
+#pragma unroll
+                for (int h = 0; h < COUTP / 8; ++h)
+                    if (column && y + row < H)
+                        rv[row][h] = *reinterpret_cast<const uint4 *>(res + (o0 + (long long)row * Wp) * COUTP + 8 * h);
+        }
         // warp-uniform outcome: tcgen05.ld below is executed by whole warps
         ok = __all_sync(0xffffffffu, mbar_wait_bounded(bar, phase));
+        if (own) {
+            const uint4 *centre = reinterpret_cast<const uint4 *>(conv_smem + CA * kChunkA);
+#pragma unroll
+            for (int row = 0; row < R; ++row)
+#pragma unroll
+                for (int h = 0; h < COUTP / 8; ++h)
+                    rv[row][h] = centre[(row * CA + h) * (kChunkA / 16) + 32 * warp + lane + 1];
+        }
         if (!__syncthreads_and(ok)) {
             // the accumulator never became ready: flag it, wait once more
             // (bounded) for the MMAs in flight, release the columns and leave
@@ -379,47 +441,55 @@ __global__ void __launch_bounds__(128) k_conv_tc(const bf16 *__restrict__ in, co
             break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        // warp w holds TMEM lanes 32w..32w+31: pixel m = 32 w + lane
-        float acc[COUTP];
-        tmem_load<COUTP>(tmem + ((uint32_t)(32 * warp) << 16), acc);
-        if (MODE == kModeHead) {
-            if (valid) outf[((long long)b * H + y) * W + x] = acc[0] + bias[0];
-        } else {
+        // the next tile's input is on its way while this one is written
+        if (t + gridDim.x < tiles) stage(t + gridDim.x);
 #pragma unroll
-            for (int q2 = 0; q2 < COUTP / 8; q2 += 2) {
-                uint32_t pk[2][4];
-                if (MODE == kModeGelu || MODE == kModeGeluRes) {
+        for (int row = 0; row < R; ++row, ++y) {
+            const bool valid = column && y < H;
+            const bool pvalid = __shfl_xor_sync(0xffffffffu, (int)valid, 1) != 0;
+            const long long o = o0 + (long long)row * Wp;
+            // warp w holds TMEM lanes 32w..32w+31: pixel m = 32 w + lane
+            float acc[COUTP];
+            tmem_load<COUTP>(tmem + row * COUTP + ((uint32_t)(32 * warp) << 16), acc);
+            if (MODE == kModeHead) {
+                if (valid) outf[((long long)b * H + y) * W + x] = acc[0] + sbias[0];
+            } else {
+#pragma unroll
+                for (int q2 = 0; q2 < COUTP / 8; q2 += 2) {
+                    uint32_t pk[2][4];
+                    if (MODE == kModeGelu || MODE == kModeGeluRes) {
+#pragma unroll
+                        for (int h = 0; h < 2; ++h)
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                float &v0 = acc[8 * (q2 + h) + 2 * e], &v1 = acc[8 * (q2 + h) + 2 * e + 1];
+                                v0 += sbias[8 * (q2 + h) + 2 * e];
+                                v1 += sbias[8 * (q2 + h) + 2 * e + 1];
+                                pk[h][e] = pack2(__float2bfloat16(v0), __float2bfloat16(v1));
+                                v0 = gelu(v0);
+                                v1 = gelu(v1);
+                            }
+                        if (pre) store_chunks<COUTP>(pre, o, q2, pk[0], pk[1], valid, pvalid, lane);
+                    }
+                    if (add && valid) {
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const uint32_t rw[4] = {rv[row][q2 + h].x, rv[row][q2 + h].y, rv[row][q2 + h].z, rv[row][q2 + h].w};
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                acc[8 * (q2 + h) + 2 * e] += __uint_as_float(rw[e] << 16);
+                                acc[8 * (q2 + h) + 2 * e + 1] += __uint_as_float(rw[e] & 0xFFFF0000u);
+                            }
+                        }
+                    }
 #pragma unroll
                     for (int h = 0; h < 2; ++h)
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            float &v0 = acc[8 * (q2 + h) + 2 * e], &v1 = acc[8 * (q2 + h) + 2 * e + 1];
-                            v0 += bias[8 * (q2 + h) + 2 * e];
-                            v1 += bias[8 * (q2 + h) + 2 * e + 1];
-                            pk[h][e] = pack2(__float2bfloat16(v0), __float2bfloat16(v1));
-                            v0 = gelu(v0);
-                            v1 = gelu(v1);
-                        }
-                    if (pre) store_chunks<COUTP>(pre, o, q2, pk[0], pk[1], valid, pvalid, lane);
+                        for (int e = 0; e < 4; ++e)
+                            pk[h][e] = pack2(__float2bfloat16(acc[8 * (q2 + h) + 2 * e]),
+                                             __float2bfloat16(acc[8 * (q2 + h) + 2 * e + 1]));
+                    store_chunks<COUTP>(out, o, q2, pk[0], pk[1], valid, pvalid, lane);
                 }
-                if (add && valid) {
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const uint32_t rw[4] = {rv[q2 + h].x, rv[q2 + h].y, rv[q2 + h].z, rv[q2 + h].w};
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            acc[8 * (q2 + h) + 2 * e] += __uint_as_float(rw[e] << 16);
-                            acc[8 * (q2 + h) + 2 * e + 1] += __uint_as_float(rw[e] & 0xFFFF0000u);
-                        }
-                    }
-                }
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
-#pragma unroll
-                    for (int e = 0; e < 4; ++e)
-                        pk[h][e] = pack2(__float2bfloat16(acc[8 * (q2 + h) + 2 * e]),
-                                         __float2bfloat16(acc[8 * (q2 + h) + 2 * e + 1]));
-                store_chunks<COUTP>(out, o, q2, pk[0], pk[1], valid, pvalid, lane);
             }
         }
     }
@@ -738,8 +808,8 @@ int launch_conv(const void *in, const void *w, const float *bias, const void *re
         const cudaError_t e = cudaFuncSetAttribute(k_conv_tc<CIN, COUTP, MODE>,
                                                    cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
         if (e != cudaSuccess) return cuda_fail(e, "conv shared memory");
-        const long long tiles = (((long long)H * (W + 2) + kTcPix - 1) / kTcPix) * B;
-        const long long ctas = 152 * 3;  // 3 CTAs of 68 KB a multiprocessor
+        const long long tiles = (((long long)((H + kTcRows - 1) / kTcRows) * (W + 2) + kTcPix - 1) / kTcPix) * B;
+        const long long ctas = 152 * kTcCtas;
         k_conv_tc<CIN, COUTP, MODE><<<(unsigned)(tiles < ctas ? tiles : ctas), 128, bytes, s>>>(
             (const bf16 *)in, (const bf16 *)w, bias, (const bf16 *)res, (bf16 *)out, (bf16 *)pre, outf, B, H, W);
     } else {

@@ -81,11 +81,12 @@ def test_gelu_gradient_wide_and_narrow_loads_agree(ch, shape, offset):
 
 
 @pytest.mark.parametrize("cin,cout,mode", [(16, 32, 0), (32, 32, 1), (32, 16, 2), (16, 32, 3), (32, 32, 3)])
-@pytest.mark.parametrize("shape", [(1, 1, 16), (1, 7, 16), (2, 3, 112), (1, 2, 128), (3, 160, 144)])
+@pytest.mark.parametrize("shape", [(1, 1, 16), (1, 7, 16), (2, 3, 112), (1, 2, 128), (2, 4, 48), (1, 9, 256),
+                                   (3, 160, 144)])
 @pytest.mark.parametrize("with_pre", [True, False])
 def test_tensor_memory_conv_tiles(cin, cout, mode, shape, with_pre):
-    """tiles of 128 pixels across the rows' ends and the image's, one and several a thread block, against the
-    warp-level kernel: BF16 outputs within one rounding (2^-7), the FP32 head within its sum's rounding; the
+    """tiles of 128 columns by 4 rows across the rows' ends and the image's, one and several a thread block,
+    the input itself added (where it has the channels) and another array, against the warp-level kernel: BF16 outputs within one rounding (2^-7), the FP32 head within its sum's rounding; the
     halo and what lies behind the buffers stay as they are"""
     torch = pytest.importorskip("torch")
     lib = tl.load()
@@ -93,6 +94,8 @@ def test_tensor_memory_conv_tiles(cin, cout, mode, shape, with_pre):
     B, H, W = shape
     gen = torch.Generator(device="cuda").manual_seed(3 * cin + cout + mode + W)
     x, res = _field(torch, shape, cin, 0, gen), _field(torch, shape, cout, 0, gen)
+    if cin == cout and with_pre:
+        res = x
     w = (0.2 * torch.randn((9, cout, cin), generator=gen, device="cuda")).bfloat16()
     bias = 0.1 * torch.randn(cout, generator=gen, device="cuda")
     got = {}
@@ -114,3 +117,43 @@ def test_tensor_memory_conv_tiles(cin, cout, mode, shape, with_pre):
             assert float(t[:, 0].abs().sum() + t[:, -1].abs().sum() + t[:, :, 0].abs().sum() + t[:, :, -1].abs().sum()) == 0
     for a, b in zip(got[1], got[0]):
         assert bool(((a - b).abs() <= 2.0 ** -7 * b.abs() + 1e-5).all())
+
+
+def test_gelu_and_its_gradient_against_fp64():
+    """through a convolution with zero weights, whose pre-activations are the bias, over the range where the
+    function bends, zeros, infinities and NaN.  Bound: BF16 rounding of the result (8 significant bits: 2^-8) and 1e-6 of FP32
+    arithmetic (a dozen roundings of values up to 20)"""
+    torch = pytest.importorskip("torch")
+    lib = tl.load()
+    lib.tl_nn_set_conv_kernel.argtypes = [C.c_int]
+    inf, nan = float("inf"), float("nan")
+    v = torch.cat([torch.linspace(-20, 20, 4001), torch.linspace(-2, 2, 4001),
+                   torch.tensor([0.0, -0.0, 1e-30, -1e-30, 1e18, -1e18, inf, -inf, nan])]).cuda()
+    v = torch.cat([v, v.new_zeros(-len(v) % 32)])
+    x, w = (torch.zeros(s, dtype=torch.bfloat16, device="cuda") for s in ((1, 3, 18, 32), (9, 32, 32)))
+    g = lambda u: u / (1 + torch.exp(-2 * (2 / torch.pi) ** 0.5 * (u + 0.044715 * u ** 3)))
+    for tc in (1, 0):
+        got = []
+        for k in range(0, len(v), 32):
+            out = torch.zeros_like(x)
+            lib.tl_nn_set_conv_kernel(tc)
+            rc = lib.tl_nn_conv(0, 32, 32, _p(x), _p(w), _p(v[k:k + 32]), None, _p(out), None, None, 1, 1, 16, None)
+            lib.tl_nn_set_conv_kernel(1)
+            assert rc == 0, tl.last_error()
+            got.append(out[0, 1, 5])
+        got = torch.cat(got).double()
+        fin = v.abs() < 1e10
+        want = g(v.double()[fin])
+        assert bool(((got[fin] - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6).all())
+        big = got[v == 1e18]
+        assert float((big - 1e18).abs().max()) <= 2.0 ** -8 * 1e18 and float(got[v == -1e18].abs().max()) == 0.0
+        assert float(got[v == inf][0]) == inf and bool(got[v == -inf].isnan().all() and got[v.isnan()].isnan().all())
+    pre = v[fin].bfloat16()
+    n = len(pre)
+    a, b, o = (torch.zeros((1, 3, n + 2, 1), dtype=torch.bfloat16, device="cuda") for _ in range(3))
+    a[0, 1, 1:-1, 0], b[0, 1, 1:-1, 0] = 1.0, pre
+    assert lib.tl_nn_gelu_backward(_p(a), _p(b), _p(o), 1, 1, 1, n, None) == 0
+    u = pre.double().requires_grad_()
+    g(u).sum().backward()
+    want = torch.where(u.grad.isnan(), torch.zeros_like(u), u.grad)  # exp overflows far below zero: the limit
+    assert bool(((o[0, 1, 1:-1, 0].double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6).all())
