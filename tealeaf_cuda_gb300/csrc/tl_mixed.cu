@@ -636,6 +636,12 @@ __global__ void __launch_bounds__(kBlockThreads) k_pp_step(
 // stored) and is updated in place.  Every value is computed with the
 // operations of k_pp_step in the same order, so T fused steps give the bits
 // of T single steps.
+// What bounds it: the latency of shared memory and of the chain through the
+// levels, with 12 warps a multiprocessor (168 registers a thread): issue slots
+// and shared memory are each half used, HBM 40 %.  (8192^2 cells, block-Jacobi,
+// 5 steps: 692 us; with the pairs (0, 1) and (2, 3), whose neighbours are not
+// pairs, and Ky above a strip read from shared memory: 716.  r - alpha w formed in
+// the first pass instead of by a pass of its own: 130 us more a pass.)
 constexpr int kFusedPrefetch = 1;  // strips beyond the next one that are prefetched into L2
 
 // CTA width (threads = columns) of a T-step pass.  Two CTAs run on an SM;
@@ -737,9 +743,12 @@ __host__ __device__ constexpr size_t fused_smem() {
     return sizeof(float4) * (fused_threads<T>() + 2) * (fused_narr<PC>() * (T + 1) + 2 * T);
 }
 
-// row k (0..3, known at compile time) of a column's strip
+// a column's strip in a float4: rows 0, 2, 1, 3, so that the pairs (0, 2) and
+// (1, 3), which are each other's neighbours above and below, are register pairs
+__device__ __forceinline__ float4 rows4(const float (&v)[4]) { return make_float4(v[0], v[2], v[1], v[3]); }
+// row k (0..3, known at compile time) of it
 __device__ __forceinline__ float row_of(const float4 &v, int k) {
-    return k == 0 ? v.x : (k == 1 ? v.y : (k == 2 ? v.z : v.w));
+    return k == 0 ? v.x : (k == 1 ? v.z : (k == 2 ? v.y : v.w));
 }
 
 // Paired FP32 arithmetic (f32x2): two rows of a strip in one instruction,
@@ -774,7 +783,7 @@ __device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
     return r;
 }
-// cell_apply on rows (k, k+1): the same four fused steps in the same order
+// cell_apply on two rows: the same four fused steps in the same order
 __device__ __forceinline__ f2 cell_apply2(f2 c, f2 n, f2 s, f2 w, f2 e, f2 kyn, f2 kyc, f2 kxe, f2 kxc) {
     f2 v = fma2(kyn, sub2(c, n), c);
     v = fma2(kyc, sub2(c, s), v);
@@ -950,11 +959,11 @@ __global__ void __launch_bounds__(fused_threads<T>(), 2) k_pp_fused(PpFusedArgs 
             }
             {
                 float4 *cf = cfb + slot * NA * SR + tid;
-                xsb[(s & 1) * SR + tid] = make_float4(s0[0], s0[1], s0[2], s0[3]);
+                xsb[(s & 1) * SR + tid] = rows4(s0);
 #pragma unroll
-                for (int q = 0; q < NA; ++q)
-                    cf[q * SR] = make_float4(ld.ldC[q][0], ld.ldC[q][1], ld.ldC[q][2], ld.ldC[q][3]);
+                for (int q = 0; q < NA; ++q) cf[q * SR] = rows4(ld.ldC[q]);
             }
+            const float ky_s = ld.ldC[1][0];  // Ky below strip s
             if (s + 1 < s_end) load(s + 1, ld);
             if (s + 1 + kFusedPrefetch < s_end) prefetch(s + 1 + kFusedPrefetch);
             // levels 1..T; FULL: every level's strip lies in the field and has 4
@@ -964,6 +973,7 @@ __global__ void __launch_bounds__(fused_threads<T>(), 2) k_pp_fused(PpFusedArgs 
             auto levels = [&](auto full) {
                 constexpr bool FULL = decltype(full)::value;
                 float cS[4], cR[4], cU[4];  // level t-1's output of this iteration
+                float ky_top = ky_s;        // and the Ky below its strip: the face above row 3 of level t's
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     cS[k] = s0[k];
@@ -975,7 +985,6 @@ __global__ void __launch_bounds__(fused_threads<T>(), 2) k_pp_fused(PpFusedArgs 
                     const int q = s - t;
                     const int m = FULL ? 4 : (q >= 0 && q < nstrips && incol) ? min(4, a.ny - 4 * q) : 0;
                     const int sq = slot - t < 0 ? slot - t + R : slot - t;  // ring slot of strip q
-                    const int sn = sq + 1 == R ? 0 : sq + 1;                  // and of strip q + 1
                     const float4 *cf = cfb + sq * NA * SR + tid;
                     const float4 *xp = xsb + ((t - 1) * 2 + ((s - 1) & 1)) * SR + tid;
                     const float(&x0)[4] = in.sdP[t - 1];
@@ -983,26 +992,24 @@ __global__ void __launch_bounds__(fused_threads<T>(), 2) k_pp_fused(PpFusedArgs 
                     // the strip's coefficients, its west / east neighbours' sd and the
                     // east neighbour's Kx: one float4 (4 rows) each
                     const float4 kx4 = cf[0], ky4 = cf[SR], kxe4 = cf[1];
-                    const float ky_top = cfb[sn * NA * SR + SR + tid].x;  // the face above row 3
                     const float4 xw4 = xp[-1], xe4 = xp[1];
                     // one inner step on the strip's first mm rows (mm == 4: no row tests)
                     auto step = [&](const int mm) {
                         float z[4];
                         if (mm == 4) {
-                            // a full strip: the stencil of rows (0, 1) and (2, 3) as
+                            // a full strip: the stencil of rows (0, 2) and (1, 3) as
                             // f32x2 pairs
-                            const f2 c01 = pk2(x0[0], x0[1]), c23 = pk2(x0[2], x0[3]);
-                            const f2 x12 = pk2(x0[1], x0[2]);  // north of rows 0, 1 and south of rows 2, 3
-                            const f2 r01 = sub2(pk2(in.rtP[t - 1][0], in.rtP[t - 1][1]),
-                                                cell_apply2(c01, x12, pk2(in.sdL[t - 1], x0[0]), pk2(xw4.x, xw4.y),
-                                                            pk2(xe4.x, xe4.y), pk2(ky4.y, ky4.z), pk2(ky4.x, ky4.y),
+                            const f2 c02 = pk2(x0[0], x0[2]), c13 = pk2(x0[1], x0[3]);
+                            const f2 r02 = sub2(pk2(in.rtP[t - 1][0], in.rtP[t - 1][2]),
+                                                cell_apply2(c02, c13, pk2(in.sdL[t - 1], x0[1]), pk2(xw4.x, xw4.y),
+                                                            pk2(xe4.x, xe4.y), pk2(ky4.z, ky4.w), pk2(ky4.x, ky4.y),
                                                             pk2(kxe4.x, kxe4.y), pk2(kx4.x, kx4.y)));
-                            const f2 r23 = sub2(pk2(in.rtP[t - 1][2], in.rtP[t - 1][3]),
-                                                cell_apply2(c23, pk2(x0[3], cS[0]), x12, pk2(xw4.z, xw4.w),
-                                                            pk2(xe4.z, xe4.w), pk2(ky4.w, ky_top), pk2(ky4.z, ky4.w),
+                            const f2 r13 = sub2(pk2(in.rtP[t - 1][1], in.rtP[t - 1][3]),
+                                                cell_apply2(c13, pk2(x0[2], cS[0]), c02, pk2(xw4.z, xw4.w),
+                                                            pk2(xe4.z, xe4.w), pk2(ky4.y, ky_top), pk2(ky4.z, ky4.w),
                                                             pk2(kxe4.z, kxe4.w), pk2(kx4.z, kx4.w)));
-                            up2(r01, oR[0], oR[1]);
-                            up2(r23, oR[2], oR[3]);
+                            up2(r02, oR[0], oR[2]);
+                            up2(r13, oR[1], oR[3]);
                         } else {
 #pragma unroll
                         for (int k = 0; k < 4; ++k) {
@@ -1041,16 +1048,15 @@ __global__ void __launch_bounds__(fused_threads<T>(), 2) k_pp_fused(PpFusedArgs 
                             for (int k = 0; k < 4; ++k)
                                 if (k < mm) z[k] = oR[k];
                         }
-                        if (mm == 4 && !LAST) {
-                            // paired updates too, except in the last pass (whose FP64
-                            // stores leave no registers for them)
+                        if (mm == 4) {
+                            // paired updates too
                             const f2 al2 = pk2(al[t - 1], al[t - 1]), be2 = pk2(be[t - 1], be[t - 1]);
-                            const f2 s01 = fma2(al2, pk2(x0[0], x0[1]), mul2(be2, pk2(z[0], z[1])));
-                            const f2 s23 = fma2(al2, pk2(x0[2], x0[3]), mul2(be2, pk2(z[2], z[3])));
-                            up2(s01, oS[0], oS[1]);
-                            up2(s23, oS[2], oS[3]);
-                            up2(add2(pk2(in.utP[t - 1][0], in.utP[t - 1][1]), s01), oU[0], oU[1]);
-                            up2(add2(pk2(in.utP[t - 1][2], in.utP[t - 1][3]), s23), oU[2], oU[3]);
+                            const f2 s02 = fma2(al2, pk2(x0[0], x0[2]), mul2(be2, pk2(z[0], z[2])));
+                            const f2 s13 = fma2(al2, pk2(x0[1], x0[3]), mul2(be2, pk2(z[1], z[3])));
+                            up2(s02, oS[0], oS[2]);
+                            up2(s13, oS[1], oS[3]);
+                            up2(add2(pk2(in.utP[t - 1][0], in.utP[t - 1][2]), s02), oU[0], oU[2]);
+                            up2(add2(pk2(in.utP[t - 1][1], in.utP[t - 1][3]), s13), oU[1], oU[3]);
                         } else {
 #pragma unroll
                             for (int k = 0; k < 4; ++k) {
@@ -1063,6 +1069,7 @@ __global__ void __launch_bounds__(fused_threads<T>(), 2) k_pp_fused(PpFusedArgs 
                     };
                     if (FULL || m == 4) step(4);
                     else step(m);
+                    ky_top = ky4.x;
                     // level t-1's output of this iteration is what level t reads next time
                     out.sdL[t - 1] = x0[3];
 #pragma unroll
@@ -1075,7 +1082,7 @@ __global__ void __launch_bounds__(fused_threads<T>(), 2) k_pp_fused(PpFusedArgs 
                         cU[k] = oU[k];
                     }
                     if (t < T) {
-                        xsb[(t * 2 + (s & 1)) * SR + tid] = make_float4(oS[0], oS[1], oS[2], oS[3]);
+                        xsb[(t * 2 + (s & 1)) * SR + tid] = rows4(oS);
                     } else if (own && q >= sb && q < se) {
 #pragma unroll
                         for (int k = 0; k < 4; ++k) {
