@@ -270,9 +270,9 @@ int solve_timestep(Chunk *c, tl_solve_info_t *info);       // tl_solve.cu
 // run `iters`-iteration graphs of `body` (graph slot `phase`) until the
 // device sets DevScalars::done; *done_out receives it (tl_solve.cu)
 int run_phase(Chunk *c, int (*body)(Chunk *), int iters, int phase, int *done_out);
-// the same with a loop kernel a launch (`loop`), where the device and the
-// chunk's switches allow one; else run_phase
-int run_loop(Chunk *c, int (*loop)(Chunk *), int (*body)(Chunk *), int iters, int phase, int *done_out);
+// the same with a loop kernel a launch (`loop`) if it pays and the device can
+// hold its CTAs at once; else run_phase
+int run_loop(Chunk *c, int (*loop)(Chunk *), int (*body)(Chunk *), int iters, int phase, bool pays, int *done_out);
 constexpr int kPhaseMixedInner = 4;
 constexpr int kPhaseMixedPre = 5;
 int solve_timestep_mixed(Chunk *c, tl_solve_info_t *info); // tl_mixed.cu

@@ -1,5 +1,5 @@
 // tl_loop.cuh -- what the kernels that run many iterations in one launch share
-// (tl_loop.cu: FP64; tl_mixed_loop.cu: mixed-precision PPCG): the meetings of
+// (tl_loop.cu: FP64; tl_mixed_loop.cu: mixed-precision PPCG; tl_mixed.cu: FP32 CG): the meetings of
 // their thread blocks, the walk over the runs, pass 1 of a CG iteration, the
 // launch.
 //
@@ -355,7 +355,7 @@ __device__ __forceinline__ void cg_pass1(const Geo &g, const CgArgs &a, const do
 }
 
 // ppcg: the outer iteration of PPCG, whose z is never r itself
-CgArgs cg_args(Chunk *c, bool ppcg = false) {
+[[maybe_unused]] CgArgs cg_args(Chunk *c, bool ppcg = false) {
     CgArgs a;
     a.u = c->u;
     a.r = c->r;
@@ -402,27 +402,23 @@ using ShapeSmall = LoopShape<2, 4>;
 using ShapeLarge = LoopShape<4, 2>;
 
 // groups of the busiest CTA of a loop kernel
-int loop_depth(const Chunk *c) {
+[[maybe_unused]] int loop_depth(const Chunk *c) {
     const int slots = c->g.groups < c->g.sms ? c->g.groups : c->g.sms;
     return (c->g.groups + slots - 1) / slots;
 }
 
-// one cooperative launch of a loop kernel; TL_ERR_STATE if the device cannot
-// hold its CTAs at once (the caller then runs the passes one by one)
+// one cooperative launch of a loop kernel of `slots` CTAs; TL_ERR_STATE if the
+// device cannot hold them at once (the caller then runs the passes one by one).
+// L has the groups and their depth; the rest is filled in.
 template <class K, class... A>
-int launch_shape(Chunk *c, K kernel, int groups, size_t smem, A... a) {
+int launch_coop(Chunk *c, K kernel, LoopArgs &L, int slots, int threads, size_t smem, A... a) {
     const long long cells = (long long)c->nx * c->ny;
-    const int slots = c->g.groups < c->g.sms ? c->g.groups : c->g.sms;
-    LoopArgs L;
-    L.g = c->g;
     L.sc = c->sc;
     L.partials = c->loop_partials;
     L.arrived = c->loop_arrived;
     L.base = c->loop_arrived + 1;
     L.cg_alphas = c->cg_alphas;
     L.cg_betas = c->cg_betas;
-    L.depth = loop_depth(c);
-    L.per_round = L.depth < groups ? L.depth : groups;
     // a launch of some tens of milliseconds at most
     const long long it = (1LL << 30) / cells;
     L.iters = it < 16 ? 16 : it > 1024 ? 1024 : (int)it;
@@ -430,8 +426,7 @@ int launch_shape(Chunk *c, K kernel, int groups, size_t smem, A... a) {
     cudaError_t e = cudaSuccess;
     if (smem) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess)
-        e = cudaLaunchCooperativeKernel((const void *)kernel, dim3(slots), dim3(L.per_round * kGroupThreads + 32),
-                                        args, smem, c->stream);
+        e = cudaLaunchCooperativeKernel((const void *)kernel, dim3(slots), dim3(threads), args, smem, c->stream);
     if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
         cudaGetLastError();
         c->loop_ok = false;
@@ -441,8 +436,17 @@ int launch_shape(Chunk *c, K kernel, int groups, size_t smem, A... a) {
     c->launches++;
     return TL_OK;
 }
+template <class K, class... A>
+int launch_shape(Chunk *c, K kernel, int groups, size_t smem, A... a) {
+    LoopArgs L;
+    L.g = c->g;
+    L.depth = loop_depth(c);
+    L.per_round = L.depth < groups ? L.depth : groups;
+    return launch_coop(c, kernel, L, c->g.groups < c->g.sms ? c->g.groups : c->g.sms,
+                       L.per_round * kGroupThreads + 32, smem, a...);
+}
 
-int loop_groups(const Chunk *c) {
+[[maybe_unused]] int loop_groups(const Chunk *c) {
     return c->g.groups <= ShapeSmall::kGroups * c->g.sms ? ShapeSmall::kGroups : ShapeLarge::kGroups;
 }
 // (smem: dynamic shared memory beside the kernel's own)

@@ -27,6 +27,7 @@
 
 #include "tl_mixed.cuh"
 #include "tl_device.cuh"
+#include "tl_loop.cuh"
 
 namespace tl {
 
@@ -200,6 +201,11 @@ __device__ __forceinline__ float4 ld4(const float *__restrict__ f, int64_t i) {
     return *reinterpret_cast<const float4 *>(f + i);
 }
 
+// past L1: arrays that a loop kernel's other CTAs write
+__device__ __forceinline__ float4 ld4cg(const float *f, int64_t i) {
+    return __ldcg(reinterpret_cast<const float4 *>(f + i));
+}
+
 // store the first `nv` of four values (all four when nv == 4)
 __device__ __forceinline__ void st4(float *__restrict__ f, int64_t i, float4 v, int nv) {
     if (nv >= 4) {
@@ -263,19 +269,11 @@ __device__ __forceinline__ void reduce_v(CSum acc, double *partials, unsigned in
 // once, so no wave of blocks is left half empty and little is read twice.
 // p' goes to the other of two buffers (DevScalars::p_sel): the
 // neighbours' p' are computed again from z and p.
-__global__ void __launch_bounds__(kBlockThreads) k_v_pw(GeoV g, float *__restrict__ d, float *__restrict__ p0,
-                                                        float *__restrict__ p1, const float *__restrict__ z,
-                                                        const float *__restrict__ kx, const float *__restrict__ ky,
-                                                        float *__restrict__ w, double *partials, unsigned int *counter,
-                                                        DevScalars *sc) {
-    if (*(volatile const int *)&sc->done) return;
-    const bool sel = sc->p_sel != 0;
-    const float *__restrict__ p = sel ? p1 : p0;
-    float *__restrict__ po = sel ? p0 : p1;
-    const float alpha = (float)sc->in_alpha, beta = (float)sc->in_beta;
-    const int lane = threadIdx.x & 31, run = blockIdx.x * kBlockWarps + (threadIdx.x >> 5);
-    const int band = run / g.tiles_x, c = (run - band * g.tiles_x) * kVCols + lane * 4;
-    const int jb = band * g.rows, je = min(jb + g.rows, g.ny);
+__device__ __forceinline__ CSum v_pw(const GeoV &g, int c, int jb, int je, float *__restrict__ d,
+                                     const float *__restrict__ p, float *__restrict__ po, const float *__restrict__ z,
+                                     const float *__restrict__ kx, const float *__restrict__ ky,
+                                     float *__restrict__ w, float alpha, float beta) {
+    const int lane = threadIdx.x & 31;
     const int nv = min(4, g.nx - c);           // valid columns of this lane
     const bool live = c < g.nx + 4;            // lanes that load (the first one past nx reads the halo)
     CSum acc = {0.f, 0.f};
@@ -293,28 +291,29 @@ __global__ void __launch_bounds__(kBlockThreads) k_v_pw(GeoV g, float *__restric
         // flight.  A row is loaded only when it exists: padded rows run to ny + h,
         // so row ny (the halo) is the last one read; nothing past the run's next row.
         auto ldrow = [&](const float *f, int64_t at, int row) { return (live && row <= je) ? ld4(f, at) : z4; };
-        float4 xm = next_p(ldrow(z, i - P, j0 - 1), ldrow(p, i - P, j0 - 1));
-        float4 pc = ldrow(p, i, j0), pn = ldrow(p, i + P, j0 + 1);  // old p of rows rr, rr + 1
-        float4 x0 = next_p(ldrow(z, i, j0), pc), xp = next_p(ldrow(z, i + P, j0 + 1), pn);
+        auto ldnew = [&](const float *f, int64_t at, int row) { return (live && row <= je) ? ld4cg(f, at) : z4; };
+        float4 xm = next_p(ldnew(z, i - P, j0 - 1), ldnew(p, i - P, j0 - 1));
+        float4 pc = ldnew(p, i, j0), pn = ldnew(p, i + P, j0 + 1);  // old p of rows rr, rr + 1
+        float4 x0 = next_p(ldnew(z, i, j0), pc), xp = next_p(ldnew(z, i + P, j0 + 1), pn);
         float4 ky0 = ldrow(ky, i, j0), ky1 = ldrow(ky, i + P, j0 + 1);
-        float4 kxv = ldrow(kx, i, j0), dv = ldrow(d, i, j0);
+        float4 kxv = ldrow(kx, i, j0), dv = ldnew(d, i, j0);
         // the last lane's east face; the first and last lane's neighbours
         const bool edge = live && (lane == 0 || lane == 31);
         const int eo = lane == 0 ? -1 : 4;
         float kxe_edge = lane == 31 && live ? kx[i + 4] : 0.f;
-        float ze = edge ? z[i + eo] : 0.f, pe = edge ? p[i + eo] : 0.f;
+        float ze = edge ? __ldcg(z + i + eo) : 0.f, pe = edge ? __ldcg(p + i + eo) : 0.f;
         for (; j0 < je; j0 += kVUnroll)
 #pragma unroll
         for (int rr = 0; rr < kVUnroll; ++rr) {
             if (j0 + rr >= je) break;
             const int64_t in = i + P, inn = i + 2 * P;
             const int rn = j0 + rr + 1, rnn = j0 + rr + 2;
-            const float4 zpp = ldrow(z, inn, rnn), ppp = ldrow(p, inn, rnn);
+            const float4 zpp = ldnew(z, inn, rnn), ppp = ldnew(p, inn, rnn);
             const float4 ky2 = ldrow(ky, inn, rnn);
-            const float4 kxn = ldrow(kx, in, rn), dn = ldrow(d, in, rn);
+            const float4 kxn = ldrow(kx, in, rn), dn = ldnew(d, in, rn);
             const bool more = rn < je;
             const float kxe_n = lane == 31 && live && more ? kx[in + 4] : 0.f;
-            const float ze_n = edge && more ? z[in + eo] : 0.f, pe_n = edge && more ? p[in + eo] : 0.f;
+            const float ze_n = edge && more ? __ldcg(z + in + eo) : 0.f, pe_n = edge && more ? __ldcg(p + in + eo) : 0.f;
             float kxe = __shfl_down_sync(0xffffffffu, kxv.x, 1);
             float xe = __shfl_down_sync(0xffffffffu, x0.x, 1);
             float xw = __shfl_up_sync(0xffffffffu, x0.w, 1);
@@ -354,6 +353,19 @@ __global__ void __launch_bounds__(kBlockThreads) k_v_pw(GeoV g, float *__restric
             i += P;
         }
     }
+    return acc;
+}
+__global__ void __launch_bounds__(kBlockThreads) k_v_pw(GeoV g, float *__restrict__ d, float *__restrict__ p0,
+                                                        float *__restrict__ p1, const float *__restrict__ z,
+                                                        const float *__restrict__ kx, const float *__restrict__ ky,
+                                                        float *__restrict__ w, double *partials, unsigned int *counter,
+                                                        DevScalars *sc) {
+    if (*(volatile const int *)&sc->done) return;
+    const bool sel = sc->p_sel != 0;
+    const int run = blockIdx.x * kBlockWarps + (threadIdx.x >> 5), band = run / g.tiles_x;
+    const CSum acc = v_pw(g, (run - band * g.tiles_x) * kVCols + (threadIdx.x & 31) * 4, band * g.rows,
+                          min(band * g.rows + g.rows, g.ny), d, sel ? p1 : p0, sel ? p0 : p1, z, kx, ky, w,
+                          (float)sc->in_alpha, (float)sc->in_beta);
     reduce_v(acc, partials, counter, sc, kInW);
 }
 
@@ -362,16 +374,10 @@ __global__ void __launch_bounds__(kBlockThreads) k_v_pw(GeoV g, float *__restric
 // k_pp_step on the warp's two strips; ky, cp and bfp with 1/diag in each
 // strip's first row)
 template <int PC>
-__global__ void __launch_bounds__(kBlockThreads, 3) k_v_rz(GeoV g, float *__restrict__ r, float *__restrict__ z,
-                                                        const float *__restrict__ w, const float *__restrict__ mi,
-                                                        const float *__restrict__ ky, const float *__restrict__ cp,
-                                                        const float *__restrict__ bfp, double *partials,
-                                                        unsigned int *counter, DevScalars *sc) {
-    if (*(volatile const int *)&sc->done) return;
-    const float alpha = (float)sc->in_alpha;
-    const int lane = threadIdx.x & 31, run = blockIdx.x * kBlockWarps + (threadIdx.x >> 5);
-    const int band = run / g.tiles_x, c = (run - band * g.tiles_x) * kVCols + lane * 4;
-    const int jb = band * g.rows, je = min(jb + g.rows, g.ny);
+__device__ __forceinline__ CSum v_rz(const GeoV &g, int c, int jb, int je, float *__restrict__ r,
+                                     float *__restrict__ z, const float *__restrict__ w, const float *__restrict__ mi,
+                                     const float *__restrict__ ky, const float *__restrict__ cp,
+                                     const float *__restrict__ bfp, float alpha) {
     const int nv = min(4, g.nx - c);
     CSum acc = {0.f, 0.f};
     if (nv > 0) {
@@ -386,8 +392,8 @@ __global__ void __launch_bounds__(kBlockThreads, 3) k_v_rz(GeoV g, float *__rest
             for (int k = 0; k < 4; ++k) {
                 if (k >= m) break;
                 const int64_t i = i0 + (int64_t)k * P;
-                wv[k] = ld4(w, i);
-                rv[k] = ld4(r, i);
+                wv[k] = ld4cg(w, i);
+                rv[k] = ld4cg(r, i);
                 if (PC == TL_PREC_JAC_DIAG) f[k] = ld4(mi, i);
                 if (PC == TL_PREC_JAC_BLOCK) f[k] = ld4(bfp, i);
             }
@@ -435,7 +441,69 @@ __global__ void __launch_bounds__(kBlockThreads, 3) k_v_rz(GeoV g, float *__rest
             }
         }
     }
+    return acc;
+}
+template <int PC>
+__global__ void __launch_bounds__(kBlockThreads, 3) k_v_rz(GeoV g, float *__restrict__ r, float *__restrict__ z,
+                                                        const float *__restrict__ w, const float *__restrict__ mi,
+                                                        const float *__restrict__ ky, const float *__restrict__ cp,
+                                                        const float *__restrict__ bfp, double *partials,
+                                                        unsigned int *counter, DevScalars *sc) {
+    if (*(volatile const int *)&sc->done) return;
+    const int run = blockIdx.x * kBlockWarps + (threadIdx.x >> 5), band = run / g.tiles_x;
+    const CSum acc = v_rz<PC>(g, (run - band * g.tiles_x) * kVCols + (threadIdx.x & 31) * 4, band * g.rows,
+                              min(band * g.rows + g.rows, g.ny), r, z, w, mi, ky, cp, bfp, (float)sc->in_alpha);
     reduce_v(acc, partials, counter, sc, kInUr);
+}
+
+// Both passes of many iterations in one launch (tl_loop.cuh): 15 passing warps
+// a multiprocessor (128 registers each, as four warps share a quarter of them), each with the same run in both passes.
+// What bounds it: the two meetings and the latency of one row after another
+// (1024^2 cells, jac_diag: 16.6 us an iteration, 20.2 as two launches of passes).
+constexpr int kVLoopRows = 7;  // rows of the longest runs (inner_loop_pays)
+constexpr int kVLoopWarps = 15, kVLoopThreads = kVLoopWarps * 32 + 32;
+struct VLoopArgs {
+    float *d, *p0, *p1, *r, *z, *w;
+    const float *src;  // z, or r without a preconditioner
+    const float *kx, *ky, *mi, *cp, *bfp;
+};
+template <int PC>
+__global__ void __launch_bounds__(kVLoopThreads, 1) k_v_loop(LoopArgs L, GeoV g, VLoopArgs a) {
+    if (*(volatile const int *)&L.sc->done) return;
+    __shared__ LoopShared S;
+    loop_begin(L, S);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp == kVLoopWarps) {
+        S.sh[0][warp][lane] = 0.0;  // (completes a group of sums)
+        for (int it = 0; it < L.iters; ++it) {
+            loop_meet<1>(L, S, kEpiStore, [&] { inner_epilogue(&S.sc, kInW, S.sc.sum[0]); });
+            if (S.stalled) break;
+            loop_meet<1>(L, S, kEpiStore, [&] { inner_epilogue(&S.sc, kInUr, S.sc.sum[0]); });
+            if (S.stalled || S.sc.done) break;
+        }
+    } else {
+        // runs one after the other on all CTAs, so that few are spread widely
+        const int run = warp * (int)gridDim.x + (int)blockIdx.x, band = run / g.tiles_x;
+        const int c = (run - band * g.tiles_x) * kVCols + lane * 4;
+        const int jb = min(band * g.rows, g.ny), je = min(jb + g.rows, g.ny);
+        for (int it = 0; it < L.iters; ++it) {
+            const bool sel = S.sc.p_sel != 0;
+            CSum acc = v_pw(g, c, jb, je, a.d, sel ? a.p1 : a.p0, sel ? a.p0 : a.p1, a.src, a.kx, a.ky, a.w,
+                            (float)S.sc.in_alpha, (float)S.sc.in_beta);
+            S.sh[0][warp][lane] = (double)acc.s + (double)acc.e;
+            loop_arrive<1>(L, S);
+            loop_met();
+            loop_scalars();
+            if (S.stalled) break;
+            acc = v_rz<PC>(g, c, jb, je, a.r, a.z, a.w, a.mi, a.ky, a.cp, a.bfp, (float)S.sc.in_alpha);
+            S.sh[0][warp][lane] = (double)acc.s + (double)acc.e;
+            loop_arrive<1>(L, S);
+            loop_met();
+            loop_scalars();
+            if (S.stalled || S.sc.done) break;
+        }
+    }
+    loop_end(L, S);
 }
 
 // ------------------------------------ PPCG inner steps in FP32 (mixed form)
@@ -1373,18 +1441,18 @@ int launch_v(Chunk *c, const char *name, F &&launch) {
     return TL_OK;
 }
 
-// runs for `ctas` blocks a multiprocessor: at least 8 rows, a multiple of `unit`.
+// runs for `warps` a multiprocessor: at least `least` rows, a multiple of `unit`.
 // (Never more blocks than the tiles that the partial sums have room for.  Whole
 // strips in both passes left an eighth of the device idle at 3000 x 2100, 24
 // rows where 21 do: 43.7 and 28.7 us, now 41.9 and 28.1.)
-GeoV run_geo(const Chunk *c, int ctas, int unit, unsigned *grid) {
+GeoV run_geo(const Chunk *c, int warps, int unit, unsigned *grid, int least = 8) {
     const Mixed *mx = (const Mixed *)c->mixed;
     GeoV g{c->nx, c->ny, c->h, c->pitch, mx->vtiles_x, mx->vtiles, 0};
-    const int warps = c->sms * ctas * kBlockWarps, bands = warps / g.tiles_x > 1 ? warps / g.tiles_x : 1;
+    const int bands = c->sms * warps / g.tiles_x > 1 ? c->sms * warps / g.tiles_x : 1;
     const int per = (c->ny + bands - 1) / bands;
-    g.rows = ((per > 8 ? per : 8) + unit - 1) / unit * unit;
+    g.rows = ((per > least ? per : least) + unit - 1) / unit * unit;
     const long long runs = (long long)g.tiles_x * ((c->ny + g.rows - 1) / g.rows);
-    *grid = (unsigned)((runs + kBlockWarps - 1) / kBlockWarps);
+    if (grid) *grid = (unsigned)((runs + kBlockWarps - 1) / kBlockWarps);
     return g;
 }
 
@@ -1394,7 +1462,8 @@ int inner_body_pc(Chunk *c) {
     const bool diag = PC != TL_PREC_NONE;
     unsigned grid, grid_rz;
     // (the block solve takes whole strips)
-    const GeoV g = run_geo(c, 2, 1, &grid), g_rz = run_geo(c, 3, PC == TL_PREC_JAC_BLOCK ? 4 : 1, &grid_rz);
+    const GeoV g = run_geo(c, 2 * kBlockWarps, 1, &grid);
+    const GeoV g_rz = run_geo(c, 3 * kBlockWarps, PC == TL_PREC_JAC_BLOCK ? 4 : 1, &grid_rz);
     cudaStream_t s = c->stream;
     int rc;
     if ((rc = launch_v(c, "mixed_pw", [&] {
@@ -1406,6 +1475,35 @@ int inner_body_pc(Chunk *c) {
         k_v_rz<PC><<<grid_rz, kBlockThreads, 0, s>>>(g_rz, mx->r, mx->z, mx->w, mx->mi, mx->ky, mx->cp, mx->bfp,
                                                   mx->partials, mx->counter, c->sc);
     });
+}
+
+template <int PC>
+int inner_loop_pc(Chunk *c) {
+    Mixed *mx = mixed_of(c);
+    const GeoV g = run_geo(c, kVLoopWarps, PC == TL_PREC_JAC_BLOCK ? 4 : 1, nullptr, 4);
+    const int runs = g.tiles_x * ((c->ny + g.rows - 1) / g.rows), slots = runs < c->sms ? runs : c->sms;
+    LoopArgs L{};
+    L.depth = (kVLoopWarps + kGroupWarps - 1) / kGroupWarps;
+    L.g.groups = slots * L.depth;
+    const VLoopArgs a{mx->d, mx->p, mx->sd[0], mx->r, mx->z, mx->w, PC != TL_PREC_NONE ? mx->z : mx->r,
+                      mx->kx, mx->ky, mx->mi, mx->cp, mx->bfp};
+    return launch_coop(c, k_v_loop<PC>, L, slots, kVLoopThreads, 0, g, a);
+}
+
+// The FP32 CG iterations in loops: while the runs are short.  Microseconds an
+// iteration with and without jac_diag, loop and two launches of passes: 13 / 12
+// and 22 / 21 at 96 x 80 (runs of 4 rows), 17 / 15 and 20 / 19 at 1024^2 (4), 20 /
+// 17 and 23 / 22 at 1200^2 (6), 25 / 19 and 26 / 24 at 1400^2 (7), 30 / 21 and 27 /
+// 24 at 520 x 4000 (9), 42 / 27 and 37 / 27 at 1700^2 (10), 83 / 63 and 71 / 60 at
+// 3000 x 2100 (22): 15 warps a multiprocessor are too few for the passes' loads.
+bool inner_loop_pays(const Chunk *c) {
+    const GeoV g = run_geo(c, kVLoopWarps, 1, nullptr, 4);
+    // (a field with more tiles side by side than there are warps has runs left over)
+    return c->loop_ok && !c->profiling && !c->cfg.reflective_boundary && g.tiles_x <= c->sms * kVLoopWarps &&
+           g.rows <= kVLoopRows;
+}
+int inner_loop(Chunk *c) {
+    return by_precond(c, [&](auto pc) { return inner_loop_pc<decltype(pc)::value>(c); });
 }
 
 // the inner CG iteration of the mixed CG solve (none or jac_diag)
@@ -1671,7 +1769,7 @@ int mixed_ppcg_presteps(Chunk *c, int *done_out) {
 #undef TL_PRE_INIT
     if (rc) return rc;
     int done = kRunning;
-    if ((rc = run_phase(c, prestep_body, kItersInner, kPhaseMixedPre, &done))) return rc;
+    if ((rc = run_loop(c, inner_loop, prestep_body, kItersInner, kPhaseMixedPre, inner_loop_pays(c), &done))) return rc;
     // u += d, r = u0 - A u (FP64): the phase after the switch starts from the
     // true residual
     BodyUpdateU bu{c->u, mx->d, mx->p, mx->sd[0], c->pitch, c->pitch, nullptr, 0.f};
@@ -1767,7 +1865,7 @@ int solve_timestep_mixed(Chunk *c, tl_solve_info_t *info) {
             if ((rc = run32(c, "mixed_init", bi, kInInit, false))) return rc;
         }
         int done = kRunning;
-        if ((rc = run_phase(c, inner_body, kItersInner, kPhaseMixedInner, &done))) return rc;
+        if ((rc = run_loop(c, inner_loop, inner_body, kItersInner, kPhaseMixedInner, inner_loop_pays(c), &done))) return rc;
         if (done == kBreakdown) {
             set_error("mixed solve: breakdown in the FP32 inner iteration");
             status = TL_ERR_BREAKDOWN;

@@ -202,8 +202,8 @@ int run_phase(Chunk *c, int (*body)(Chunk *), int iters, int phase, int *done_ou
     return TL_OK;
 }
 
-int run_loop(Chunk *c, int (*loop)(Chunk *), int (*body)(Chunk *), int iters, int phase, int *done_out) {
-    if (!loop_pays(c)) return run_phase(c, body, iters, phase, done_out);
+int run_loop(Chunk *c, int (*loop)(Chunk *), int (*body)(Chunk *), int iters, int phase, bool pays, int *done_out) {
+    if (!pays) return run_phase(c, body, iters, phase, done_out);
     for (;;) {
         int rc = loop(c);
         if (rc == TL_ERR_STATE && !c->loop_ok) return run_phase(c, body, iters, phase, done_out);
@@ -398,29 +398,29 @@ int solve_timestep(Chunk *c, tl_solve_info_t *info) {
                     done = kSwitch;
                 }
             } else {
-                rc = run_loop(c, launch_cg_loop, body_cg, kItersCg, kPhaseCg, &done);
+                rc = run_loop(c, launch_cg_loop, body_cg, kItersCg, kPhaseCg, loop_pays(c), &done);
                 if (!rc && !cf.reflective_boundary) rc = launch_cg_finish(c, false);
             }
             break;
         case kPhasePpcg:
             if (ppcg_fused(c)) {
                 if ((rc = ppcg_alloc(c))) return rc;
-                rc = run_loop(c, launch_ppcg_loop, body_ppcg, kItersPpcg, kPhasePpcg, &done);
+                rc = run_loop(c, launch_ppcg_loop, body_ppcg, kItersPpcg, kPhasePpcg, loop_pays(c), &done);
                 if (!rc) rc = launch_ppcg_finish(c);
             } else {
                 if (cf.precision == TL_PRECISION_MIXED && mixed_loop_pays(c))
-                    rc = run_loop(c, launch_mixed_ppcg_loop, body_ppcg, kItersPpcg, kPhasePpcg, &done);
+                    rc = run_loop(c, launch_mixed_ppcg_loop, body_ppcg, kItersPpcg, kPhasePpcg, loop_pays(c), &done);
                 else
                     rc = run_phase(c, body_ppcg, kItersPpcg, kPhasePpcg, &done);
                 if (!rc && cf.precision == TL_PRECISION_MIXED) rc = launch_ppcg_finish(c);
             }
             break;
         case kPhaseCheby:
-            rc = run_loop(c, launch_cheby_loop, body_cheby, kItersCheby, kPhaseCheby, &done);
+            rc = run_loop(c, launch_cheby_loop, body_cheby, kItersCheby, kPhaseCheby, loop_pays(c), &done);
             if (!rc && !cf.reflective_boundary) rc = launch_cheby_finish(c);
             break;
         case kPhaseJacobi:
-            rc = run_loop(c, launch_jacobi_loop, body_jacobi, kItersJacobi, kPhaseJacobi, &done);
+            rc = run_loop(c, launch_jacobi_loop, body_jacobi, kItersJacobi, kPhaseJacobi, loop_pays(c), &done);
             if (!rc && !cf.reflective_boundary) rc = launch_jacobi_finish(c);
             break;
         }
