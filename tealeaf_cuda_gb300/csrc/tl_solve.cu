@@ -4,11 +4,13 @@
 // The reference returns every dot product to the host (a blocking cudaMemcpy
 // after each reduction, host_reductions_kernel_cuda.hpp:32) and computes
 // alpha, beta and the exit test in Fortran.  Here those scalars live in
-// DevScalars: the last CTA of each reducing kernel applies the same formulas,
-// so the iteration runs without the host.  Iterations are captured into a CUDA
-// graph (kIters iterations per graph); every kernel of an iteration returns at
-// once when `done` is set, so a graph launched past convergence is a chain of
-// empty kernels.  The host polls the scalars of graph k while graph k+1 runs.
+// DevScalars and the kernels apply the same formulas, so the iteration runs
+// without the host: either one cooperative launch runs many iterations
+// (run_loop; tl_loop.cuh), or iterations are captured into a CUDA graph (kIters
+// iterations per graph; run_phase), where the last CTA of each reducing kernel
+// applies the formulas, every kernel returns at once when `done` is set, so a
+// graph launched past convergence is a chain of empty kernels, and the host polls
+// the scalars of graph k while graph k+1 runs.
 //
 // The host still owns what the reference computes on the host once per solve:
 // the Lanczos eigenvalue estimate (tqli), the Chebyshev coefficients and the
