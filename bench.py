@@ -101,7 +101,6 @@ BYTES_PER_CELL = {
     "mixed_pw": 32,      # read z, p, d, Kx, Ky; write p, d, w
     "mixed_init": 28,    # read r (FP64), Mi; write r, z, p, d
     "mixed_update_u": 24,  # read u (FP64), d, p; write u (FP64)
-    "mixed_convert": 40,   # read Kx, Ky (FP64); write Kx, Ky, Mi (FP32)
     "mixed_pp_init": 28,   # read r, z (FP64); write sd, rtemp, utemp
 }
 
@@ -163,6 +162,9 @@ def bytes_per_cell(kernel, precond):
     if kernel == "mixed_rz":
         # read r, w + the preconditioner (Mi; or Ky, cp, bfp); write r, z
         return {"none": 12, "jac_diag": 20, "jac_block": 28}[precond]
+    if kernel == "mixed_convert":
+        # read Kx, Ky and the preconditioner (FP64; Mi or cp, bfp); write them in FP32
+        return {"none": 24, "jac_diag": 36, "jac_block": 48}[precond]
     if kernel == "mixed_init":
         # read r (FP64) + the preconditioner; write r, z, p, d
         return {"none": 24, "jac_diag": 28, "jac_block": 36}[precond]

@@ -1195,44 +1195,38 @@ __global__ void __launch_bounds__(fused_threads<T>(), 2) k_pp_fused(PpFusedArgs 
     if (RRN) fused_rrn_reduce(racc, a.partials, a.counter, sc);
 }
 
-// FP32 copies of the preconditioner: Mi = 1/diag, block cp, and bfp with
-// 1/diag at each strip's first row
-__global__ void k_pp_convert(GeoV g, int pitch64, const double *__restrict__ dg, const double *__restrict__ cp64,
-                             const double *__restrict__ bfp64, float *__restrict__ mi, float *__restrict__ cp,
-                             float *__restrict__ bfp) {
-    const long long n = (long long)g.nx * g.ny;
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n;
-         k += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(k % g.nx), j = (int)(k / g.nx);
-        const int64_t a = (int64_t)(i + g.h) + (int64_t)(j + g.h) * g.pitch;
-        const int64_t b = (int64_t)(i + g.h) + (int64_t)(j + g.h) * pitch64;
-        mi[a] = (float)(1.0 / dg[b]);
-        cp[a] = (float)cp64[b];
-        bfp[a] = (j % 4 == 0) ? (float)(1.0 / dg[b]) : (float)bfp64[b];
+// FP32 copies of the operator (with the faces east of the last column and above
+// the last row) and, of the preconditioner, what PC takes: Mi, or the strips' cp
+// and bfp with 1/diag in each strip's first row.  mi64: 1/diag, or null to divide
+// here; rd64: 1/diag of the strips' first rows, a row a strip.  A thread keeps its
+// column.  HBM-bound (48 bytes a cell with block-Jacobi).  8192^2 cells, block:
+// 0.56 ms; as two kernels that converted each face twice and divided what cg_init
+// had divided, 1.76 and 1.00.
+template <int PC>
+__global__ void __launch_bounds__(128) k_convert(int nx, int ny, int h, int pitch, const double *__restrict__ kx64,
+                                                 const double *__restrict__ ky64, const double *__restrict__ dg64,
+                                                 const double *__restrict__ mi64, const double *__restrict__ cp64,
+                                                 const double *__restrict__ bfp64, const double *__restrict__ rd64,
+                                                 float *__restrict__ kx, float *__restrict__ ky,
+                                                 float *__restrict__ mi, float *__restrict__ cp,
+                                                 float *__restrict__ bfp) {
+    const int i = blockIdx.x * 128 + threadIdx.x;
+    if (i > nx) return;
+#pragma unroll 2
+    for (int j = blockIdx.y; j <= ny; j += gridDim.y) {
+        const int64_t a = (int64_t)(i + h) + (int64_t)(j + h) * pitch;
+        if (j < ny) kx[a] = (float)kx64[a];
+        if (i == nx) continue;
+        ky[a] = (float)ky64[a];
+        if (j == ny) continue;
+        if (PC == TL_PREC_JAC_DIAG) mi[a] = (float)(mi64 ? mi64[a] : 1.0 / dg64[a]);
+        if (PC == TL_PREC_JAC_BLOCK) {
+            cp[a] = (float)cp64[a];
+            bfp[a] = (float)(j % kStrip == 0 ? rd64[(i + h) + (int64_t)(j / kStrip) * pitch] : bfp64[a]);
+        }
     }
 }
 
-// Kx, Ky -> FP32; Mi = 1/diag(A) computed in FP64, stored in FP32
-struct BodyConvert {
-    const double *kx64, *ky64;
-    float *kx, *ky, *mi;
-    int pitch32, pitch64, nx, ny, h;
-    __device__ void setup(DevScalars *) {}
-    __device__ void operator()(int64_t b32, int64_t b64, int m, CSum &) const {
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-            if (k < m) {
-                const int64_t i = b64 + (int64_t)k * pitch64, j = b32 + (int64_t)k * pitch32;
-                const double diag = (1.0 + (ky64[i + pitch64] + ky64[i])) + (kx64[i + 1] + kx64[i]);
-                kx[j] = (float)kx64[i];
-                ky[j] = (float)ky64[i];
-                mi[j] = (float)(1.0 / diag);
-                // the east face of the last column and the north face of the top row
-                kx[j + 1] = (float)kx64[i + 1];
-                ky[j + pitch32] = (float)ky64[i + pitch64];
-            }
-    }
-};
 
 template <int PC>
 struct BodyInnerInit {  // r = (float) r64; z = M^-1 r; p = z; d = 0; sum r.z
@@ -1521,6 +1515,19 @@ int prestep_body(Chunk *c) {
     }
 }
 
+int launch_convert(Chunk *c, const double *mi64) {
+    Mixed *mx = mixed_of(c);
+    const int bx = (c->nx + 128) / 128, by = c->sms * 16 / bx;
+    const dim3 grid(bx, by < 1 ? 1 : by > c->ny + 1 ? c->ny + 1 : by);
+    return by_precond(c, [&](auto pc) {
+        return launch_v(c, "mixed_convert", [&] {
+            k_convert<decltype(pc)::value><<<grid, 128, 0, c->stream>>>(c->nx, c->ny, c->h, c->pitch, c->kx, c->ky, c->diag,
+                                                                        mi64, c->cp, c->bfp, c->rdiag, mx->kx, mx->ky,
+                                                                        mx->mi, mx->cp, mx->bfp);
+        });
+    });
+}
+
 }  // namespace
 
 // FP32 copies of the operator and of the PPCG preconditioner, after cg_init
@@ -1528,13 +1535,7 @@ int prestep_body(Chunk *c) {
 int mixed_ppcg_prepare(Chunk *c) {
     int rc;
     if ((rc = mixed_alloc(c))) return rc;
-    Mixed *mx = mixed_of(c);
-    BodyConvert bc{c->kx, c->ky, mx->kx, mx->ky, mx->mi, c->pitch, c->pitch, c->nx, c->ny, c->h};
-    if ((rc = run32(c, "mixed_convert", bc, kInNone, false))) return rc;
-    const GeoV g{c->nx, c->ny, c->h, c->pitch, mx->vtiles_x, mx->vtiles};
-    return launch_v(c, "mixed_pp_convert", [&] {
-        k_pp_convert<<<1216, 256, 0, c->stream>>>(g, c->pitch, c->diag, c->cp, c->bfp, mx->mi, mx->cp, mx->bfp);
-    });
+    return launch_convert(c, c->mi);
 }
 
 template <int T, int PC, bool LAST, bool FIRST, bool RRN>
@@ -1810,8 +1811,7 @@ int solve_timestep_mixed(Chunk *c, tl_solve_info_t *info) {
     c->ry = ry;
     const int zero[4] = {1, 1, 1, 1};
     if ((rc = launch_common_init(c, cf.coefficient, rx, ry, zero, 0))) return rc;
-    BodyConvert bc{c->kx, c->ky, mx->kx, mx->ky, mx->mi, c->pitch, c->pitch, c->nx, c->ny, c->h};
-    if ((rc = run32(c, "mixed_convert", bc, kInNone, false))) return rc;
+    if ((rc = launch_convert(c, nullptr))) return rc;
 
     DevScalars &h = *c->sc_host;
     memset(&h, 0, sizeof h);
