@@ -471,10 +471,12 @@ template <int PC>
 __global__ void __launch_bounds__(kVLoopThreads, 1) k_v_loop(LoopArgs L, GeoV g, VLoopArgs a) {
     if (*(volatile const int *)&L.sc->done) return;
     __shared__ LoopShared S;
-    loop_begin(L, S);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // completes the last group of sums; before loop_begin's barrier, which alone
+    // orders it for the passing warps (kBarSums counts them only)
+    if (warp == kVLoopWarps) S.sh[0][warp][lane] = 0.0;
+    loop_begin(L, S);
     if (warp == kVLoopWarps) {
-        S.sh[0][warp][lane] = 0.0;  // (completes a group of sums)
         for (int it = 0; it < L.iters; ++it) {
             loop_meet<1>(L, S, kEpiStore, [&] { inner_epilogue(&S.sc, kInW, S.sc.sum[0]); });
             if (S.stalled) break;
