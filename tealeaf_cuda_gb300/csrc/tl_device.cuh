@@ -32,20 +32,23 @@ __device__ __forceinline__ void strip_block_solve(const double *__restrict__ dg,
     }
 }
 
-// x / b for b >= 1 whose correctly rounded reciprocal y is known: two residual
+// x / b, bit for bit, from the correctly rounded reciprocal y of b: two residual
 // corrections of x y.  The first leaves an error below an ulp, and from there, y
 // being correctly rounded, the second rounds correctly (Markstein, "Computation
 // of elementary functions on the IBM RISC System/6000 processor", 1990, theorem
-// on division).  5 fused multiply-adds where the division operator takes about
-// twice as many FP64 instructions; the sign of a zero result may differ from it.
-// Values so small that the residuals would underflow are divided.
+// on division; no quotient of 2^-863 or more underflows while |b| < 2^150).  5
+// fused multiply-adds where the division operator takes about twice as many
+// FP64 instructions.  Divided instead: an x so small that the residuals would
+// underflow, and whatever gives no finite q (the corrections turn an infinite
+// quotient, or one by an infinite b, into NaN).  A zero x gives its sign to q.
 static __device__ __noinline__ double div_slow(double x, double b) { return x / b; }
 __device__ __forceinline__ double div_by(double x, double b, double y) {
     double q = x * y;
     q = fma(fma(-b, q, x), y, q);
     q = fma(fma(-b, q, x), y, q);
-    const unsigned int e = ((unsigned int)__double2hiint(x) >> 20) & 0x7FFu;  // biased exponent
-    if (e < 160u && x != 0.0) q = div_slow(x, b);
+    const unsigned int ex = ((unsigned int)__double2hiint(x) >> 20) & 0x7FFu;  // biased exponents
+    const unsigned int eq = ((unsigned int)__double2hiint(q) >> 20) & 0x7FFu;
+    if (ex < 160u || eq == 0x7FFu) q = x == 0.0 ? x * y : div_slow(x, b);
     return q;
 }
 

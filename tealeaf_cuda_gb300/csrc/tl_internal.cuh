@@ -122,7 +122,8 @@ struct Chunk {
     double *density, *energy0, *energy1, *u, *u0, *p, *r, *w, *z, *mi, *kx, *ky, *sd,
         *rtemp, *utemp, *r_store, *cp, *bfp, *volume, *un;
     double *diag;                // diag(A), refreshed with Kx/Ky by common_init
-    double *rdiag;               // block-Jacobi: 1 / diag of each strip's first row (nstrips rows)
+    double *rdiag;               // block-Jacobi: 1 / diag of each strip's first row (nstrips rows); of
+                                 // the present diag only once cg_init has followed common_init
     double *sd_alt;              // FP64 PPCG: second buffer of sd (allocated on first use)
     double *stage;               // (rows x (nx + 2h)) contiguous copy buffer of
                                  // tl_get_field / tl_set_field (allocated on first use)
