@@ -178,10 +178,12 @@ __global__ void k_prev(Geo g, const double *__restrict__ u0, double *__restrict_
 __device__ __forceinline__ float clampf(float v) { return fminf(fmaxf(v, -kClamp), kClamp); }
 
 // (float)(x / b), y the correctly rounded 1 / b: the quotient within 0.5000001
-// ulps of FP64 (x / b below FP64's smallest residuals is zero in FP32)
+// ulps of FP64 (x / b below FP64's smallest residuals is zero in FP32).  An
+// infinite or NaN x y is the quotient itself; corrected, infinity would be NaN.
 __device__ __forceinline__ float quotient(double x, double b, double y) {
     const double q = x * y;
-    return (float)fma(fma(-b, q, x), y, q);
+    const bool finite = (__double2hiint(q) & 0x7FF00000) != 0x7FF00000;
+    return (float)(finite ? fma(fma(-b, q, x), y, q) : q);
 }
 
 // network inputs of cell (i, j), as BF16 into the padded NHWC input
