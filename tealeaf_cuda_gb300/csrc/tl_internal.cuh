@@ -125,6 +125,7 @@ struct Chunk {
     double *rdiag;               // block-Jacobi: 1 / diag of each strip's first row (nstrips rows); of
                                  // the present diag only once cg_init has followed common_init
     double *sd_alt;              // FP64 PPCG: second buffer of sd (allocated on first use)
+    bool no_sd_alt;              // there was no memory for it: FP64 PPCG runs its single pieces
     double *stage;               // (rows x (nx + 2h)) contiguous copy buffer of
                                  // tl_get_field / tl_set_field (allocated on first use)
     std::vector<void *> allocations;
@@ -244,7 +245,7 @@ int launch_cg_loop(Chunk *c);    // many iterations in one launch
 int launch_ppcg_pass2(Chunk *c);             // r_store, r, and the start of the inner steps
 int launch_ppcg_step(Chunk *c, int step);    // one inner step; the last sums (r - r_store).z and r.z
 int launch_ppcg_loop(Chunk *c);
-int ppcg_alloc(Chunk *c);                    // sd_alt
+int ppcg_alloc(Chunk *c);                    // sd_alt, or no_sd_alt
 int launch_ppcg_finish(Chunk *c);            // u, p and sd in their places
 int launch_cheby_step(Chunk *c);
 int launch_cheby_loop(Chunk *c);

@@ -792,6 +792,14 @@ int ppcg_alloc(Chunk *c) {
     if (c->sd_alt) return TL_OK;
     void *p;
     const int rc = dalloc(c, &p, c->alloc_elems * sizeof(double));
+    if (rc == TL_ERR_ALLOC) {
+        // the single pieces need no second buffer; the chunk keeps to them, as
+        // its graph of iterations holds them from now on
+        cudaGetLastError();
+        set_error("%s", "");
+        c->no_sd_alt = true;
+        return TL_OK;
+    }
     if (rc) return rc;
     c->sd_alt = (double *)p + c->lead;
     return TL_OK;

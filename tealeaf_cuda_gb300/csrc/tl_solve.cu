@@ -79,9 +79,11 @@ int body_cg(Chunk *c) {
 }
 
 // FP64 PPCG in fused passes: not with reflective boundaries (sd and p are
-// mirrored between the pieces) nor without an inner step
+// mirrored between the pieces), nor without an inner step or the memory for
+// sd's second buffer
 bool ppcg_fused(const Chunk *c) {
-    return c->cfg.precision != TL_PRECISION_MIXED && !c->cfg.reflective_boundary && c->cfg.ppcg_inner_steps >= 1;
+    return c->cfg.precision != TL_PRECISION_MIXED && !c->cfg.reflective_boundary && c->cfg.ppcg_inner_steps >= 1 &&
+           !c->no_sd_alt;
 }
 
 // Mixed PPCG in loops: while the fused passes cannot fill the device, and only
@@ -405,8 +407,8 @@ int solve_timestep(Chunk *c, tl_solve_info_t *info) {
             }
             break;
         case kPhasePpcg:
+            if (ppcg_fused(c) && (rc = ppcg_alloc(c))) return rc;
             if (ppcg_fused(c)) {
-                if ((rc = ppcg_alloc(c))) return rc;
                 rc = run_loop(c, launch_ppcg_loop, body_ppcg, kItersPpcg, kPhasePpcg, loop_pays(c), &done);
                 if (!rc) rc = launch_ppcg_finish(c);
             } else {
