@@ -217,6 +217,13 @@ int tl_default_chunk_init(const tl_config_t *cfg);
  * 0 disarms it.  Returns TL_ERR_ARG for nth < 0. */
 int tl_test_fail_alloc(int nth);
 
+/* tl_test_loops -- no counterpart in the reference; a test hook for the kernels
+ * that run many iterations a launch.  start_wait, wait: clocks that their thread
+ * blocks wait for one another's start (then the solve goes on in separate
+ * passes) and at a meeting (then it returns TL_ERR_CUDA); below 0: the defaults,
+ * about two seconds.  iters: iterations a launch, 0: by the number of cells. */
+int tl_test_loops(tl_chunk_t *ch, long long start_wait, long long wait, int iters);
+
 /* tl_dot_noalloc -- no counterpart in the reference.  The dot-product
  * reduction of tea_leaf_calc_2norm (sum of a[i]*b[i]) for callers that
  * cannot let the library allocate: hosts that set up their whole

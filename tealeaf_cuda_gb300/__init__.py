@@ -154,6 +154,7 @@ def load():
     lib.tl_set_field.argtypes = [C.c_void_p, C.c_int, C.c_void_p]
     lib.tl_set_dt.argtypes = [C.c_void_p, C.c_double]
     lib.tl_set_inner_fusion.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_int]
+    lib.tl_test_loops.argtypes = [C.c_void_p, C.c_longlong, C.c_longlong, C.c_int]
     lib.tl_kernel_launches.restype = C.c_longlong
     lib.tl_kernel_launches.argtypes = [C.c_void_p]
     lib.tl_default_chunk.restype = C.c_void_p

@@ -204,6 +204,7 @@ static int chunk_alloc(const tl_config_t *cfg, Chunk **out) {
     int coop = 0;
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device);
     c->loop_ok = coop != 0;
+    c->loop_start_wait = c->loop_wait = -1;
     if ((rc = dalloc(c, &p, sizeof(DevScalars)))) { chunk_release(c); return rc; }
     c->sc = (DevScalars *)p;
     size_t nit = (size_t)cfg->max_iters + 4;
@@ -463,6 +464,17 @@ int tl_test_fail_alloc(int nth) {
         return TL_ERR_ARG;
     }
     g_fail_alloc_countdown.store(nth);
+    return TL_OK;
+}
+
+int tl_test_loops(tl_chunk_t *ch, long long start_wait, long long wait, int iters) {
+    if (!ch || !ch->c || iters < 0) {
+        set_error("tl_test_loops: bad argument");
+        return TL_ERR_ARG;
+    }
+    ch->c->loop_start_wait = start_wait;
+    ch->c->loop_wait = wait;
+    ch->c->loop_iters = iters;
     return TL_OK;
 }
 

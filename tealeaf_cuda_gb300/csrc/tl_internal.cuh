@@ -58,7 +58,15 @@ struct DevScalars {
     int p_sel;                     // which of the two buffers holds the iterate (p, u or sd)
 };
 
-enum DoneCode { kRunning = 0, kConverged = 1, kMaxIters = 2, kSwitch = 3, kBreakdown = 4, kStalled = 5 };
+enum DoneCode {
+    kRunning = 0,
+    kConverged = 1,
+    kMaxIters = 2,
+    kSwitch = 3,
+    kBreakdown = 4,
+    kStalled = 5,     // a loop kernel's wait ran out
+    kNotStarted = 6   // not all of its CTAs started in time: it did nothing
+};
 
 // What the last CTA of a kernel does with the grid-wide sums.
 enum Epilogue : int {
@@ -142,7 +150,10 @@ struct Chunk {
     cudaEvent_t poll_ev[2];
     // the meeting points of the loop kernels (tl_loop.cu)
     double *loop_partials;
-    unsigned int *loop_arrived;  // [0] arrivals, [1] arrivals before the next launch
+    unsigned int *loop_arrived;  // [0] arrivals, [1] arrivals before the next launch, [32] the gate
+    unsigned int loop_round;     // launches so far
+    long long loop_start_wait, loop_wait;  // clocks; below 0: the defaults (tl_test_loops)
+    int loop_iters;              // iterations a launch; 0: by the number of cells (tl_test_loops)
     bool loop_ok;                // the device can hold a loop kernel's CTAs at once
     double *cg_alphas, *cg_betas;          // device, max_iters + 2
     double *ch_alphas, *ch_betas;          // device coefficient arrays

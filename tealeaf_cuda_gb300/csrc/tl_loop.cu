@@ -99,7 +99,7 @@ template <int PC, class Shape>
 __global__ void __launch_bounds__(Shape::kThreads, 1) k_cg_loop(LoopArgs L, CgArgs a) {
     if (*(volatile const int *)&L.sc->done) return;
     __shared__ LoopShared S;
-    loop_begin(L, S);
+    if (!loop_begin(L, S)) return;
     if (threadIdx.x >= blockDim.x - 32) {
         for (int it = 0; it < L.iters; ++it) {
             loop_meet<1>(L, S, kEpiCgPw);
@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(Shape::kThreads, 1) k_cheby_loop(LoopArgs L, S
         StepCoef co;
         bool sel, go;
     } T[2];  // what step `it` needs, in T[it & 1]
-    loop_begin(L, S);
+    if (!loop_begin(L, S)) return;
     const bool control = threadIdx.x >= blockDim.x - 32;
     // the next step's coefficients (the control warp's first lane)
     auto next = [&](int it) {
@@ -515,7 +515,7 @@ template <int PC, class Shape>
 __global__ void __launch_bounds__(Shape::kThreads, 1) k_ppcg_loop(LoopArgs L, StepArgs a, CgArgs cg) {
     if (*(volatile const int *)&L.sc->done) return;
     __shared__ LoopShared S;
-    loop_begin(L, S);
+    if (!loop_begin(L, S)) return;
     const double theta_r = 1.0 / S.sc.theta;
     if (threadIdx.x >= blockDim.x - 32) {
         for (int it = 0; it < L.iters; ++it) {
@@ -676,7 +676,7 @@ template <class Shape>
 __global__ void __launch_bounds__(Shape::kThreads, 1) k_jacobi_loop(LoopArgs L, StepArgs a) {
     if (*(volatile const int *)&L.sc->done) return;
     __shared__ LoopShared S;
-    loop_begin(L, S);
+    if (!loop_begin(L, S)) return;
     if (threadIdx.x >= blockDim.x - 32) {
         for (int it = 0; it < L.iters; ++it) {
             loop_meet<1>(L, S, kEpiJacobiStep);

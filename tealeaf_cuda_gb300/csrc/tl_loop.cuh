@@ -8,8 +8,11 @@
 // meeting at each sum.  A CTA stores its partial sum, counts itself in (one
 // atomic on one word) and polls that word; then every CTA adds the same
 // partials in the same order and runs the scalar epilogue on its own copy of
-// the scalars.  A wait that runs out (about two seconds) stops the solve with
-// an error.  Measured on GB300, in clocks: one meeting 2450 to 3200 at any
+// the scalars.  Before anything else the CTAs gather (loop_gather): one that
+// other streams' kernels keep from starting for about two seconds makes the
+// launch return with nothing done, and the passes go on one by one.  Once
+// gathered, a wait of two seconds means that the device does not go on: it stops
+// the solve with an error.  Measured on GB300, in clocks: one meeting 2450 to 3200 at any
 // number of CTAs (an FP64 dependency is 64, a trip to L2 400); letting
 // every CTA poll every other's flag took 7000 with 152 of them, the last
 // arriver's adding and publishing for all 6900, clusters with a leader each
@@ -24,7 +27,7 @@ namespace tl {
 
 namespace {
 
-constexpr long long kLoopWaitCycles = 4000000000LL;  // ~2 s
+constexpr long long kLoopWaitCycles = 4000000000LL;  // ~2 s: the default of both limits
 // A CTA has its multiprocessor's groups (up to 8) in rounds of L.per_round at a
 // time.  One more warp, the control warp, runs the meetings and the scalar
 // code, so that the others' registers hold nothing but their passes.
@@ -35,6 +38,10 @@ struct LoopArgs {
     double *partials;        // [2][kMaxSlots][kLoopSums]
     unsigned int *arrived;   // CTAs that have come to a meeting, over all launches of a solve
     unsigned int *base;      // the value of `arrived` when the launch began
+    unsigned int *gate;      // 2 round + 1: the launch of that round goes on, 2 round: it does not
+    unsigned int round;      // this launch's number
+    long long start_wait;    // clocks to wait for the CTAs to start,
+    long long wait;          // and for them to come to a meeting
     double *cg_alphas, *cg_betas;
     int depth;      // groups of the busiest CTA
     int per_round;  // groups a CTA takes at a time
@@ -50,6 +57,7 @@ struct LoopShared {
     unsigned int target;  // `arrived` when every CTA has come to the meeting
     int parity;
     int stalled;
+    int gathered;
 };
 
 // named barriers (0 is __syncthreads) of the CTA's warps
@@ -113,7 +121,7 @@ __device__ __forceinline__ void loop_meet(const LoopArgs &L, LoopShared &S, int 
                 unsigned int v;
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(L.arrived) : "memory");
                 if ((int)(v - S.target) >= 0) break;
-                if (clock64() - t0 > kLoopWaitCycles) {
+                if (clock64() - t0 > L.wait) {
                     S.stalled = 1;
                     break;
                 }
@@ -159,7 +167,41 @@ __device__ __forceinline__ void loop_meet(const LoopArgs &L, LoopShared &S, int 
     bar_arrive(kBarScalars, blockDim.x);
 }
 
-__device__ __forceinline__ void loop_begin(const LoopArgs &L, LoopShared &S) {
+// whether every CTA of the launch is there, the same answer in all of them (one
+// thread a CTA).  The last to arrive says yes, the first whose wait runs out no;
+// the word that either sets first stands, also for a CTA that starts later.  After
+// a no the last CTA to arrive counts the launch's arrivals off and tells the host.
+__device__ __forceinline__ bool loop_gather(const LoopArgs &L, unsigned int target) {
+    const unsigned int yes = 2 * L.round + 1, no = 2 * L.round;
+    // an earlier launch's word until this one's answer
+    unsigned int word = *(volatile unsigned int *)L.gate;
+    auto answer = [&](unsigned int mine) {
+        if (word >> 1 == L.round) return word;
+        const unsigned int was = atomicCAS(L.gate, word, mine);
+        return was == word ? mine : was;
+    };
+    unsigned int before;
+    // (release: what was read so far, the base among it, was read before)
+    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(before) : "l"(L.arrived) : "memory");
+    if (before + 1 == target) {
+        const bool go = answer(yes) == yes;
+        if (!go) {
+            *L.base = target;
+            *(volatile int *)&L.sc->done = kNotStarted;
+        }
+        return go;
+    }
+    const long long t0 = clock64();
+    for (;;) {
+        unsigned int v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(L.gate) : "memory");
+        if (v >> 1 == L.round) return v == yes;
+        if (clock64() - t0 > L.start_wait) return answer(no) == yes;
+    }
+}
+
+// false: the launch does nothing
+__device__ __forceinline__ bool loop_begin(const LoopArgs &L, LoopShared &S) {
     static_assert(sizeof(DevScalars) % sizeof(int) == 0, "copied by words");
     for (int k = threadIdx.x; k < (int)(sizeof(DevScalars) / sizeof(int)); k += blockDim.x)
         ((int *)&S.sc)[k] = ((const int *)L.sc)[k];
@@ -167,8 +209,14 @@ __device__ __forceinline__ void loop_begin(const LoopArgs &L, LoopShared &S) {
         S.target = *L.base + gridDim.x;
         S.parity = 0;
         S.stalled = 0;
+        S.gathered = 1;
+        if (gridDim.x > 1) {
+            S.gathered = loop_gather(L, S.target);
+            S.target += gridDim.x;
+        }
     }
     __syncthreads();
+    return S.gathered != 0;
 }
 
 // CTA 0 hands the scalars on, and the arrivals counted so far (every CTA has
@@ -417,11 +465,15 @@ int launch_coop(Chunk *c, K kernel, LoopArgs &L, int slots, int threads, size_t 
     L.partials = c->loop_partials;
     L.arrived = c->loop_arrived;
     L.base = c->loop_arrived + 1;
+    L.gate = c->loop_arrived + 32;
+    L.round = ++c->loop_round & 0x7FFFFFFFu;
+    L.start_wait = c->loop_start_wait >= 0 ? c->loop_start_wait : kLoopWaitCycles;
+    L.wait = c->loop_wait >= 0 ? c->loop_wait : kLoopWaitCycles;
     L.cg_alphas = c->cg_alphas;
     L.cg_betas = c->cg_betas;
     // a launch of some tens of milliseconds at most
     const long long it = (1LL << 30) / cells;
-    L.iters = it < 16 ? 16 : it > 1024 ? 1024 : (int)it;
+    L.iters = c->loop_iters > 0 ? c->loop_iters : it < 16 ? 16 : it > 1024 ? 1024 : (int)it;
     void *args[] = {&L, &a...};
     cudaError_t e = cudaSuccess;
     if (smem) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

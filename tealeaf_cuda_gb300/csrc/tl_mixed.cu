@@ -475,7 +475,7 @@ __global__ void __launch_bounds__(kVLoopThreads, 1) k_v_loop(LoopArgs L, GeoV g,
     // completes the last group of sums; before loop_begin's barrier, which alone
     // orders it for the passing warps (kBarSums counts them only)
     if (warp == kVLoopWarps) S.sh[0][warp][lane] = 0.0;
-    loop_begin(L, S);
+    if (!loop_begin(L, S)) return;
     if (warp == kVLoopWarps) {
         for (int it = 0; it < L.iters; ++it) {
             loop_meet<1>(L, S, kEpiStore, [&] { inner_epilogue(&S.sc, kInW, S.sc.sum[0]); });

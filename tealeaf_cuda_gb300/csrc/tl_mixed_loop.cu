@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(Shape::kThreads, 1) k_mixed_ppcg_loop(LoopArgs
     if (*(volatile const int *)&L.sc->done) return;
     __shared__ LoopShared S;
     extern __shared__ float4 smem[];
-    loop_begin(L, S);
+    if (!loop_begin(L, S)) return;
     const float theta_r = (float)(1.0 / S.sc.theta);
     if (threadIdx.x >= blockDim.x - 32) {
         for (int it = 0; it < L.iters; ++it) {

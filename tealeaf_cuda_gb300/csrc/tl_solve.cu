@@ -213,11 +213,18 @@ int run_loop(Chunk *c, int (*loop)(Chunk *), int (*body)(Chunk *), int iters, in
         if (rc == TL_ERR_STATE && !c->loop_ok) return run_phase(c, body, iters, phase, done_out);
         if (rc) return rc;
         if ((rc = chunk_sync_scalars(c))) return rc;
+        if (c->sc_host->done == kNotStarted) {
+            // other work holds multiprocessors: kernels that do not wait for one
+            // another go on from where the launch before this one came to
+            c->sc_host->done = kRunning;
+            if ((rc = chunk_push_scalars(c))) return rc;
+            return run_phase(c, body, iters, phase, done_out);
+        }
         if (c->sc_host->done != kRunning) break;
     }
     *done_out = c->sc_host->done;
     if (*done_out == kStalled) {
-        cudaMemsetAsync(c->loop_arrived, 0, 2 * sizeof(unsigned int), c->stream);
+        TL_CUDA(cudaMemsetAsync(c->loop_arrived, 0, 2 * sizeof(unsigned int), c->stream));
         set_error("the device-resident loop gave up waiting for its thread blocks");
         return TL_ERR_CUDA;
     }
