@@ -106,8 +106,8 @@ def test_blocks_that_start_late(method, precond, start_wait, iters):
     if mixed_cg and start_wait > 0:
         pytest.skip("some launches in loops and some in passes: no bits to compare with")
     deck = _deck(method, precond, (700, 333))
-    got = []
-    for late in (False, True):
+
+    def second_step(late):
         with tl.Chunk(tl.parse_deck(deck)) as ch:
             ch.start()
             ch.timestep()
@@ -115,10 +115,18 @@ def test_blocks_that_start_late(method, precond, start_wait, iters):
                 _set(ch, start_wait=start_wait, iters=iters)
             elif mixed_cg:
                 assert tl.load().tl_set_profiling(ch._h, 1) == 0
-            got.append(_solve(ch, method, steps=1))
-    usual, late = got
-    if start_wait == 0 and not mixed_cg:
-        assert late[2] > usual[2]  # passes
+            return _solve(ch, method, steps=1)
+
+    usual = second_step(False)
+    # now and then all blocks start within one another's first look, and none is late
+    for _ in range(30):
+        late = second_step(True)
+        if not mixed_cg:
+            _same(late, usual)
+        if late[2] > usual[2] or (mixed_cg and late[2] == usual[2]) or start_wait > 0:
+            break
+    else:
+        pytest.fail("no launch was late")
     _same(late, usual)
 
 
