@@ -465,26 +465,30 @@ struct BodyCgWStoreZr {  // BodyCgW and BodyStoreZr in one pass: w = A p, r_stor
 
 // w.z and r.z.  Mixed PPCG's rrn: r - r_store is -alpha w but for r's rounding,
 // so (r - r_store).z = -alpha w.z takes one FP64 instruction a cell instead of
-// two and no stored r; r.z is the next iteration's rro.  HBM-bound.
+// two and reads no r_store; r.z is the next iteration's rro.  HBM-bound.
+// (WZ false: r.z alone, where the last inner pass has summed the other.)
+template <bool WZ>
 struct BodyMixedZr {
-    const double *w, *r, *z;
+    const double *w, *z, *r0, *r1;
+    const int *sel;  // r is in r1 while p is in its second buffer
     int pitch;
-    __device__ void setup() {}
-    __device__ void operator()(int64_t base, int m, double (&acc)[2]) const {
+    const double *r;
+    __device__ void setup() { r = *sel ? r1 : r0; }
+    __device__ void operator()(int64_t base, int m, double (&acc)[WZ ? 2 : 1]) const {
         double wv[4], rv[4], zv[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k)
             if (k < m) {
                 const int64_t i = base + (int64_t)k * pitch;
-                wv[k] = w[i];
+                if (WZ) wv[k] = w[i];
                 rv[k] = r[i];
                 zv[k] = z[i];
             }
 #pragma unroll
         for (int k = 0; k < 4; ++k)
             if (k < m) {
-                acc[0] = fma(wv[k], zv[k], acc[0]);
-                acc[1] = fma(rv[k], zv[k], acc[1]);
+                if (WZ) acc[0] = fma(wv[k], zv[k], acc[0]);
+                acc[WZ ? 1 : 0] = fma(rv[k], zv[k], acc[WZ ? 1 : 0]);
             }
     }
 };
@@ -902,10 +906,10 @@ int launch_ppcg_w_store_zr(Chunk *c, bool fast) {
 
 int launch_mixed_zr(Chunk *c, bool did_rrn) {
     if (did_rrn) {
-        BodyNorm b{c->r, c->z, c->pitch};
+        BodyMixedZr<false> b{c->w, c->z, c->r, c->r_store, &c->sc->p_sel, c->pitch, nullptr};
         return run<1>(c, "ppcg_zr", b, kEpiZrFinish, true);
     }
-    BodyMixedZr b{c->w, c->r, c->z, c->pitch};
+    BodyMixedZr<true> b{c->w, c->z, c->r, c->r_store, &c->sc->p_sel, c->pitch, nullptr};
     return run<2>(c, "ppcg_wz", b, kEpiWzZrFinish, true);
 }
 

@@ -157,6 +157,7 @@ __global__ void __launch_bounds__(Shape::kThreads, 1) k_cg_loop(LoopArgs L, CgAr
 __global__ void __launch_bounds__(kGroupThreads) k_cg_finish(Geo g, CgArgs a, const DevScalars *__restrict__ sc) {
     const double *pin = sc->p_sel ? a.p1 : a.p0;
     const double alpha = sc->alpha, beta = sc->beta;
+    const bool swapped = a.rs && sc->p_sel;  // mixed PPCG: r and r_store take turns as p's buffers do
     const int lane = threadIdx.x & 31;
     for_runs(g, blockIdx.x, threadIdx.x >> 5, [&](int i0, int jb, int je) {
         const int i = i0 + lane;
@@ -179,8 +180,11 @@ __global__ void __launch_bounds__(kGroupThreads) k_cg_finish(Geo g, CgArgs a, co
                     const int64_t c = base + (int64_t)k * g.pitch;
                     a.u[c] = fma(alpha, pv[k], uv[k]);
                     a.p0[c] = fma(beta, pv[k], sv[k]);
-                    // mixed PPCG does without r_store: the r before the last update
-                    if (a.rs) a.rs[c] = fma(alpha, a.w[c], a.r[c]);
+                    if (swapped) {
+                        const double r = a.rs[c];
+                        a.rs[c] = a.r[c];
+                        a.r[c] = r;
+                    }
                 }
         }
     });

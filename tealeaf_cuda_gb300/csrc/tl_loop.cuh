@@ -258,7 +258,7 @@ struct CgArgs {
     double *p0, *p1;    // p's two buffers (DevScalars::p_sel)
     const double *src;  // z, or r without a preconditioner
     const double *kx, *ky, *dg, *mi, *cp, *bfp, *rd;
-    double *rs;         // r_store, where the last pass sets it
+    double *rs;         // r_store, where r takes turns with it (mixed PPCG), else null
 };
 
 // the block-Jacobi factors of the strip whose first row is at c (row j0)

@@ -748,7 +748,7 @@ struct PpFusedArgs {
     // LAST with rrn: also sum (r - r_store).z, the PPCG outer rrn
     // (tea_leaf_ppcg.cuknl:279-297), and run its scalar update
     int rrn;
-    const double *r64, *rs64;
+    const double *r64, *rs64;  // r and r_store, or the other way round (DevScalars::p_sel)
     double *partials;
     unsigned int *counter;
 };
@@ -889,6 +889,8 @@ __global__ void __launch_bounds__(fused_threads<T>(), 2) k_pp_fused(PpFusedArgs 
     for (int k = tid; k < (R * NA + 2 * T) * SR; k += NT) smem4[k] = make_float4(0.f, 0.f, 0.f, 0.f);
     const float theta_r = FIRST ? (float)(1.0 / sc->theta) : 0.f;
     double racc = 0.0;  // LAST with rrn: this thread's (r - r_store).z
+    const double *const r64 = (FIRST || RRN) && sc->p_sel ? a.rs64 : a.r64;
+    const double *const rs64 = RRN && sc->p_sel ? a.r64 : a.rs64;
     // the CTA's share of the band-major sequence of (band, strip) pairs: a
     // share that reaches the end of a band goes on at the top of the next
     // one with a new pipeline (what a pipeline holds before its first strip
@@ -935,7 +937,7 @@ __global__ void __launch_bounds__(fused_threads<T>(), 2) k_pp_fused(PpFusedArgs 
                 const bool v = incol && s >= 0 && row < a.ny;
                 const int i = cbase + (row + a.h) * a.pitch;
                 if constexpr (FIRST) {
-                    o.ldR64[k] = v ? a.r64[cbase + (row + a.h) * a.pitch64] : 0.0;
+                    o.ldR64[k] = v ? r64[cbase + (row + a.h) * a.pitch64] : 0.0;
                 } else {
                     o.ldS[k] = v ? a.sd_in[i] : 0.f;
                     o.ldR[k] = v ? a.rt_in[i] : 0.f;
@@ -971,7 +973,7 @@ __global__ void __launch_bounds__(fused_threads<T>(), 2) k_pp_fused(PpFusedArgs 
             const int row = 4 * s2 + pf_k;
             if (pf_on && s2 >= 0 && row < a.ny) {
                 if (FIRST && pf_arr == 0) {
-                    const double *p = a.r64 + (int64_t)(row + a.h) * a.pitch64 + a.h;
+                    const double *p = r64 + (int64_t)(row + a.h) * a.pitch64 + a.h;
                     asm volatile("prefetch.global.L2 [%0];" ::"l"(p + wc0));
                     asm volatile("prefetch.global.L2 [%0];" ::"l"(p + wc1));
                 } else {
@@ -1162,7 +1164,7 @@ __global__ void __launch_bounds__(fused_threads<T>(), 2) k_pp_fused(PpFusedArgs 
                                     const int i64 = cbase + (row + a.h) * a.pitch64;
                                     const double zv = (double)oU[k];
                                     a.z64[i64] = zv;
-                                    if (RRN) racc = fma(a.r64[i64] - a.rs64[i64], zv, racc);
+                                    if (RRN) racc = fma(r64[i64] - rs64[i64], zv, racc);
                                 } else {
                                     const int i = cbase + (row + a.h) * a.pitch;
                                     a.sd_out[i] = oS[k];
@@ -1300,17 +1302,23 @@ struct BodyUpdateU {  // u += d (FP64), with the last iteration's d += alpha p (
 // preconditioner, so M^-1 uses the FP32 operator copies (the block solve of
 // k_pp_step, 1/diag in bfp's first row).  START false: the r update alone
 // (the first fused inner pass then starts the inner steps from r itself).
-// rs: r_store, where the last inner pass sums (r - r_store).z.
+// r and r_store take turns (DevScalars::p_sel): the new r goes where the r
+// before the old one was, so the old one stays and nothing is stored twice.
 template <int PC, bool START>
 struct BodyPpUr {
     const double *w;
-    double *r, *rs;
+    double *r, *rn;  // the old r and the new one
     const float *mi, *ky, *cp, *bfp;
     float *sd, *rtemp, *utemp;
     int pitch32, pitch64;
     double alpha;
     float theta_r;
     __device__ void setup(DevScalars *sc) {
+        if (!sc->p_sel) {
+            double *const t = r;
+            r = rn;
+            rn = t;
+        }
         alpha = sc->alpha;
         theta_r = (float)(1.0 / sc->theta);
     }
@@ -1339,9 +1347,8 @@ struct BodyPpUr {
         for (int k = 0; k < 4; ++k)
             if (k < m) {
                 const int64_t i = b64 + (int64_t)k * pitch64;
-                if (rs) rs[i] = rv[k];
                 rv[k] = fma(-alpha, wv[k], rv[k]);
-                r[i] = rv[k];
+                rn[i] = rv[k];
                 rf[k] = (float)rv[k];
             }
         if (!START) return;
@@ -1730,10 +1737,9 @@ int mixed_ppcg_ur_inner(Chunk *c, bool *did_rrn) {
     // with fused passes the first pass starts the inner steps from r, and
     // this pass only updates r
     const bool start = fused_steps(c) == 1;
-    const bool fold = !start && c->inner_fold_rrn;
 #define TL_PP_UR(PC, S)                                                                                       \
-    BodyPpUr<PC, S>{c->w, c->r, fold ? c->r_store : nullptr, mx->mi, mx->ky, mx->cp, mx->bfp, mx->sd[0],     \
-                    mx->rtemp, mx->utemp, c->pitch, c->pitch, 0.0, 0.f}
+    BodyPpUr<PC, S>{c->w, c->r, c->r_store, mx->mi, mx->ky, mx->cp, mx->bfp, mx->sd[0], mx->rtemp,          \
+                    mx->utemp, c->pitch, c->pitch, 0.0, 0.f}
     if (!start) rc = run32(c, "mixed_pp_ur", TL_PP_UR(TL_PREC_NONE, false), kInNone, true);
     else if (c->cfg.precond == TL_PREC_JAC_BLOCK)
         rc = run32(c, "mixed_pp_ur", TL_PP_UR(TL_PREC_JAC_BLOCK, true), kInNone, true);

@@ -18,9 +18,12 @@
 // preconditioner.  As many of those arrays as fit are kept in shared memory for
 // the whole launch (a warp's strips in slots of 4 rows by 32 columns, 16-byte
 // loads); only sd goes through L2.  At 1024^2 with block-Jacobi an outer
-// iteration takes 91 us (123 with every array in L2, loaded row by row): the
+// iteration takes 89 us (123 with every array in L2, loaded row by row): the
 // nine plain steps 3.6 us each, their meetings 1.4 each, the FP64 passes 20
-// and 9.5 us.
+// and 9.5 us.  (The new r in the other of two buffers, which keeps the old one for
+// r_store, costs 0.5 % at 512^2, 2.9 % at 1024^2 and 1.2 % at 1400^2; r, r_store and
+// p's two buffers rotating through three, and the iteration once in the code for
+// each place of r, cost as much or more.)
 #include <type_traits>
 
 #include "tl_loop.cuh"
@@ -33,7 +36,7 @@ namespace {
 struct MixedArgs {
     float *sd0, *sd1, *rtemp, *utemp;
     const float *kx, *ky, *mi, *cp, *bfp;  // bfp: 1/diag in each strip's first row
-    double *r, *z;
+    double *r0, *r1, *z;  // r and r_store take turns (DevScalars::p_sel)
     const double *w;
     const double *alphas, *betas;
     int inner;
@@ -152,11 +155,12 @@ __device__ __forceinline__ void precondition(const float (&x)[4], const float (&
     }
 }
 
-// r -= alpha w and the start of the inner steps on a run: rtemp = r, sd = utemp
+// r_new = r_old - alpha w and the start of the inner steps on a run: rtemp = r_new, sd = utemp
 // = M^-1 rtemp / theta
 template <int PC, bool ALL, class Ready>
-__device__ __forceinline__ void mixed_start(const Geo &g, const MixedArgs &a, float4 *smem, int slot, int i0, int jb,
-                                            int je, float theta_r, double &alpha, Ready ready) {
+__device__ __forceinline__ void mixed_start(const Geo &g, const MixedArgs &a, float4 *smem, int slot,
+                                            const double *__restrict__ r_old, double *__restrict__ r_new, int i0,
+                                            int jb, int je, float theta_r, double &alpha, Ready ready) {
     const int i = i0 + (threadIdx.x & 31);
     Strip s{slot, (i + g.h) + (jb + g.h) * g.pitch, g.pitch, 0};
     for (int j0 = jb; j0 < je; j0 += kStrip, s.c += kStrip * s.P, ++s.slot) {
@@ -166,7 +170,7 @@ __device__ __forceinline__ void mixed_start(const Geo &g, const MixedArgs &a, fl
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             w[k] = k < s.m ? __ldcg(a.w + s.c + k * s.P) : 0.0;
-            r[k] = k < s.m ? __ldcg(a.r + s.c + k * s.P) : 0.0;
+            r[k] = k < s.m ? __ldcg(r_old + s.c + k * s.P) : 0.0;
         }
         if (PC != TL_PREC_NONE) private_load<PC, ALL, kPre>(a, smem, s, pre);
         if (PC == TL_PREC_JAC_BLOCK) {
@@ -177,7 +181,7 @@ __device__ __forceinline__ void mixed_start(const Geo &g, const MixedArgs &a, fl
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             const double rv = fma(-alpha, w[k], r[k]);
-            if (k < s.m) a.r[s.c + k * s.P] = rv;
+            if (k < s.m) r_new[s.c + k * s.P] = rv;
             x[k] = (float)rv;
         }
         precondition<PC>(x, pre, kyn, cp, z);
@@ -196,8 +200,8 @@ __device__ __forceinline__ void mixed_start(const Geo &g, const MixedArgs &a, fl
 // while the strip before is computed; what waits for L2 is the run's first load.
 template <int PC, bool ALL, bool LAST>
 __device__ __forceinline__ void mixed_step(const Geo &g, const MixedArgs &a, float4 *smem, int slot,
-                                           const float *__restrict__ xin, float *__restrict__ xout, int i0, int jb,
-                                           int je, float al, float be, double (&acc)[LAST ? 2 : 1]) {
+                                           const float *__restrict__ xin, float *__restrict__ xout, const double *r,
+                                           int i0, int jb, int je, float al, float be, double (&acc)[LAST ? 2 : 1]) {
     const int lane = threadIdx.x & 31, i = i0 + lane;
     const bool own = i < g.nx;
     Strip s{slot, (i + g.h) + (jb + g.h) * g.pitch, g.pitch, 0};
@@ -277,7 +281,7 @@ __device__ __forceinline__ void mixed_step(const Geo &g, const MixedArgs &a, flo
                     const double zv = (double)f[k];
                     a.z[at] = zv;
                     acc[0] = fma(__ldcg(a.w + at), zv, acc[0]);
-                    acc[LAST ? 1 : 0] = fma(__ldcg(a.r + at), zv, acc[LAST ? 1 : 0]);
+                    acc[LAST ? 1 : 0] = fma(__ldcg(r + at), zv, acc[LAST ? 1 : 0]);
                 }
         } else {
             float *po = xout + s.c;
@@ -342,7 +346,7 @@ __global__ void __launch_bounds__(Shape::kThreads, 1) k_mixed_ppcg_loop(LoopArgs
             if (it > 0) loop_met();
             const bool sel = S.sc.p_sel != 0;
             const double *pin = sel ? cg.p1 : cg.p0;
-            double *pout = sel ? cg.p0 : cg.p1;
+            double *pout = sel ? cg.p0 : cg.p1, *r_new = sel ? a.r0 : a.r1;
             bool asked = false, go = false;
             auto ready1 = [&] {
                 if (!asked) {
@@ -371,7 +375,8 @@ __global__ void __launch_bounds__(Shape::kThreads, 1) k_mixed_ppcg_loop(LoopArgs
                 return go;
             };
             slot_pass<0>(L, S, [&](int i0, int jb, int je, int slot, double (&)[1]) {
-                mixed_start<PC, ALL>(L.g, a, smem, slot, i0, jb, je, theta_r, ab.alpha, ready2);
+                mixed_start<PC, ALL>(L.g, a, smem, slot, sel ? a.r1 : a.r0, r_new, i0, jb, je, theta_r, ab.alpha,
+                                     ready2);
             });
             if (!ready2()) break;
             for (int st = 1; st <= a.inner; ++st) {
@@ -383,11 +388,11 @@ __global__ void __launch_bounds__(Shape::kThreads, 1) k_mixed_ppcg_loop(LoopArgs
                 float *xout = st & 1 ? a.sd1 : a.sd0;
                 if (st < a.inner)
                     slot_pass<0>(L, S, [&](int i0, int jb, int je, int slot, double (&acc)[1]) {
-                        mixed_step<PC, ALL, false>(L.g, a, smem, slot, xin, xout, i0, jb, je, al, be, acc);
+                        mixed_step<PC, ALL, false>(L.g, a, smem, slot, xin, xout, r_new, i0, jb, je, al, be, acc);
                     });
                 else
                     slot_pass<2>(L, S, [&](int i0, int jb, int je, int slot, double (&acc)[2]) {
-                        mixed_step<PC, ALL, true>(L.g, a, smem, slot, xin, xout, i0, jb, je, al, be, acc);
+                        mixed_step<PC, ALL, true>(L.g, a, smem, slot, xin, xout, r_new, i0, jb, je, al, be, acc);
                     });
             }
             if (S.stalled) break;
@@ -411,7 +416,8 @@ int launch_mixed_ppcg_loop(Chunk *c) {
     a.mi = mx->mi;
     a.cp = mx->cp;
     a.bfp = mx->bfp;
-    a.r = c->r;
+    a.r0 = c->r;
+    a.r1 = c->r_store;
     a.z = c->z;
     a.w = c->w;
     a.alphas = c->ch_alphas;
