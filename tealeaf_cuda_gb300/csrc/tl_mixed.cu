@@ -1451,7 +1451,7 @@ int launch_v(Chunk *c, const char *name, F &&launch) {
 GeoV run_geo(const Chunk *c, int warps, int unit, unsigned *grid, int least = 8) {
     const Mixed *mx = (const Mixed *)c->mixed;
     GeoV g{c->nx, c->ny, c->h, c->pitch, mx->vtiles_x, mx->vtiles, 0};
-    const int bands = c->sms * warps / g.tiles_x > 1 ? c->sms * warps / g.tiles_x : 1;
+    const int bands = c->g.sms * warps / g.tiles_x > 1 ? c->g.sms * warps / g.tiles_x : 1;
     const int per = (c->ny + bands - 1) / bands;
     g.rows = ((per > least ? per : least) + unit - 1) / unit * unit;
     const long long runs = (long long)g.tiles_x * ((c->ny + g.rows - 1) / g.rows);
@@ -1484,7 +1484,7 @@ template <int PC>
 int inner_loop_pc(Chunk *c) {
     Mixed *mx = mixed_of(c);
     const GeoV g = run_geo(c, kVLoopWarps, PC == TL_PREC_JAC_BLOCK ? 4 : 1, nullptr, 4);
-    const int runs = g.tiles_x * ((c->ny + g.rows - 1) / g.rows), slots = runs < c->sms ? runs : c->sms;
+    const int runs = g.tiles_x * ((c->ny + g.rows - 1) / g.rows), slots = runs < c->g.sms ? runs : c->g.sms;
     LoopArgs L{};
     L.depth = (kVLoopWarps + kGroupWarps - 1) / kGroupWarps;
     L.g.groups = slots * L.depth;
@@ -1502,7 +1502,7 @@ int inner_loop_pc(Chunk *c) {
 bool inner_loop_pays(const Chunk *c) {
     const GeoV g = run_geo(c, kVLoopWarps, 1, nullptr, 4);
     // (a field with more tiles side by side than there are warps has runs left over)
-    return c->loop_ok && !c->profiling && !c->cfg.reflective_boundary && g.tiles_x <= c->sms * kVLoopWarps &&
+    return c->loop_ok && !c->profiling && !c->cfg.reflective_boundary && g.tiles_x <= c->g.sms * kVLoopWarps &&
            g.rows <= kVLoopRows;
 }
 int inner_loop(Chunk *c) {
