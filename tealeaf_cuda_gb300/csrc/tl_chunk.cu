@@ -142,7 +142,7 @@ static int chunk_alloc(const tl_config_t *cfg, Chunk **out) {
     c->warm_projection = TL_WARM_PROJ_ENERGY;
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
-    c->sms = sms > 0 ? sms : 152;
+    c->sms = sms > 0 ? sms : kSms;
     c->grid_red = sms > 0 ? sms * 4 : 512;
     if (c->grid_red > kMaxRedBlocks) c->grid_red = kMaxRedBlocks;
     c->g.sms = c->sms < kMaxSlots ? c->sms : kMaxSlots;

@@ -809,7 +809,7 @@ int launch_conv(const void *in, const void *w, const float *bias, const void *re
                                                    cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
         if (e != cudaSuccess) return cuda_fail(e, "conv shared memory");
         const long long tiles = (((long long)((H + kTcRows - 1) / kTcRows) * (W + 2) + kTcPix - 1) / kTcPix) * B;
-        const long long ctas = 152 * kTcCtas;
+        const long long ctas = kSms * kTcCtas;
         k_conv_tc<CIN, COUTP, MODE><<<(unsigned)(tiles < ctas ? tiles : ctas), 128, bytes, s>>>(
             (const bf16 *)in, (const bf16 *)w, bias, (const bf16 *)res, (bf16 *)out, (bf16 *)pre, outf, B, H, W);
     } else {
@@ -903,7 +903,7 @@ int tl_nn_wgrad(const void *dpre, const void *in, int cin, int coutp, float *par
     const long long blocks = (groups + groups_per_cta - 1) / groups_per_cta;  // room in `partial`
     const long long tasks = (((long long)H * (W + 2) + kWgSeg - 1) / kWgSeg) * B;
     const int n = 9 * cin * coutp;
-    long long ctas = tasks < 152 * 3 ? tasks : 152 * 3;
+    long long ctas = tasks < kSms * 3 ? tasks : kSms * 3;
     const bool bias_here = db && blocks >= 2;
     if (bias_here) {
         // ctas blocks and ctas * coutp floats: floor(blocks * n / (n + coutp))

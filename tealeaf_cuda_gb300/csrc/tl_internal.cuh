@@ -19,11 +19,12 @@
 
 namespace tl {
 
+constexpr int kSms = 152;          // multiprocessors of GB300, where a launch has no chunk to ask
 constexpr int kStrip = 4;          // block-Jacobi strip height (cuda_kernel_header.hpp:11)
 constexpr int kWarpCols = 32;      // columns per warp: one column per lane
-constexpr int kBlockWarps = 8;     // warps per CTA; each warp owns one 4-row strip
+constexpr int kBlockWarps = 8;     // warps per CTA of the FP32 kernels
 constexpr int kBlockThreads = kWarpCols * kBlockWarps;
-constexpr int kGroupWarps = 4;     // FP64 kernels: warps (4-row strips) of a tile
+constexpr int kGroupWarps = 4;     // FP64 kernels: warps of a group, each with a run of strips
 constexpr int kGroupThreads = kWarpCols * kGroupWarps;
 constexpr int kGroupsPerSm = 8;    // 128 threads each: 32 warps a multiprocessor
 constexpr int kMaxSlots = 256;     // multiprocessors a reduction is spread over

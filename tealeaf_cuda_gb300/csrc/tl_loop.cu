@@ -10,9 +10,6 @@
 // instead of 12 and 128.  The neighbours' p' are computed again from z and p
 // (p' goes to the other of two buffers); a last pass brings u and p up to
 // date.  Every value is that of the one-piece kernels, bit for bit.
-#include <math.h>
-#include <string.h>
-
 #include "tl_loop.cuh"
 
 namespace tl {
@@ -263,7 +260,7 @@ __device__ __forceinline__ void step_pass(const Geo &g, const StepArgs &a, const
         const double edge = ex, face = ef;
         e += kStrip * P;
         load_edge(j0 + kStrip);
-        double rv[4], xc[4], qv[4];
+        double rv[4], xc[4] = {}, qv[4] = {};
         // the row's new values from its r and z
         auto finish = [&](int k, double r, double z, double m) {
             const int64_t at = c + k * P;

@@ -62,7 +62,7 @@ constexpr int kCin[kLayers] = {16, 32, 32, 32, 32, 32};
 constexpr int kCout[kLayers] = {32, 32, 32, 32, 32, 16};
 constexpr int kInputs = 7;          // network input channels in use
 constexpr int kFeatures = kInputs + 1;  // + the training target
-constexpr int kGramBlocks = 608;    // 152 SMs x 4
+constexpr int kGramBlocks = 4 * kSms;
 constexpr int kHist = 8;            // previous increments kept (the ring; a chunk uses up to warm_history)
 constexpr int kMaxDirs = kHist + 1; // + the network's direction
 constexpr int kGramPairs = kMaxDirs * (kMaxDirs + 1) / 2;
