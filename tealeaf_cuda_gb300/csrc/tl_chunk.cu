@@ -150,8 +150,16 @@ static int chunk_alloc(const tl_config_t *cfg, Chunk **out) {
         // the shortest runs that the device's groups take in one go
         const long long warps = (long long)c->g.sms * kGroupsPerSm * kGroupWarps;
         const long long bands = warps / c->g.tiles_x > 1 ? warps / c->g.tiles_x : 1;
-        c->g.run = (int)((c->g.nstrips + bands - 1) / bands);
-        c->g.runs = c->g.tiles_x * ((c->g.nstrips + c->g.run - 1) / c->g.run);
+        c->g.run = c->g.band = (int)((c->g.nstrips + bands - 1) / bands);
+        c->g.bands = (c->g.nstrips + c->g.run - 1) / c->g.run;
+        c->g.longer = 0;
+        if (c->g.run > kLoopRun) {
+            // as many bands as there are warps for, of two lengths
+            c->g.bands = (int)bands;
+            c->g.band = c->g.nstrips / c->g.bands;
+            c->g.longer = c->g.nstrips % c->g.bands;
+        }
+        c->g.runs = c->g.tiles_x * c->g.bands;
         c->g.sets = (c->g.runs + kGroupWarps - 1) / kGroupWarps;
         c->g.groups = c->g.sets < c->g.sms * kGroupsPerSm ? c->g.sets : c->g.sms * kGroupsPerSm;
     }

@@ -6,32 +6,6 @@
 
 namespace tl {
 
-// block-Jacobi strip solve z = M^-1 x (tea_block_jacobi.cuknl:11-46)
-__device__ __forceinline__ void strip_block_solve(const double *__restrict__ dg,
-                                                  const double *__restrict__ ky,
-                                                  const double *__restrict__ cp,
-                                                  const double *__restrict__ bfp, int pitch,
-                                                  int64_t base, int m, const double (&x)[4],
-                                                  double (&z)[4]) {
-    double dp[4];
-    dp[0] = x[0] / dg[base];
-#pragma unroll
-    for (int k = 1; k < 4; ++k)
-        if (k < m) {
-            const int64_t i = base + (int64_t)k * pitch;
-            dp[k] = fma(ky[i], dp[k - 1], x[k]) * bfp[i];
-        }
-#pragma unroll
-    for (int k = 3; k >= 0; --k) {
-        if (k == m - 1) {
-            z[k] = dp[k];
-        } else if (k < m - 1) {
-            const int64_t i = base + (int64_t)k * pitch;
-            z[k] = fma(-cp[i], z[k + 1], dp[k]);
-        }
-    }
-}
-
 // x / b, bit for bit, from the correctly rounded reciprocal y of b: two residual
 // corrections of x y.  The first leaves an error below an ulp, and from there, y
 // being correctly rounded, the second rounds correctly (Markstein, "Computation
@@ -50,6 +24,33 @@ __device__ __forceinline__ double div_by(double x, double b, double y) {
     const unsigned int eq = ((unsigned int)__double2hiint(q) >> 20) & 0x7FFu;
     if (ex < 160u || eq == 0x7FFu) q = x == 0.0 ? x * y : div_slow(x, b);
     return q;
+}
+
+// block-Jacobi strip solve z = M^-1 x (tea_block_jacobi.cuknl:11-46); y0: 1 / diag
+// of the strip's first row
+__device__ __forceinline__ void strip_block_solve(const double *__restrict__ dg, double y0,
+                                                  const double *__restrict__ ky,
+                                                  const double *__restrict__ cp,
+                                                  const double *__restrict__ bfp, int pitch,
+                                                  int64_t base, int m, const double (&x)[4],
+                                                  double (&z)[4]) {
+    double dp[4];
+    dp[0] = div_by(x[0], dg[base], y0);
+#pragma unroll
+    for (int k = 1; k < 4; ++k)
+        if (k < m) {
+            const int64_t i = base + (int64_t)k * pitch;
+            dp[k] = fma(ky[i], dp[k - 1], x[k]) * bfp[i];
+        }
+#pragma unroll
+    for (int k = 3; k >= 0; --k) {
+        if (k == m - 1) {
+            z[k] = dp[k];
+        } else if (k < m - 1) {
+            const int64_t i = base + (int64_t)k * pitch;
+            z[k] = fma(-cp[i], z[k + 1], dp[k]);
+        }
+    }
 }
 
 // strip_block_solve on values that are in registers: the first row's diagonal

@@ -5,9 +5,12 @@
 //
 // Order of a grid-wide sum.  A run is 32 columns, one a lane, by some 4-row
 // strips, taken from the top down by one warp; the field is cut into bands of
-// `run` strips, as few as the device's warps take in one go, so runs side by
+// strips, as few as the device's warps take in one go, so runs side by
 // side are at the same rows at the same time and find their neighbours' values
-// in the caches.  Four runs side by side are a set, a group's 4 warps.  Group q
+// in the caches.  Bands of more than kLoopRun strips are as many as there are
+// warps for, of two lengths that differ by one: with ceil(nstrips / bands) in all of
+// them 7 % of the warps had nothing at 2600^2 cells (CG with block-Jacobi 268 us
+// an iteration, now 238).  Four runs side by side are a set, a group's 4 warps.  Group q
 // of G takes the sets q, q + G, ...; a lane adds up its cells in that order,
 // row by row.  The group adds its warps lane by lane, (w0 + w1) + (w2 + w3), then its lanes in
 // an xor butterfly.  The groups q, q + S, q + 2S, ... are slot q of S = one a
@@ -198,7 +201,7 @@ __device__ __forceinline__ void for_runs(const Geo &g, int group, int warp, F f)
         const int r = t * kGroupWarps + warp;
         if (r >= g.runs) break;
         const int b = r / g.tiles_x, tx = r - b * g.tiles_x;
-        const int s0 = b * g.run, s1 = min(s0 + g.run, g.nstrips);
+        const int s0 = b * g.band + min(b, g.longer), s1 = min(s0 + g.band + (b < g.longer), g.nstrips);
         f(tx * kWarpCols, s0 * kStrip, min(s1 * kStrip, g.ny));
     }
 }
@@ -218,7 +221,7 @@ __device__ __forceinline__ double group_sum(const double (*sh)[32], int lane) {
 }
 
 // grid-wide sums of one-group CTAs; the last CTA (a ticket, nobody waits)
-// adds the partials and runs the epilogue
+// adds the partials, a warp a sum if there are several, and runs the epilogue
 template <int NV>
 __device__ __forceinline__ void grid_reduce(double (&acc)[NV > 0 ? NV : 1], const RedCtx &red, int sms) {
     constexpr int N = NV > 0 ? NV : 1;
@@ -245,20 +248,36 @@ __device__ __forceinline__ void grid_reduce(double (&acc)[NV > 0 ? NV : 1], cons
     __threadfence();
     const int groups = gridDim.x, slots = groups < sms ? groups : sms;
     double tot[N];
+    if (NV > 1) {
+        // a warp a sum
+        static_assert(NV <= kGroupWarps, "a warp a sum");
+        __shared__ double all[N];
+        if (warp < NV) {
+            const double *part = red.partials + warp * kMaxRedBlocks;
+            double t = 0.0;
+            for (int c = lane; c < slots; c += 32) {
+                double s = __ldcg(&part[c]);
+                for (int q = c + slots; q < groups; q += slots) s += __ldcg(&part[q]);
+                t = c == lane ? s : t + s;
+            }
+            t = warp_sum(t);
+            if (lane == 0) all[warp] = t;
+        }
+        __syncthreads();
 #pragma unroll
-    for (int v = 0; v < NV; ++v) {
+        for (int v = 0; v < NV; ++v) tot[v] = all[v];
+    } else if (NV == 1) {
         for (int c = threadIdx.x; c < slots; c += kGroupThreads) {
-            double t = __ldcg(&red.partials[v * kMaxRedBlocks + c]);
-            for (int q = c + slots; q < groups; q += slots) t += __ldcg(&red.partials[v * kMaxRedBlocks + q]);
+            double t = __ldcg(&red.partials[c]);
+            for (int q = c + slots; q < groups; q += slots) t += __ldcg(&red.partials[q]);
             slot[c] = t;
         }
         __syncthreads();
         if (warp == 0) {
             double t = lane < slots ? slot[lane] : 0.0;
             for (int c = lane + 32; c < slots; c += 32) t += slot[c];
-            tot[v] = warp_sum(t);
+            tot[0] = warp_sum(t);
         }
-        __syncthreads();
     }
     if (threadIdx.x == 0) {
         run_epilogue(red, tot, NV);

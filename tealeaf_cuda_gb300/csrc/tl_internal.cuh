@@ -27,6 +27,7 @@ constexpr int kBlockThreads = kWarpCols * kBlockWarps;
 constexpr int kGroupWarps = 4;     // FP64 kernels: warps of a group, each with a run of strips
 constexpr int kGroupThreads = kWarpCols * kGroupWarps;
 constexpr int kGroupsPerSm = 8;    // 128 threads each: 32 warps a multiprocessor
+constexpr int kLoopRun = 8;        // most strips of a run that loop kernels take (loop_pays)
 constexpr int kMaxSlots = 256;     // multiprocessors a reduction is spread over
 constexpr int kMaxRedBlocks = kMaxSlots * kGroupsPerSm;  // grid cap for reducing kernels
 
@@ -104,8 +105,10 @@ struct Geo {
     int tiles_y;        // ceil(nstrips / 8)
     int tiles;
     // the FP64 kernels' runs of strips (tl_fp64.cuh)
-    int run;            // strips of a run
-    int runs;           // tiles_x * ceil(nstrips / run)
+    int run;            // strips of the longest run
+    int bands;          // runs above one another:
+    int band, longer;   // `band` strips each, one more in the first `longer`, what is there in the last
+    int runs;           // tiles_x * bands
     int sets;           // ceil(runs / 4): a set is four runs side by side
     int groups;         // 4-warp groups that share them: min(sets, sms * 8)
     int sms;            // multiprocessors (at most kMaxSlots): the slots of a sum
@@ -131,8 +134,8 @@ struct Chunk {
     double *density, *energy0, *energy1, *u, *u0, *p, *r, *w, *z, *mi, *kx, *ky, *sd,
         *rtemp, *utemp, *r_store, *cp, *bfp, *volume, *un;
     double *diag;                // diag(A), refreshed with Kx/Ky by common_init
-    double *rdiag;               // block-Jacobi: 1 / diag of each strip's first row (nstrips rows); of
-                                 // the present diag only once cg_init has followed common_init
+    double *rdiag;               // block-Jacobi: 1 / diag of each strip's first row (nstrips rows),
+                                 // stored with diag
     double *sd_alt;              // FP64 PPCG: second buffer of sd (allocated on first use)
     bool no_sd_alt;              // there was no memory for it: FP64 PPCG runs its single pieces
     double *stage;               // (rows x (nx + 2h)) contiguous copy buffer of

@@ -24,9 +24,23 @@
 
 namespace tl {
 
+// 1 / diag of the strips' first rows (Chunk::rdiag) as the bodies index it: by
+// the strip's first cell and its number
+static double *first_rows(Chunk *c) { return c->rdiag ? c->rdiag - (int64_t)c->h * c->pitch : nullptr; }
+__device__ __forceinline__ double first_row(const double *rd, int strip, int64_t base, int pitch) {
+    return rd[base - (int64_t)(3 * strip) * pitch];
+}
+// a body that has a member `strip` is told the strip's number
+template <class Body>
+__device__ __forceinline__ auto set_strip(Body &body, int s, int) -> decltype((void)(body.strip = s)) {
+    body.strip = s;
+}
+template <class Body>
+__device__ __forceinline__ void set_strip(Body &, int, long) {}
+
 // The grid-stride strip kernel: Body processes one strip column.
-template <int NV, class Body>
-__global__ void __launch_bounds__(kGroupThreads) k_strips(Geo g, Body body, RedCtx red) {
+template <int NV, class Body, int CTAS>
+__global__ void __launch_bounds__(kGroupThreads, CTAS) k_strips(Geo g, Body body, RedCtx red) {
     if (red.done && *(volatile const int *)red.done) return;
     double acc[NV > 0 ? NV : 1];
 #pragma unroll
@@ -36,8 +50,10 @@ __global__ void __launch_bounds__(kGroupThreads) k_strips(Geo g, Body body, RedC
     for_runs(g, blockIdx.x, warp, [&](int i0, int jb, int je) {
         const int i = i0 + lane;
         if (i >= g.nx) return;
-        for (int j0 = jb; j0 < je; j0 += kStrip)
+        for (int j0 = jb; j0 < je; j0 += kStrip) {
+            set_strip(body, j0 / kStrip, 0);
             body((int64_t)(i + g.h) + (int64_t)(j0 + g.h) * g.pitch, min(kStrip, je - j0), acc);
+        }
     });
     if (red.epi != kEpiNone) grid_reduce<NV>(acc, red, g.sms);
 }
@@ -64,8 +80,8 @@ struct BodyCgInit {  // tea_leaf_kernel_cuda.cu:164-186 fused per strip
     const double *r, *kx, *ky;
     double *p, *z, *mi, *cp, *bfp;
     int pitch;
-    double *rd;  // 1 / diag of the strips' first rows, a row a strip
-    int h;
+    const double *rd;
+    int strip;
     __device__ void setup() {}
     __device__ void operator()(int64_t base, int m, double (&acc)[1]) const {
         double rv[4], zv[4];
@@ -73,10 +89,9 @@ struct BodyCgInit {  // tea_leaf_kernel_cuda.cu:164-186 fused per strip
         for (int k = 0; k < 4; ++k)
             if (k < m) rv[k] = r[base + (int64_t)k * pitch];
         if (PC == TL_PREC_JAC_BLOCK) {
-            const int row = (int)(base / pitch);
-            rd[base - (int64_t)row * pitch + (int64_t)((row - h) / kStrip) * pitch] = 1.0 / dg[base];
+            const double y0 = first_row(rd, strip, base, pitch);
             // block_init (tea_block_jacobi.cuknl:83-111)
-            double cprev = (-ky[base + pitch]) / dg[base];
+            double cprev = div_by(-ky[base + pitch], dg[base], y0);
             cp[base] = cprev;
 #pragma unroll
             for (int k = 1; k < 4; ++k)
@@ -87,7 +102,7 @@ struct BodyCgInit {  // tea_leaf_kernel_cuda.cu:164-186 fused per strip
                     cprev = (-ky[i + pitch]) * bf;
                     cp[i] = cprev;
                 }
-            strip_block_solve(dg, ky, cp, bfp, pitch, base, m, rv, zv);
+            strip_block_solve(dg, y0, ky, cp, bfp, pitch, base, m, rv, zv);
         }
 #pragma unroll
         for (int k = 0; k < 4; ++k)
@@ -139,6 +154,8 @@ struct BodyCgUr {  // tea_leaf_cg.cuknl:72-137
     double alpha_v;
     int pitch;
     double alpha;
+    const double *rd;
+    int strip;
     __device__ void setup() { alpha = coef(alpha_p, alpha_v); }
     __device__ void operator()(int64_t base, int m, double (&acc)[1]) const {
         // every load of the strip before the first store (the arrays may
@@ -160,7 +177,7 @@ struct BodyCgUr {  // tea_leaf_cg.cuknl:72-137
                 uv[k] = fma(alpha, pv[k], uv[k]);
                 rv[k] = fma(-alpha, wv[k], rv[k]);
             }
-        if (PC == TL_PREC_JAC_BLOCK) strip_block_solve(dg, ky, cp, bfp, pitch, base, m, rv, zv);
+        if (PC == TL_PREC_JAC_BLOCK) strip_block_solve(dg, first_row(rd, strip, base, pitch), ky, cp, bfp, pitch, base, m, rv, zv);
 #pragma unroll
         for (int k = 0; k < 4; ++k)
             if (k < m) {
@@ -211,6 +228,8 @@ struct BodyChebyInitP {  // tea_leaf_cheby.cuknl:5-68
     double *p, *r, *w;
     double theta;
     int pitch;
+    const double *rd;
+    int strip;
     __device__ void setup() {}
     __device__ void operator()(int64_t base, int m, double (&acc)[1]) const {
         double xc[4], ax[4], rv[4], zv[4];
@@ -223,7 +242,7 @@ struct BodyChebyInitP {  // tea_leaf_cheby.cuknl:5-68
                 rv[k] = u0[i] - ax[k];
                 r[i] = rv[k];
             }
-        if (PC == TL_PREC_JAC_BLOCK) strip_block_solve(dg, ky, cp, bfp, pitch, base, m, rv, zv);
+        if (PC == TL_PREC_JAC_BLOCK) strip_block_solve(dg, first_row(rd, strip, base, pitch), ky, cp, bfp, pitch, base, m, rv, zv);
 #pragma unroll
         for (int k = 0; k < 4; ++k)
             if (k < m) {
@@ -244,6 +263,8 @@ struct BodyChebyCalcP {  // tea_leaf_cheby.cuknl:84-152 (+ r.r for the exit test
     int step_v;          // 1-based step
     int pitch;
     double al, be;
+    const double *rd;
+    int strip;
     __device__ void setup() {
         const int st = step_p ? *step_p : step_v;
         al = alphas[st - 1];
@@ -261,7 +282,7 @@ struct BodyChebyCalcP {  // tea_leaf_cheby.cuknl:84-152 (+ r.r for the exit test
                 r[i] = rv[k];
                 acc[0] = fma(rv[k], rv[k], acc[0]);
             }
-        if (PC == TL_PREC_JAC_BLOCK) strip_block_solve(dg, ky, cp, bfp, pitch, base, m, rv, zv);
+        if (PC == TL_PREC_JAC_BLOCK) strip_block_solve(dg, first_row(rd, strip, base, pitch), ky, cp, bfp, pitch, base, m, rv, zv);
 #pragma unroll
         for (int k = 0; k < 4; ++k)
             if (k < m) {
@@ -294,6 +315,8 @@ struct BodyPpcgInit {  // tea_leaf_ppcg.cuknl:319-420
     const double *r, *mi, *kx, *ky, *cp, *bfp;
     double *p, *z;
     int step, pitch;
+    const double *rd;
+    int strip;
     __device__ void setup() {}
     __device__ void operator()(int64_t base, int m, double (&acc)[1]) const {
         double zv[4], rv[4];
@@ -301,7 +324,7 @@ struct BodyPpcgInit {  // tea_leaf_ppcg.cuknl:319-420
         for (int k = 0; k < 4; ++k)
             if (k < m) rv[k] = r[base + (int64_t)k * pitch];
         const bool do_z = (PC != TL_PREC_NONE || step == 3) && (step == 1 || step == 2);
-        if (do_z && PC == TL_PREC_JAC_BLOCK) strip_block_solve(dg, ky, cp, bfp, pitch, base, m, rv, zv);
+        if (do_z && PC == TL_PREC_JAC_BLOCK) strip_block_solve(dg, first_row(rd, strip, base, pitch), ky, cp, bfp, pitch, base, m, rv, zv);
 #pragma unroll
         for (int k = 0; k < 4; ++k)
             if (k < m) {
@@ -334,13 +357,15 @@ struct BodyPpcgInitSd {  // tea_leaf_ppcg.cuknl:5-55 (not used by the driver)
     double *sd;
     double theta;
     int pitch;
+    const double *rd;
+    int strip;
     __device__ void setup() {}
     __device__ void operator()(int64_t base, int m, double (&acc)[1]) const {
         double rv[4], zv[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k)
             if (k < m) rv[k] = r[base + (int64_t)k * pitch];
-        if (PC == TL_PREC_JAC_BLOCK) strip_block_solve(dg, ky, cp, bfp, pitch, base, m, rv, zv);
+        if (PC == TL_PREC_JAC_BLOCK) strip_block_solve(dg, first_row(rd, strip, base, pitch), ky, cp, bfp, pitch, base, m, rv, zv);
 #pragma unroll
         for (int k = 0; k < 4; ++k)
             if (k < m) {
@@ -401,6 +426,8 @@ struct BodyPpcgCalcSdNew {  // tea_leaf_ppcg.cuknl:178-244
     int step;  // 1-based inner step
     int pitch;
     double al, be;
+    const double *rd;
+    int strip;
     __device__ void setup() {
         al = alphas[step - 1];
         be = betas[step - 1];
@@ -410,7 +437,7 @@ struct BodyPpcgCalcSdNew {  // tea_leaf_ppcg.cuknl:178-244
 #pragma unroll
         for (int k = 0; k < 4; ++k)
             if (k < m) rv[k] = rtemp[base + (int64_t)k * pitch];
-        if (PC == TL_PREC_JAC_BLOCK) strip_block_solve(dg, ky, cp, bfp, pitch, base, m, rv, zv);
+        if (PC == TL_PREC_JAC_BLOCK) strip_block_solve(dg, first_row(rd, strip, base, pitch), ky, cp, bfp, pitch, base, m, rv, zv);
 #pragma unroll
         for (int k = 0; k < 4; ++k)
             if (k < m) {
@@ -567,13 +594,17 @@ struct BodyDiag {  // diag(A) of tea_leaf_common.cuknl:137-139, once per solve
     const double *kx, *ky;
     double *dg;
     int pitch;
+    double *rd;  // block-Jacobi: and 1 / diag of the strip's first row
+    int strip;
     __device__ void setup() {}
     __device__ void operator()(int64_t base, int m, double (&acc)[1]) const {
 #pragma unroll
         for (int k = 0; k < 4; ++k)
             if (k < m) {
                 const int64_t i = base + (int64_t)k * pitch;
-                dg[i] = diag_at(kx, ky, i, pitch);
+                const double d = diag_at(kx, ky, i, pitch);
+                dg[i] = d;
+                if (k == 0 && rd) rd[base - (int64_t)(3 * strip) * pitch] = 1.0 / d;
             }
     }
 };
@@ -690,7 +721,12 @@ __global__ void k_reflect(Geo g, double *__restrict__ f, int depth, int pass) {
 
 // ------------------------------------------------------------- launchers
 
-template <int NV, class Body>
+// NV: the sums that the body adds up; CTAS: CTAs that a multiprocessor holds at
+// once.  A sum's runs are cut for kGroupsPerSm of them, so the kernels that add up
+// are held to 64 registers: with 72 to 91 six or five were resident, and the
+// other two or three of a multiprocessor's groups had it to themselves.
+// (4096^2 cells: cg_ur with block-Jacobi 345 -> 234 us, cheby_p 454 to 618 -> 330 to 480.)
+template <int NV, int CTAS = NV == 0 ? 0 : kGroupsPerSm, class Body>
 static int run(Chunk *c, const char *name, const Body &body, int epi, bool fast) {
     int slot = -1;
     if (c->profiling && !c->capturing) prof_begin(c, name, &slot);
@@ -698,12 +734,14 @@ static int run(Chunk *c, const char *name, const Body &body, int epi, bool fast)
     // multiprocessor then holds more warps than the 32 that the runs are cut for.
     // (8192^2 cells: copy 257 -> 183 us, finalise 1017 -> 929, generate 2886 -> 2581, diag 546 -> 520.)
     Geo g = c->g;
-    if (epi == kEpiNone && g.run > 2) {
-        g.run = 2;
-        g.runs = g.tiles_x * ((g.nstrips + 1) / 2);
+    if ((epi == kEpiNone || NV == 0) && g.run > 2) {
+        g.run = g.band = 2;
+        g.bands = (g.nstrips + 1) / 2;
+        g.longer = 0;
+        g.runs = g.tiles_x * g.bands;
         g.sets = g.groups = (g.runs + kGroupWarps - 1) / kGroupWarps;
     }
-    k_strips<NV, Body><<<g.groups, kGroupThreads, 0, c->stream>>>(g, body, red_ctx(c, epi, fast));
+    k_strips<NV, Body, CTAS><<<g.groups, kGroupThreads, 0, c->stream>>>(g, body, red_ctx(c, epi, fast));
     if (slot >= 0) prof_end(c, slot);
     c->launches++;
     cudaError_t e = cudaGetLastError();
@@ -727,8 +765,8 @@ int launch_common_init(Chunk *c, int coefficient, double rx, double ry, const in
     c->launches++;
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "common_init launch");
-    BodyDiag bd{c->kx, c->ky, c->diag, c->pitch};
-    return run<1>(c, "diag", bd, kEpiNone, false);
+    BodyDiag bd{c->kx, c->ky, c->diag, c->pitch, first_rows(c), 0};
+    return run<0>(c, "diag", bd, kEpiNone, false);
 }
 
 int launch_norm(Chunk *c, const double *a, const double *bb, int epi) {
@@ -740,17 +778,17 @@ int launch_cg_init(Chunk *c, int epi) {
     switch (c->cfg.precond) {
     case TL_PREC_JAC_BLOCK: {
         BodyCgInit<TL_PREC_JAC_BLOCK> b{c->diag, c->r, c->kx, c->ky, c->p, c->z, c->mi, c->cp, c->bfp, c->pitch,
-                                        c->rdiag, c->h};
+                                        first_rows(c), 0};
         return run<1>(c, "cg_init", b, epi, false);
     }
     case TL_PREC_JAC_DIAG: {
         BodyCgInit<TL_PREC_JAC_DIAG> b{c->diag, c->r, c->kx, c->ky, c->p, c->z, c->mi, c->cp, c->bfp, c->pitch,
-                                        c->rdiag, c->h};
+                                        first_rows(c), 0};
         return run<1>(c, "cg_init", b, epi, false);
     }
     default: {
         BodyCgInit<TL_PREC_NONE> b{c->diag, c->r, c->kx, c->ky, c->p, c->z, c->mi, c->cp, c->bfp, c->pitch,
-                                        c->rdiag, c->h};
+                                        first_rows(c), 0};
         return run<1>(c, "cg_init", b, epi, false);
     }
     }
@@ -764,7 +802,7 @@ int launch_cg_w(Chunk *c, int epi, bool fast) {
 template <int PC>
 static int cg_ur(Chunk *c, double alpha, int epi, bool fast) {
     BodyCgUr<PC> b{c->diag, c->u, c->r, c->z, c->p, c->w, c->mi, c->kx, c->ky, c->cp, c->bfp,
-                   fast ? &c->sc->alpha : nullptr, alpha, c->pitch, 0.0};
+                   fast ? &c->sc->alpha : nullptr, alpha, c->pitch, 0.0, first_rows(c), 0};
     return run<1>(c, "cg_ur", b, epi, fast);
 }
 
@@ -779,25 +817,25 @@ int launch_cg_ur(Chunk *c, double alpha, int epi, bool fast) {
 int launch_cg_p(Chunk *c, double beta, int epi, bool fast) {
     const double *src = c->cfg.precond != TL_PREC_NONE ? c->z : c->r;
     BodyAxpyP b{c->p, src, fast ? &c->sc->beta : nullptr, beta, c->pitch, 0.0};
-    return run<1>(c, "cg_p", b, epi, fast);
+    return run<0>(c, "cg_p", b, epi, fast);
 }
 
 int launch_cheby_init(Chunk *c, double theta) {
     switch (c->cfg.precond) {
     case TL_PREC_JAC_BLOCK: {
         BodyChebyInitP<TL_PREC_JAC_BLOCK> b{c->diag, c->u, c->u0, c->kx, c->ky, c->mi, c->cp, c->bfp,
-                                            c->p, c->r, c->w, theta, c->pitch};
-        return run<1>(c, "cheby_init", b, kEpiNone, false);
+                                            c->p, c->r, c->w, theta, c->pitch, first_rows(c), 0};
+        return run<0>(c, "cheby_init", b, kEpiNone, false);
     }
     case TL_PREC_JAC_DIAG: {
         BodyChebyInitP<TL_PREC_JAC_DIAG> b{c->diag, c->u, c->u0, c->kx, c->ky, c->mi, c->cp, c->bfp,
-                                           c->p, c->r, c->w, theta, c->pitch};
-        return run<1>(c, "cheby_init", b, kEpiNone, false);
+                                           c->p, c->r, c->w, theta, c->pitch, first_rows(c), 0};
+        return run<0>(c, "cheby_init", b, kEpiNone, false);
     }
     default: {
         BodyChebyInitP<TL_PREC_NONE> b{c->diag, c->u, c->u0, c->kx, c->ky, c->mi, c->cp, c->bfp,
-                                       c->p, c->r, c->w, theta, c->pitch};
-        return run<1>(c, "cheby_init", b, kEpiNone, false);
+                                       c->p, c->r, c->w, theta, c->pitch, first_rows(c), 0};
+        return run<0>(c, "cheby_init", b, kEpiNone, false);
     }
     }
 }
@@ -806,7 +844,7 @@ template <int PC>
 static int cheby_p(Chunk *c, int step, int epi, bool fast) {
     BodyChebyCalcP<PC> b{c->diag, c->u, c->u0, c->kx, c->ky, c->mi, c->cp, c->bfp, c->ch_alphas,
                          c->ch_betas, c->p, c->r, c->w,
-                         fast ? &c->sc->cheby_calc_steps : nullptr, step, c->pitch, 0.0, 0.0};
+                         fast ? &c->sc->cheby_calc_steps : nullptr, step, c->pitch, 0.0, 0.0, first_rows(c), 0};
     return run<1>(c, "cheby_p", b, epi, fast);
 }
 
@@ -820,12 +858,12 @@ int launch_cheby_calc_p(Chunk *c, int step, int epi, bool fast) {
 
 int launch_cheby_calc_u(Chunk *c, int epi, bool fast) {
     BodyAdd b{c->u, c->p, c->pitch};
-    return run<1>(c, "cheby_calc_u", b, epi, fast);
+    return run<0>(c, "cheby_calc_u", b, epi, fast);
 }
 
 template <int PC>
 static int ppcg_init(Chunk *c, int step, int epi) {
-    BodyPpcgInit<PC> b{c->diag, c->r, c->mi, c->kx, c->ky, c->cp, c->bfp, c->p, c->z, step, c->pitch};
+    BodyPpcgInit<PC> b{c->diag, c->r, c->mi, c->kx, c->ky, c->cp, c->bfp, c->p, c->z, step, c->pitch, first_rows(c), 0};
     return run<1>(c, "ppcg_init", b, epi, false);
 }
 
@@ -840,16 +878,16 @@ int launch_ppcg_init(Chunk *c, int step, int epi) {
 int launch_ppcg_init_sd(Chunk *c, double theta) {
     switch (c->cfg.precond) {
     case TL_PREC_JAC_BLOCK: {
-        BodyPpcgInitSd<TL_PREC_JAC_BLOCK> b{c->diag, c->r, c->mi, c->kx, c->ky, c->cp, c->bfp, c->sd, theta, c->pitch};
-        return run<1>(c, "ppcg_init_sd", b, kEpiNone, false);
+        BodyPpcgInitSd<TL_PREC_JAC_BLOCK> b{c->diag, c->r, c->mi, c->kx, c->ky, c->cp, c->bfp, c->sd, theta, c->pitch, first_rows(c), 0};
+        return run<0>(c, "ppcg_init_sd", b, kEpiNone, false);
     }
     case TL_PREC_JAC_DIAG: {
-        BodyPpcgInitSd<TL_PREC_JAC_DIAG> b{c->diag, c->r, c->mi, c->kx, c->ky, c->cp, c->bfp, c->sd, theta, c->pitch};
-        return run<1>(c, "ppcg_init_sd", b, kEpiNone, false);
+        BodyPpcgInitSd<TL_PREC_JAC_DIAG> b{c->diag, c->r, c->mi, c->kx, c->ky, c->cp, c->bfp, c->sd, theta, c->pitch, first_rows(c), 0};
+        return run<0>(c, "ppcg_init_sd", b, kEpiNone, false);
     }
     default: {
-        BodyPpcgInitSd<TL_PREC_NONE> b{c->diag, c->r, c->mi, c->kx, c->ky, c->cp, c->bfp, c->sd, theta, c->pitch};
-        return run<1>(c, "ppcg_init_sd", b, kEpiNone, false);
+        BodyPpcgInitSd<TL_PREC_NONE> b{c->diag, c->r, c->mi, c->kx, c->ky, c->cp, c->bfp, c->sd, theta, c->pitch, first_rows(c), 0};
+        return run<0>(c, "ppcg_init_sd", b, kEpiNone, false);
     }
     }
 }
@@ -858,22 +896,22 @@ int launch_ppcg_init_sd_new(Chunk *c, double theta, bool fast) {
     const double *tp = fast ? &c->sc->theta : nullptr;
     if (c->cfg.precond != TL_PREC_NONE) {
         BodyPpcgInitSdNew<TL_PREC_JAC_DIAG> b{c->r, c->z, c->sd, c->rtemp, c->utemp, tp, theta, c->pitch};
-        return run<1>(c, "ppcg_init_sd_new", b, kEpiNone, fast);
+        return run<0>(c, "ppcg_init_sd_new", b, kEpiNone, fast);
     }
     BodyPpcgInitSdNew<TL_PREC_NONE> b{c->r, c->z, c->sd, c->rtemp, c->utemp, tp, theta, c->pitch};
-    return run<1>(c, "ppcg_init_sd_new", b, kEpiNone, fast);
+    return run<0>(c, "ppcg_init_sd_new", b, kEpiNone, fast);
 }
 
 int launch_ppcg_update_r(Chunk *c, bool fast) {
     BodyPpcgUpdateR b{c->diag, c->sd, c->kx, c->ky, c->rtemp, c->pitch};
-    return run<1>(c, "ppcg_update_r", b, kEpiNone, fast);
+    return run<0>(c, "ppcg_update_r", b, kEpiNone, fast);
 }
 
 template <int PC>
 static int ppcg_sd(Chunk *c, int step, bool fast) {
     BodyPpcgCalcSdNew<PC> b{c->diag, c->rtemp, c->mi, c->kx, c->ky, c->cp, c->bfp, c->ch_alphas,
-                            c->ch_betas, c->sd, c->utemp, step, c->pitch, 0.0, 0.0};
-    return run<1>(c, "ppcg_sd", b, kEpiNone, fast);
+                            c->ch_betas, c->sd, c->utemp, step, c->pitch, 0.0, 0.0, first_rows(c), 0};
+    return run<0>(c, "ppcg_sd", b, kEpiNone, fast);
 }
 
 int launch_ppcg_calc_sd_new(Chunk *c, int step, bool fast) {
@@ -886,7 +924,7 @@ int launch_ppcg_calc_sd_new(Chunk *c, int step, bool fast) {
 
 int launch_copy(Chunk *c, double *dst, const double *src, bool fast) {
     BodyCopy b{dst, src, c->pitch};
-    return run<1>(c, "copy", b, kEpiNone, fast);
+    return run<0>(c, "copy", b, kEpiNone, fast);
 }
 
 int launch_ppcg_rrn(Chunk *c, int epi, bool fast) {
@@ -915,7 +953,7 @@ int launch_mixed_zr(Chunk *c, bool did_rrn) {
 
 int launch_ppcg_p(Chunk *c, double beta, int epi, bool fast) {
     BodyAxpyP b{c->p, c->z, fast ? &c->sc->beta : nullptr, beta, c->pitch, 0.0};
-    return run<1>(c, "ppcg_p", b, epi, fast);
+    return run<0>(c, "ppcg_p", b, epi, fast);
 }
 
 int launch_jacobi(Chunk *c, int epi, bool fast) {
@@ -927,7 +965,7 @@ int launch_jacobi(Chunk *c, int epi, bool fast) {
 
 int launch_finalise(Chunk *c) {
     BodyFinalise b{c->u, c->density, c->energy1, c->pitch};
-    return run<1>(c, "finalise", b, kEpiNone, false);
+    return run<0>(c, "finalise", b, kEpiNone, false);
 }
 
 int launch_field_summary(Chunk *c) {
@@ -939,13 +977,13 @@ int launch_set_field(Chunk *c) { return launch_copy(c, c->energy1, c->energy0, f
 
 int launch_fill(Chunk *c, double *f, double v) {
     BodyFill b{f, v, c->pitch};
-    return run<1>(c, "fill", b, kEpiNone, false);
+    return run<0>(c, "fill", b, kEpiNone, false);
 }
 
 int launch_generate(Chunk *c, int nstates, const tl_state_t *states_dev) {
     BodyGenerate b{c->density, c->energy0, c->u, c->u0, c->vertexx, c->vertexy, c->cellx,
                    c->celly, states_dev, nstates, c->h, c->pitch};
-    return run<1>(c, "generate", b, kEpiNone, false);
+    return run<0>(c, "generate", b, kEpiNone, false);
 }
 
 int launch_reflect(Chunk *c, double *f, int depth) {

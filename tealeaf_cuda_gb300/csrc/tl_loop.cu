@@ -81,8 +81,11 @@ __global__ void __launch_bounds__(kGroupThreads, 4) k_cg_pass1(Geo g, CgArgs a, 
     grid_reduce<1>(acc, red, g.sms);
 }
 
+// (block-Jacobi: 4 CTAs a multiprocessor, in two even goes.  At the 80 registers
+// that let six in the other two had it to themselves: 101.2 and 215.7 us at 2600^2
+// and 4096^2 cells, 101.8 and 204.8 with four, 103.7 and 209.7 with eight of 64.)
 template <int PC>
-__global__ void __launch_bounds__(kGroupThreads, PC == TL_PREC_JAC_BLOCK ? 6 : 8) k_cg_pass2(Geo g, CgArgs a, RedCtx red) {
+__global__ void __launch_bounds__(kGroupThreads, PC == TL_PREC_JAC_BLOCK ? 4 : 8) k_cg_pass2(Geo g, CgArgs a, RedCtx red) {
     if (*(volatile const int *)red.done) return;
     AlphaBeta ab{red.sc->alpha, 0.0};
     double acc[1] = {0.0};
@@ -412,8 +415,9 @@ __device__ __forceinline__ void ppcg_pass2(const Geo &g, const StepArgs &a, int 
     }
 }
 
+// (all 8 CTAs of a multiprocessor at once: block-Jacobi at 4096^2 cells 260 -> 220 us)
 template <int PC>
-__global__ void __launch_bounds__(kGroupThreads) k_ppcg_pass2(Geo g, StepArgs a, const DevScalars *sc) {
+__global__ void __launch_bounds__(kGroupThreads, 8) k_ppcg_pass2(Geo g, StepArgs a, const DevScalars *sc) {
     if (*(volatile const int *)&sc->done) return;
     const double theta_r = 1.0 / sc->theta;
     double alpha = sc->alpha;
@@ -862,7 +866,7 @@ int launch_jacobi_finish(Chunk *c) {
 // graph of passes: 14.5 and 24.5 at 512^2 (run 1), 37 and 51 at 1024^2 (2), 71
 // and 82 at 1400^2 (4), 127 and 133 at 2048^2 (7), 223 and 215 at 2816^2 (13).
 bool loop_pays(const Chunk *c) {
-    return c->loop_ok && !c->profiling && !c->cfg.reflective_boundary && c->g.run <= 8;
+    return c->loop_ok && !c->profiling && !c->cfg.reflective_boundary && c->g.run <= kLoopRun;
 }
 
 }  // namespace tl
