@@ -98,7 +98,6 @@ BYTES_PER_CELL = {
     "ppcg_w_zr": 64,     # read p, Kx, Ky, diag, r, z; write w, r_store
     "ppcg_rrn": 24,      # read r, r_store, z
     # mixed precision: FP32 inner iteration (4-byte elements)
-    "mixed_pw": 32,      # read z, p, d, Kx, Ky; write p, d, w
     "mixed_init": 28,    # read r (FP64), Mi; write r, z, p, d
     "mixed_update_u": 24,  # read u (FP64), d, p; write u (FP64)
     "mixed_pp_init": 28,   # read r, z (FP64); write sd, rtemp, utemp
@@ -159,9 +158,12 @@ def bytes_per_cell(kernel, precond):
         # read rtemp, sd, utemp + the preconditioner (Mi; or diag, Ky, cp,
         # bfp); write sd, utemp
         return {"none": 40, "jac_diag": 48, "jac_block": 72}[precond]
+    if kernel == "mixed_pw":
+        # read z (r; r and Mi), p, d, Kx, Ky; write p, d, w
+        return {"none": 32, "jac_diag": 36, "jac_block": 32}[precond]
     if kernel == "mixed_rz":
-        # read r, w + the preconditioner (Mi; or Ky, cp, bfp); write r, z
-        return {"none": 12, "jac_diag": 20, "jac_block": 28}[precond]
+        # read r, w + the preconditioner (Mi; or Ky, cp, bfp); write r (and z)
+        return {"none": 12, "jac_diag": 16, "jac_block": 28}[precond]
     if kernel == "mixed_convert":
         # read Kx, Ky and the preconditioner (FP64; Mi or cp, bfp); write them in FP32
         return {"none": 24, "jac_diag": 36, "jac_block": 48}[precond]

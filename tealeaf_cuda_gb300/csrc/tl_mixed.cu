@@ -263,16 +263,22 @@ __device__ __forceinline__ void reduce_v(CSum acc, double *partials, unsigned in
 // beta here are those of the iteration before, 0 in the first.
 //   k_v_pw  d += alpha p, p' = z + beta p, w = A p'; sum p'.w
 //   k_v_rz  r -= alpha w, z = M^-1 r; sum r.z and the exit test
-// 32 + 20 bytes a cell (jac_diag) where separate d/r, p and w passes took 60.
+// 36 + 16 bytes a cell (jac_diag) where separate d/r, p and w passes took 60.
+// With jac_diag z is not stored: pass 1 forms it from r and Mi.  That moves the
+// same bytes (32 + 20 with z), but eight arrays take part instead of nine: where
+// they just fit in L2 pw and rz took 36.5 us at 1730^2 cells, the three passes
+// 35.6, now 31.6; 92.1, 99.6 and 87.4 at 3000^2, 330, 374 and 317 at 6000^2.
 // HBM-bound.  A warp marches down a run of rows of 128 columns, runs side by
 // side at the same rows; there are as many runs as the device's warps take at
 // once, so no wave of blocks is left half empty and little is read twice.
 // p' goes to the other of two buffers (DevScalars::p_sel): the
 // neighbours' p' are computed again from z and p.
+// MI: z is r, and M^-1 r is formed here (jac_diag).
+template <bool MI>
 __device__ __forceinline__ CSum v_pw(const GeoV &g, int c, int jb, int je, float *__restrict__ d,
                                      const float *__restrict__ p, float *__restrict__ po, const float *__restrict__ z,
-                                     const float *__restrict__ kx, const float *__restrict__ ky,
-                                     float *__restrict__ w, float alpha, float beta) {
+                                     const float *__restrict__ mi, const float *__restrict__ kx,
+                                     const float *__restrict__ ky, float *__restrict__ w, float alpha, float beta) {
     const int lane = threadIdx.x & 31;
     const int nv = min(4, g.nx - c);           // valid columns of this lane
     const bool live = c < g.nx + 4;            // lanes that load (the first one past nx reads the halo)
@@ -282,7 +288,8 @@ __device__ __forceinline__ CSum v_pw(const GeoV &g, int c, int jb, int je, float
         int64_t i = (int64_t)(c + g.h) + (int64_t)(jb + g.h) * P;
         int j0 = jb;
         const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-        auto next_p = [&](const float4 &zv, const float4 &pv) {
+        auto next_p = [&](float4 zv, const float4 &mv, const float4 &pv) {
+            if (MI) zv = make_float4(zv.x * mv.x, zv.y * mv.y, zv.z * mv.z, zv.w * mv.w);
             return make_float4(fmaf(beta, pv.x, zv.x), fmaf(beta, pv.y, zv.y), fmaf(beta, pv.z, zv.z),
                                fmaf(beta, pv.w, zv.w));
         };
@@ -292,9 +299,11 @@ __device__ __forceinline__ CSum v_pw(const GeoV &g, int c, int jb, int je, float
         // so row ny (the halo) is the last one read; nothing past the run's next row.
         auto ldrow = [&](const float *f, int64_t at, int row) { return (live && row <= je) ? ld4(f, at) : z4; };
         auto ldnew = [&](const float *f, int64_t at, int row) { return (live && row <= je) ? ld4cg(f, at) : z4; };
-        float4 xm = next_p(ldnew(z, i - P, j0 - 1), ldnew(p, i - P, j0 - 1));
+        auto ldmi = [&](int64_t at, int row) { return MI ? ldrow(mi, at, row) : z4; };
+        float4 xm = next_p(ldnew(z, i - P, j0 - 1), ldmi(i - P, j0 - 1), ldnew(p, i - P, j0 - 1));
         float4 pc = ldnew(p, i, j0), pn = ldnew(p, i + P, j0 + 1);  // old p of rows rr, rr + 1
-        float4 x0 = next_p(ldnew(z, i, j0), pc), xp = next_p(ldnew(z, i + P, j0 + 1), pn);
+        float4 x0 = next_p(ldnew(z, i, j0), ldmi(i, j0), pc);
+        float4 xp = next_p(ldnew(z, i + P, j0 + 1), ldmi(i + P, j0 + 1), pn);
         float4 ky0 = ldrow(ky, i, j0), ky1 = ldrow(ky, i + P, j0 + 1);
         float4 kxv = ldrow(kx, i, j0), dv = ldnew(d, i, j0);
         // the last lane's east face; the first and last lane's neighbours
@@ -302,22 +311,24 @@ __device__ __forceinline__ CSum v_pw(const GeoV &g, int c, int jb, int je, float
         const int eo = lane == 0 ? -1 : 4;
         float kxe_edge = lane == 31 && live ? kx[i + 4] : 0.f;
         float ze = edge ? __ldcg(z + i + eo) : 0.f, pe = edge ? __ldcg(p + i + eo) : 0.f;
+        float me = MI && edge ? mi[i + eo] : 0.f;
         for (; j0 < je; j0 += kVUnroll)
 #pragma unroll
         for (int rr = 0; rr < kVUnroll; ++rr) {
             if (j0 + rr >= je) break;
             const int64_t in = i + P, inn = i + 2 * P;
             const int rn = j0 + rr + 1, rnn = j0 + rr + 2;
-            const float4 zpp = ldnew(z, inn, rnn), ppp = ldnew(p, inn, rnn);
+            const float4 zpp = ldnew(z, inn, rnn), mpp = ldmi(inn, rnn), ppp = ldnew(p, inn, rnn);
             const float4 ky2 = ldrow(ky, inn, rnn);
             const float4 kxn = ldrow(kx, in, rn), dn = ldnew(d, in, rn);
             const bool more = rn < je;
             const float kxe_n = lane == 31 && live && more ? kx[in + 4] : 0.f;
             const float ze_n = edge && more ? __ldcg(z + in + eo) : 0.f, pe_n = edge && more ? __ldcg(p + in + eo) : 0.f;
+            const float me_n = MI && edge && more ? mi[in + eo] : 0.f;
             float kxe = __shfl_down_sync(0xffffffffu, kxv.x, 1);
             float xe = __shfl_down_sync(0xffffffffu, x0.x, 1);
             float xw = __shfl_up_sync(0xffffffffu, x0.w, 1);
-            const float xb = fmaf(beta, pe, ze);
+            const float xb = fmaf(beta, pe, MI ? ze * me : ze);
             if (lane == 31 && live) {
                 kxe = kxe_edge;
                 xe = xb;
@@ -341,7 +352,7 @@ __device__ __forceinline__ CSum v_pw(const GeoV &g, int c, int jb, int je, float
             xm = x0;
             x0 = xp;
             pc = pn;
-            xp = next_p(zpp, ppp);
+            xp = next_p(zpp, mpp, ppp);
             pn = ppp;
             ky0 = ky1;
             ky1 = ky2;
@@ -350,22 +361,24 @@ __device__ __forceinline__ CSum v_pw(const GeoV &g, int c, int jb, int je, float
             kxe_edge = kxe_n;
             ze = ze_n;
             pe = pe_n;
+            me = me_n;
             i += P;
         }
     }
     return acc;
 }
+template <bool MI>
 __global__ void __launch_bounds__(kBlockThreads) k_v_pw(GeoV g, float *__restrict__ d, float *__restrict__ p0,
                                                         float *__restrict__ p1, const float *__restrict__ z,
-                                                        const float *__restrict__ kx, const float *__restrict__ ky,
+                                                        const float *__restrict__ mi, const float *__restrict__ kx, const float *__restrict__ ky,
                                                         float *__restrict__ w, double *partials, unsigned int *counter,
                                                         DevScalars *sc) {
     if (*(volatile const int *)&sc->done) return;
     const bool sel = sc->p_sel != 0;
     const int run = blockIdx.x * kBlockWarps + (threadIdx.x >> 5), band = run / g.tiles_x;
-    const CSum acc = v_pw(g, (run - band * g.tiles_x) * kVCols + (threadIdx.x & 31) * 4, band * g.rows,
-                          min(band * g.rows + g.rows, g.ny), d, sel ? p1 : p0, sel ? p0 : p1, z, kx, ky, w,
-                          (float)sc->in_alpha, (float)sc->in_beta);
+    const CSum acc = v_pw<MI>(g, (run - band * g.tiles_x) * kVCols + (threadIdx.x & 31) * 4, band * g.rows,
+                              min(band * g.rows + g.rows, g.ny), d, sel ? p1 : p0, sel ? p0 : p1, z, mi, kx, ky, w,
+                              (float)sc->in_alpha, (float)sc->in_beta);
     reduce_v(acc, partials, counter, sc, kInW);
 }
 
@@ -373,7 +386,8 @@ __global__ void __launch_bounds__(kBlockThreads) k_v_pw(GeoV g, float *__restric
 // TL_PREC_JAC_DIAG (z = Mi r) or TL_PREC_JAC_BLOCK (the 4-row strip solve of
 // k_pp_step on the warp's two strips; ky, cp and bfp with 1/diag in each
 // strip's first row)
-template <int PC>
+// STORE false: z stays here (jac_diag, whose v_pw forms it again)
+template <int PC, bool STORE = PC != TL_PREC_NONE>
 __device__ __forceinline__ CSum v_rz(const GeoV &g, int c, int jb, int je, float *__restrict__ r,
                                      float *__restrict__ z, const float *__restrict__ w, const float *__restrict__ mi,
                                      const float *__restrict__ ky, const float *__restrict__ cp,
@@ -433,7 +447,7 @@ __device__ __forceinline__ CSum v_rz(const GeoV &g, int c, int jb, int je, float
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 if (k >= m) break;
-                if (PC != TL_PREC_NONE) st4(z, i0 + (int64_t)k * P, zv[k], nv);
+                if (STORE) st4(z, i0 + (int64_t)k * P, zv[k], nv);
                 csum_add(acc, rv[k].x * zv[k].x);
                 if (nv > 1) csum_add(acc, rv[k].y * zv[k].y);
                 if (nv > 2) csum_add(acc, rv[k].z * zv[k].z);
@@ -451,7 +465,7 @@ __global__ void __launch_bounds__(kBlockThreads, 3) k_v_rz(GeoV g, float *__rest
                                                         unsigned int *counter, DevScalars *sc) {
     if (*(volatile const int *)&sc->done) return;
     const int run = blockIdx.x * kBlockWarps + (threadIdx.x >> 5), band = run / g.tiles_x;
-    const CSum acc = v_rz<PC>(g, (run - band * g.tiles_x) * kVCols + (threadIdx.x & 31) * 4, band * g.rows,
+    const CSum acc = v_rz<PC, PC == TL_PREC_JAC_BLOCK>(g, (run - band * g.tiles_x) * kVCols + (threadIdx.x & 31) * 4, band * g.rows,
                               min(band * g.rows + g.rows, g.ny), r, z, w, mi, ky, cp, bfp, (float)sc->in_alpha);
     reduce_v(acc, partials, counter, sc, kInUr);
 }
@@ -490,8 +504,8 @@ __global__ void __launch_bounds__(kVLoopThreads, 1) k_v_loop(LoopArgs L, GeoV g,
         const int jb = min(band * g.rows, g.ny), je = min(jb + g.rows, g.ny);
         for (int it = 0; it < L.iters; ++it) {
             const bool sel = S.sc.p_sel != 0;
-            CSum acc = v_pw(g, c, jb, je, a.d, sel ? a.p1 : a.p0, sel ? a.p0 : a.p1, a.src, a.kx, a.ky, a.w,
-                            (float)S.sc.in_alpha, (float)S.sc.in_beta);
+            CSum acc = v_pw<false>(g, c, jb, je, a.d, sel ? a.p1 : a.p0, sel ? a.p0 : a.p1, a.src, nullptr, a.kx, a.ky,
+                                   a.w, (float)S.sc.in_alpha, (float)S.sc.in_beta);
             S.sh[0][warp][lane] = (double)acc.s + (double)acc.e;
             loop_arrive<1>(L, S);
             loop_met();
@@ -1462,7 +1476,6 @@ GeoV run_geo(const Chunk *c, int warps, int unit, unsigned *grid, int least = 8)
 template <int PC>
 int inner_body_pc(Chunk *c) {
     Mixed *mx = mixed_of(c);
-    const bool diag = PC != TL_PREC_NONE;
     unsigned grid, grid_rz;
     // (the block solve takes whole strips)
     const GeoV g = run_geo(c, 2 * kBlockWarps, 1, &grid);
@@ -1470,8 +1483,9 @@ int inner_body_pc(Chunk *c) {
     cudaStream_t s = c->stream;
     int rc;
     if ((rc = launch_v(c, "mixed_pw", [&] {
-             k_v_pw<<<grid, kBlockThreads, 0, s>>>(g, mx->d, mx->p, mx->sd[0], diag ? mx->z : mx->r, mx->kx, mx->ky,
-                                                    mx->w, mx->partials, mx->counter, c->sc);
+             k_v_pw<PC == TL_PREC_JAC_DIAG><<<grid, kBlockThreads, 0, s>>>(
+                 g, mx->d, mx->p, mx->sd[0], PC == TL_PREC_JAC_BLOCK ? mx->z : mx->r, mx->mi, mx->kx, mx->ky, mx->w,
+                 mx->partials, mx->counter, c->sc);
          })))
         return rc;
     return launch_v(c, "mixed_rz", [&] {
