@@ -862,9 +862,19 @@ int launch_jacobi_finish(Chunk *c) {
 
 // Short runs: the loop saves the launches (2 to 13 an iteration) and their
 // waits; in long ones 16 warps a multiprocessor do not keep HBM as busy as the
-// passes' own kernels.  Microseconds an iteration of CG + jac_diag, loop and
-// graph of passes: 14.5 and 24.5 at 512^2 (run 1), 37 and 51 at 1024^2 (2), 71
-// and 82 at 1400^2 (4), 127 and 133 at 2048^2 (7), 223 and 215 at 2816^2 (13).
+// passes' own kernels, and those of 96 registers spill (tl_loop.cuh).
+// Microseconds an iteration, loop / graph of passes (PPCG with 10 inner steps):
+//                      500^2 (run 1)  1080^2 (2)   1540^2 (4)   2060^2 (7)    2200^2 (8)
+//   CG, none           14.1 / 24.8    35 / 50      65 / 82      106 / 126     122 / 137
+//   CG, jac_diag       15.1 / 25.4    41 / 55      78 / 88      128 / 136     148 / 148
+//   CG, block          17.2 / 28.2    49 / 68      94 / 110     154 / 173     173 / 191
+//   Chebyshev, none    10.9 / 18.8    31 / 44      60 / 73      100 / 116     114 / 127
+//   Chebyshev, diag    11.6 / 19.4    34 / 47      67 / 79      111 / 125     126 / 137
+//   Chebyshev, block   13.1 / 21.6    40 / 53      80 / 92      133 / 145     150 / 161
+//   PPCG, none         105 / 129      317 / 354    629 / 660    1052 / 1089   1200 / 1228
+//   PPCG, jac_diag     113 / 136      347 / 386    685 / 733    1146 / 1202   1303 / 1350
+//   Jacobi             15.1 / 19.8    46 / 53      88 / 95      152 / 158     173 / 176
+// (PPCG with block-Jacobi: ppcg_loop_pays)
 bool loop_pays(const Chunk *c) {
     return c->loop_ok && !c->profiling && !c->cfg.reflective_boundary && c->g.run <= kLoopRun;
 }

@@ -440,6 +440,10 @@ int launch_named(Chunk *c, const char *name, F &&launch) {
 // so 9 warps (with the control warp) can have 168 each, 17 have 96.
 //   depth 1, 2: 2 groups of 168 registers, the four rows of a strip at once;
 //   more:       4 groups of 96 registers, 2 rows ahead, in 1 or 2 rounds.
+// The second spills: bytes stored and loaded a thread 54 / 116 (none), 146 / 208
+// (jac_diag) and 242 / 284 (block) in CG, 106 / 124, 156 / 172 and 568 / 452 in PPCG, 32 /
+// 80 to 148 / 172 in Chebyshev, 60 / 92 in Jacobi, 22 / 32 to 52 / 68 in mixed PPCG; the
+// first only in PPCG with block-Jacobi (124 / 156) and jac_diag (4 / 8).
 // (3 groups of 128 registers, 4 rows ahead, in up to 3 rounds: 519 us an
 // iteration at 4096^2 against 442.)
 template <int GROUPS, int AHEAD>

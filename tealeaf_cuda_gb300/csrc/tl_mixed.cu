@@ -472,9 +472,8 @@ __global__ void __launch_bounds__(kBlockThreads, 3) k_v_rz(GeoV g, float *__rest
 
 // Both passes of many iterations in one launch (tl_loop.cuh): 15 passing warps
 // a multiprocessor (128 registers each, as four warps share a quarter of them), each with the same run in both passes.
-// What bounds it: the two meetings and the latency of one row after another
-// (1024^2 cells, jac_diag: 16.6 us an iteration, 20.2 as two launches of passes).
-constexpr int kVLoopRows = 7;  // rows of the longest runs (inner_loop_pays)
+// What bounds it: the two meetings and the latency of one row after another, and
+// the spills of 128 registers (inner_loop_pays, with both sides' times).
 constexpr int kVLoopWarps = 15, kVLoopThreads = kVLoopWarps * 32 + 32;
 struct VLoopArgs {
     float *d, *p0, *p1, *r, *z, *w;
@@ -1508,16 +1507,23 @@ int inner_loop_pc(Chunk *c) {
 }
 
 // The FP32 CG iterations in loops: while the runs are short.  Microseconds an
-// iteration with and without jac_diag, loop and two launches of passes: 13 / 12
-// and 22 / 21 at 96 x 80 (runs of 4 rows), 17 / 15 and 20 / 19 at 1024^2 (4), 20 /
-// 17 and 23 / 22 at 1200^2 (6), 25 / 19 and 26 / 24 at 1400^2 (7), 30 / 21 and 27 /
-// 24 at 520 x 4000 (9), 42 / 27 and 37 / 27 at 1700^2 (10), 83 / 63 and 71 / 60 at
-// 3000 x 2100 (22): 15 warps a multiprocessor are too few for the passes' loads.
+// iteration, loop and two launches of passes, by the rows of a run:
+//   none       14.3 / 17.8 at 1024^2 (4), 16.3 / 20.8 at 1200^2 (6), 18.8 / 20.9 at
+//              1340^2 (7), 20.9 / 23.1 at 520 x 4000 and 22.2 / 22.4 at 1536^2 (9), 24.4 /
+//              24.0 at 1600^2 (10)
+//   jac_diag   16.0 / 19.1 at 1024^2 (4), 19.2 / 22.3 at 1200^2 and 21.1 / 22.3 at 2000 x
+//              800 (6), 24.0 / 22.9 at 1340^2 (7), 28.0 / 24.0 at 1480^2 (8)
+//   jac_block  (the presteps of mixed PPCG; whole strips) 17.8 / 23.5 at 1024^2 (4),
+//              23.3 / 27.7 at 520 x 2700, 23.1 / 26.9 at 1200^2, but 29.6 / 28.7 at 1279^2 and
+//              28.5 / 27.1 at 2000 x 800 (6), 30.2 / 28.2 at 1340^2 (7)
+// A preconditioner's kernel holds too few registers for the passes' loads: at 128
+// a thread it spills 376 bytes (324 loaded), without one 420 (168), where the
+// passes' own kernels need 116 to 119 and spill none.
 bool inner_loop_pays(const Chunk *c) {
     const GeoV g = run_geo(c, kVLoopWarps, 1, nullptr, 4);
     // (a field with more tiles side by side than there are warps has runs left over)
     return c->loop_ok && !c->profiling && !c->cfg.reflective_boundary && g.tiles_x <= c->g.sms * kVLoopWarps &&
-           g.rows <= kVLoopRows;
+           g.rows <= (c->cfg.precond == TL_PREC_NONE ? 9 : 6);
 }
 int inner_loop(Chunk *c) {
     return by_precond(c, [&](auto pc) { return inner_loop_pc<decltype(pc)::value>(c); });

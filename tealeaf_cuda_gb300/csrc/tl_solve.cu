@@ -86,11 +86,22 @@ bool ppcg_fused(const Chunk *c) {
            !c->no_sd_alt;
 }
 
+// FP64 PPCG in loops: where loops pay, but with block-Jacobi, whose loop spills most
+// (tl_loop.cuh), up to 85 strips a multiprocessor.  Microseconds an outer iteration,
+// loop / graph of passes: 134 / 152 at 500^2 (13 strips), 437 / 450 at 1080^2 (60), 550 /
+// 601 at 1150^2 (68), 610 / 625 at 1240^2 (80), 677 / 651 at 1340^2 (93), 877 / 827 at 1540^2
+// (122), 1667 / 1545 at 2200^2 (250).
+bool ppcg_loop_pays(const Chunk *c) {
+    return loop_pays(c) && !(c->cfg.precond == TL_PREC_JAC_BLOCK &&
+                             (long long)c->g.tiles_x * c->g.nstrips > 85LL * c->g.sms);
+}
+
 // Mixed PPCG in loops: while the fused passes cannot fill the device, and only
 // with the inner steps' default settings (and fields of 32-bit offsets).
-// Microseconds an outer iteration with block-Jacobi, loop and graph of fused
-// passes: 32 and 126 at 128^2, 42 and 151 at 512^2, 91 and 181 at 1024^2 (run 2),
-// 185 and 208 at 1400^2 (4), 447 and 303 at 2048^2 (7).
+// Microseconds an outer iteration with block-Jacobi, loop / graph of fused passes:
+// 40 / 139 at 300^2, 48 / 150 at 500^2, 69 / 169 at 760^2 (run 1), 115 / 189 at 1080^2 (2),
+// 161 / 209 at 1340^2 (3), 204 / 234 at 1540^2 (4), 254 / 275 at 1730^2 (5), 317 / 291 at
+// 1900^2 (6), 461 / 317 at 2060^2 (7); jac_diag 188 / 217 and none 179 / 205 at 1540^2.
 bool mixed_loop_pays(const Chunk *c) {
     return c->inner_fuse == kInnerFuseDefault && c->inner_seg == kInnerSegDefault && !c->inner_fold_rrn &&
            c->cfg.ppcg_inner_steps >= 1 && c->g.sets == c->g.groups && c->alloc_elems < ((size_t)1 << 31) &&
@@ -416,7 +427,7 @@ int solve_timestep(Chunk *c, tl_solve_info_t *info) {
         case kPhasePpcg:
             if (ppcg_fused(c) && (rc = ppcg_alloc(c))) return rc;
             if (ppcg_fused(c)) {
-                rc = run_loop(c, launch_ppcg_loop, body_ppcg, kItersPpcg, kPhasePpcg, loop_pays(c), &done);
+                rc = run_loop(c, launch_ppcg_loop, body_ppcg, kItersPpcg, kPhasePpcg, ppcg_loop_pays(c), &done);
                 if (!rc) rc = launch_ppcg_finish(c);
             } else {
                 if (cf.precision == TL_PRECISION_MIXED && mixed_loop_pays(c))
