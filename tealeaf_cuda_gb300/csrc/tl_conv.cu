@@ -148,8 +148,8 @@ __global__ void __launch_bounds__(128) k_conv(const bf16 *__restrict__ in, const
 
 // ---------------------------------------------------------------------------
 // The same convolution on the 5th-generation tensor cores (tcgen05).  A tile is
-// 128 columns (M = 128) of kTcRows output rows.  Columns are counted over the
-// padded rows of a group of kTcRows rows and on into the next group, q = group
+// 128 columns (M = 128) of R output rows.  Columns are counted over the
+// padded rows of a group of R rows and on into the next group, q = group
 // (W + 2) + x, and a tile is any 128 consecutive q, so the two columns a row
 // that are no output are all that is computed in vain (1.4 % at W = 144, where
 // tiles of one row's pixels wasted 44 %).  W + 2 is even: an even q and the
@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(128) k_conv(const bf16 *__restrict__ in, const
 //
 // A CTA of 4 warps walks tiles: the weights stay in shared memory, and the next
 // tile's input is on its way (cp.async) while this one's result is written.
-// Shared memory holds, per input row k of kTcRows + 2, the 130 input pixels that
+// Shared memory holds, per input row k of R + 2, the 130 input pixels that
 // the three taps dx = 0, 1, 2 read, in the K-major no-swizzle layout of the MMA
 // operands: 16-byte core-matrix rows (one pixel, 8 channels), the pixels of
 // an 8-channel chunk contiguous (16 bytes apart) and the chunks kChunkA bytes
@@ -173,20 +173,20 @@ __global__ void __launch_bounds__(128) k_conv(const bf16 *__restrict__ in, const
 // lane, one channel a column) row by row and runs the epilogue of k_conv.
 // Lanes trade half of their chunks with their neighbours before a store, so
 // that every store writes whole 32-byte sectors.
-// What bounds it: latency, with three CTAs (12 warps) a multiprocessor that wait
+// What bounds it, at 4 rows: latency, with three CTAs (12 warps) a multiprocessor that wait
 // for their loads between the MMAs and the epilogue; then L2, from which an
-// input row is read (kTcRows + 2) / kTcRows times (tensor cores 11-15 % busy,
+// input row is read (R + 2) / R times (tensor cores 11-15 % busy,
 // HBM 29 %).  4096 x 4096 pixels, 32 to 32 channels with GELU and the input
 // added: 947 us, HBM's 2.1 GB take 317.  One row a tile (three reads): two
 // buffers and 3 CTAs 1250, one buffer and 5 CTAs 1090; two rows and 4 CTAs 930,
 // but 605 for the head where four rows take 527; three rows 986.  32 x 144 x 144
 // pixels with the pre-activation written: one row 64 and 58, two 53, four 53 us.
-constexpr int kTcRows = 4;                // output rows of a tile (above: 1 to 4 measured)
 constexpr int kTcPix = 128;               // pixels of a tile (MMA M)
 constexpr int kTcRow = kTcPix + 2;        // input pixels a kernel row of a tile reads
 constexpr int kChunkA = kTcRow * 16;      // bytes between 8-channel chunks of A
-constexpr int kTmemCols = 32 * kTcRows;   // accumulator columns allocated (>= kTcRows COUTP)
-constexpr int kTcCtas = 3;                // CTAs a multiprocessor (68 KB of shared memory each)
+// CTAs a multiprocessor (43, 52 and 68 KB of shared memory each at 1, 2 and 4 rows)
+__host__ __device__ constexpr int tc_ctas(int r) { return r == 1 ? 5 : r == 2 ? 4 : 3; }
+__host__ __device__ constexpr int tmem_cols(int r) { return 32 * r; }  // accumulator columns allocated (>= R COUTP)
 constexpr long long kTcWaitCycles = 2000000000LL;  // ~1 s: the MMA wait gives up after this
 
 // set by a tcgen05 conv whose MMA completion wait ran out (read and cleared
@@ -262,9 +262,9 @@ __device__ __forceinline__ void tmem_load<16>(uint32_t taddr, float (&v)[16]) {
     for (int k = 0; k < 16; ++k) v[k] = __uint_as_float(r[k]);
 }
 
-template <int CIN, int COUTP>
+template <int CIN, int COUTP, int R>
 constexpr int conv_tc_smem() {
-    return (kTcRows + 2) * (CIN / 8) * kChunkA + 9 * (CIN / 8) * COUTP * 16;
+    return (R + 2) * (CIN / 8) * kChunkA + 9 * (CIN / 8) * COUTP * 16;
 }
 
 // store 8 channels a lane of COUTP, `at` the lane's pixel: two chunks of the
@@ -288,16 +288,15 @@ __device__ __forceinline__ void store_chunks(bf16 *dst, long long at, int chunk,
         *reinterpret_cast<uint4 *>(dst + (e0 + 1) * COUTP + 8 * c) = make_uint4(odd_px[0], odd_px[1], odd_px[2], odd_px[3]);
 }
 
-template <int CIN, int COUTP, int MODE>
-__global__ void __launch_bounds__(128, kTcCtas) k_conv_tc(const bf16 *__restrict__ in, const bf16 *__restrict__ wt,
+template <int CIN, int COUTP, int MODE, int R>
+__global__ void __launch_bounds__(128, tc_ctas(R)) k_conv_tc(const bf16 *__restrict__ in, const bf16 *__restrict__ wt,
                                                  const float *__restrict__ bias,
                                                  const bf16 *__restrict__ res, bf16 *__restrict__ out,
                                                  bf16 *__restrict__ pre, float *__restrict__ outf, int B,
                                                  int H, int W) {
-    static_assert(CIN % 16 == 0 && COUTP % 16 == 0 && kTcRows * COUTP <= kTmemCols, "conv shape");
+    static_assert(CIN % 16 == 0 && COUTP % 16 == 0 && R * COUTP <= tmem_cols(R), "conv shape");
     constexpr int CA = CIN / 8;                    // 8-channel chunks of a pixel
     constexpr int CHUNK_B = 3 * COUTP * 16;        // bytes between chunks of the weights
-    constexpr int R = kTcRows;
     constexpr int A_BYTES = (R + 2) * CA * kChunkA;
     extern __shared__ __align__(128) unsigned char conv_smem[];
     unsigned char *const sb = conv_smem + A_BYTES;
@@ -313,7 +312,7 @@ __global__ void __launch_bounds__(128, kTcCtas) k_conv_tc(const bf16 *__restrict
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                          smem_addr(&tmem_slot)),
-                     "r"(kTmemCols));
+                     "r"(tmem_cols(R)));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (tid == 0) {
@@ -497,7 +496,7 @@ __global__ void __launch_bounds__(128, kTcCtas) k_conv_tc(const bf16 *__restrict
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_slot), "r"(kTmemCols));
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_slot), "r"(tmem_cols(R)));
 }
 
 // dpre = dh * gelu'(pre) over the interior (halo left at zero).  Bound by HBM
@@ -800,18 +799,49 @@ __global__ void k_gather(const float *__restrict__ fields, const int *__restrict
 // which kernel tl_nn_conv runs: the tcgen05 one (default) or mma.sync
 bool g_conv_tcgen05 = true;
 
+// tiles of r rows
+long long conv_tiles(int r, int B, int H, int W) {
+    return (((long long)((H + r - 1) / r) * (W + 2) + kTcPix - 1) / kTcPix) * B;
+}
+// Rows of a tile: four read an input row least often; one, or two, where the device
+// is not full, whose blocks have less to do one after the other, and where taller
+// tiles would be no fewer.  Microseconds with 1, 2 and 4 rows, 32 to 32 channels,
+// GELU and residual, batch x height x width (one-row tiles in brackets): 8.4, 10.3,
+// 12.5 at 1 x 64 x 64 (33), 10.3, 10.5, 12.6 at 1 x 200 x 192 (304), 12.5, 12.4, 12.5 at
+// 1 x 256 x 256 (516), 14.5, 14.5, 16.5 at 8 x 100 x 96 (616; 312 of two rows), 16.6, 16.6,
+// 16.5 at 12 x 100 x 96 (924; 468), 33, 29, 31 at 16 x 144 x 144, 60, 52, 51 at 32 x 144 x
+// 144; the head 6.4, 7.8, 8.3, then 8.3, 8.3, 8.4, 10.3, 8.4, 8.4, 10.5, 10.4, 10.4, 12.5, 11.2,
+// 10.5, 25, 21, 19 and 41, 35, 29; 512 x 1 x 32: 10.6, 14.5, 22.6.
+int conv_rows(int B, int H, int W) {
+    const long long t1 = conv_tiles(1, B, H, W), t2 = conv_tiles(2, B, H, W), t4 = conv_tiles(4, B, H, W);
+    if (t1 <= 3 * kSms || t1 <= t2) return 1;
+    return t2 <= 3 * kSms || t2 <= t4 ? 2 : 4;
+}
+
+template <int CIN, int COUTP, int MODE, int R>
+int launch_conv_tc(const void *in, const void *w, const float *bias, const void *res, void *out, void *pre,
+                   float *outf, int B, int H, int W, cudaStream_t s) {
+    constexpr int bytes = conv_tc_smem<CIN, COUTP, R>();
+    const cudaError_t e = cudaFuncSetAttribute(k_conv_tc<CIN, COUTP, MODE, R>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess) return cuda_fail(e, "conv shared memory");
+    const long long tiles = conv_tiles(R, B, H, W), ctas = kSms * tc_ctas(R);
+    k_conv_tc<CIN, COUTP, MODE, R><<<(unsigned)(tiles < ctas ? tiles : ctas), 128, bytes, s>>>(
+        (const bf16 *)in, (const bf16 *)w, bias, (const bf16 *)res, (bf16 *)out, (bf16 *)pre, outf, B, H, W);
+    return TL_OK;
+}
+
 template <int CIN, int COUTP, int MODE>
 int launch_conv(const void *in, const void *w, const float *bias, const void *res, void *out, void *pre,
                 float *outf, int B, int H, int W, cudaStream_t s) {
     if (g_conv_tcgen05) {
-        constexpr int bytes = conv_tc_smem<CIN, COUTP>();
-        const cudaError_t e = cudaFuncSetAttribute(k_conv_tc<CIN, COUTP, MODE>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        if (e != cudaSuccess) return cuda_fail(e, "conv shared memory");
-        const long long tiles = (((long long)((H + kTcRows - 1) / kTcRows) * (W + 2) + kTcPix - 1) / kTcPix) * B;
-        const long long ctas = kSms * kTcCtas;
-        k_conv_tc<CIN, COUTP, MODE><<<(unsigned)(tiles < ctas ? tiles : ctas), 128, bytes, s>>>(
-            (const bf16 *)in, (const bf16 *)w, bias, (const bf16 *)res, (bf16 *)out, (bf16 *)pre, outf, B, H, W);
+        int rc;
+        switch (conv_rows(B, H, W)) {
+        case 1: rc = launch_conv_tc<CIN, COUTP, MODE, 1>(in, w, bias, res, out, pre, outf, B, H, W, s); break;
+        case 2: rc = launch_conv_tc<CIN, COUTP, MODE, 2>(in, w, bias, res, out, pre, outf, B, H, W, s); break;
+        default: rc = launch_conv_tc<CIN, COUTP, MODE, 4>(in, w, bias, res, out, pre, outf, B, H, W, s); break;
+        }
+        if (rc) return rc;
     } else {
         const long long tasks = (long long)B * H * (W / 16);
         const unsigned grid = (unsigned)((tasks + 3) / 4);
