@@ -537,10 +537,10 @@ __global__ void k_gelu_back(const bf16 *__restrict__ dh, const bf16 *__restrict_
 
 // Weight and bias gradients:
 //   dW[tap][co][ci] = sum_p dpre[p][co] * in[p + off(tap)][ci],  db[co] = sum_p dpre[p][co]
-// A contraction over the pixels with M = co and N = ci of 16 or 32 a tap, below
-// the 64 rows of a tensor-memory MMA, so it runs on mma.sync (M = co, N = ci,
-// K = 16 pixels), one warp a tap; warp 4 also multiplies dpre by a column of
-// ones, which is db.  A CTA walks segments of kWgSeg pixels counted over the
+// A contraction over the pixels, on mma.sync (M = co, N = ci, K = 16 pixels), one
+// warp a tap; warp 4 also multiplies dpre by a column of ones, which is db.  (A
+// product for the tensor memory's units would stack the taps, dx and ci along M,
+// dy and co along N, both operands channel by channel; not tried.)  A CTA walks segments of kWgSeg pixels counted over the
 // padded rows as k_conv_tc counts them (a grid-stride loop over the segments
 // of all images; dpre enters as 0 for the two columns a row that are no pixels):
 // it stages the segment's dpre and the input that its taps read in shared memory (16-byte

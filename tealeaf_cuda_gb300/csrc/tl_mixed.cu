@@ -721,7 +721,7 @@ __global__ void __launch_bounds__(kBlockThreads) k_pp_step(
 // of T single steps.
 // What bounds it: the latency of shared memory and of the chain through the
 // levels, with 12 warps a multiprocessor (168 registers a thread): issue slots
-// and shared memory are each half used, HBM 40 %.  (8192^2 cells, block-Jacobi,
+// and shared memory are each half used, HBM half (0.51 of the copy rate).  (8192^2 cells, block-Jacobi,
 // 5 steps: 692 us; with the pairs (0, 1) and (2, 3), whose neighbours are not
 // pairs, and Ky above a strip read from shared memory: 716.  r - alpha w formed in
 // the first pass instead of by a pass of its own: 130 us more a pass.)
