@@ -220,8 +220,9 @@ int tl_test_fail_alloc(int nth);
 /* tl_test_loops -- no counterpart in the reference; a test hook for the kernels
  * that run many iterations a launch.  start_wait, wait: clocks that their thread
  * blocks wait for one another's start (then the solve goes on in separate
- * passes) and at a meeting (then it returns TL_ERR_CUDA); below 0: the defaults,
- * about two seconds.  iters: iterations a launch, 0: by the number of cells. */
+ * passes; -2: as if one had not started) and at a meeting (then it returns
+ * TL_ERR_CUDA); -1: the defaults, about two seconds.  iters: iterations a launch,
+ * 0: by the number of cells. */
 int tl_test_loops(tl_chunk_t *ch, long long start_wait, long long wait, int iters);
 
 /* tl_dot_noalloc -- no counterpart in the reference.  The dot-product

@@ -156,7 +156,7 @@ struct Chunk {
     double *loop_partials;
     unsigned int *loop_arrived;  // [0] arrivals, [1] arrivals before the next launch, [32] the gate
     unsigned int loop_round;     // launches so far
-    long long loop_start_wait, loop_wait;  // clocks; below 0: the defaults (tl_test_loops)
+    long long loop_start_wait, loop_wait;  // clocks; -1: the defaults (tl_test_loops)
     int loop_iters;              // iterations a launch; 0: by the number of cells (tl_test_loops)
     bool loop_ok;                // the device can hold a loop kernel's CTAs at once
     double *cg_alphas, *cg_betas;          // device, max_iters + 2

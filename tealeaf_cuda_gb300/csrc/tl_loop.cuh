@@ -40,7 +40,7 @@ struct LoopArgs {
     unsigned int *base;      // the value of `arrived` when the launch began
     unsigned int *gate;      // 2 round + 1: the launch of that round goes on, 2 round: it does not
     unsigned int round;      // this launch's number
-    long long start_wait;    // clocks to wait for the CTAs to start,
+    long long start_wait;    // clocks to wait for the CTAs to start (below 0: as if one had not),
     long long wait;          // and for them to come to a meeting
     double *cg_alphas, *cg_betas;
     int depth;      // groups of the busiest CTA
@@ -184,7 +184,7 @@ __device__ __forceinline__ bool loop_gather(const LoopArgs &L, unsigned int targ
     // (release: what was read so far, the base among it, was read before)
     asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(before) : "l"(L.arrived) : "memory");
     if (before + 1 == target) {
-        const bool go = answer(yes) == yes;
+        const bool go = answer(L.start_wait < 0 ? no : yes) == yes;
         if (!go) {
             *L.base = target;
             *(volatile int *)&L.sc->done = kNotStarted;
@@ -471,7 +471,7 @@ int launch_coop(Chunk *c, K kernel, LoopArgs &L, int slots, int threads, size_t 
     L.base = c->loop_arrived + 1;
     L.gate = c->loop_arrived + 32;
     L.round = ++c->loop_round & 0x7FFFFFFFu;
-    L.start_wait = c->loop_start_wait >= 0 ? c->loop_start_wait : kLoopWaitCycles;
+    L.start_wait = c->loop_start_wait == -1 ? kLoopWaitCycles : c->loop_start_wait;
     L.wait = c->loop_wait >= 0 ? c->loop_wait : kLoopWaitCycles;
     L.cg_alphas = c->cg_alphas;
     L.cg_betas = c->cg_betas;

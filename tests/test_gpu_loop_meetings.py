@@ -95,15 +95,15 @@ def test_launch_boundaries_carry_the_solve_on(method, precond, shape, iters):
 
 
 @pytest.mark.parametrize("method,precond", CASES)
-@pytest.mark.parametrize("start_wait,iters", [(0, 0), (2000, 3), (4000, 1)])
+@pytest.mark.parametrize("start_wait,iters", [(-2, 0), (0, 0), (2000, 3), (4000, 1)])
 def test_blocks_that_start_late(method, precond, start_wait, iters):
-    """Thread blocks that do not wait for the others' start: the launch does
-    nothing and the solve goes on in passes (also in the middle of a phase), to
+    """Thread blocks that do not wait for the others' start (or are told that one
+    is missing): the launch does nothing and the solve goes on in passes (also in the middle of a phase), to
     the same bits.  The second timestep is the one looked at: the first of mixed
     PPCG begins with FP32 CG iterations, whose loop and passes add in different
     orders.  Mixed CG, for the same reason, against its passes launched one by one."""
     mixed_cg = method == "mixed cg"
-    if mixed_cg and start_wait > 0:
+    if mixed_cg and start_wait >= 0:
         pytest.skip("some launches in loops and some in passes: no bits to compare with")
     deck = _deck(method, precond, (700, 333))
 
@@ -117,16 +117,9 @@ def test_blocks_that_start_late(method, precond, start_wait, iters):
                 assert tl.load().tl_set_profiling(ch._h, 1) == 0
             return _solve(ch, method, steps=1)
 
-    usual = second_step(False)
-    # now and then all blocks start within one another's first look, and none is late
-    for _ in range(30):
-        late = second_step(True)
-        if not mixed_cg:
-            _same(late, usual)
-        if late[2] > usual[2] or (mixed_cg and late[2] == usual[2]) or start_wait > 0:
-            break
-    else:
-        pytest.fail("no launch was late")
+    usual, late = second_step(False), second_step(True)
+    if start_wait < 0 and not mixed_cg:  # (else all blocks may start within one another's first look)
+        assert late[2] > usual[2]  # passes
     _same(late, usual)
 
 
